@@ -655,7 +655,8 @@ __global__ void __launch_bounds__(kThreads) k_tnode_layout(const BNode* __restri
     t.a = make_float4(A.lo_x, A.lo_y, A.lo_z, A.hi_x);
     t.b = make_float4(A.hi_y, A.hi_z, B.lo_x, B.lo_y);
     t.c = make_float4(B.lo_z, B.hi_x, B.hi_y, B.hi_z);
-    t.d = make_int4(lref, rref, 0, 0);
+    const bool up = x != 0 && nd.parent >= 0 && nd.parent < count;
+    t.d = make_int4(lref, rref, up ? max(compact[nd.parent], 0) : 0, 0);
     out[c] = t;
 }
 

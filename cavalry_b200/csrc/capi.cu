@@ -130,6 +130,7 @@ cav_status cav_ctx_destroy(cav_ctx* ctx) {
         if (ctx->hevent[k]) cudaEventDestroy(ctx->hevent[k]);
     }
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
+    if (ctx->wide_host) cudaFreeHost(ctx->wide_host);
     if (ctx->dev_stage) cudaFree(ctx->dev_stage);
     cudaFree(ctx->d_counters);
     cudaFree(ctx->d_error);
@@ -166,6 +167,7 @@ cav_status cav_set_trace_stack(cav_ctx* ctx, uint32_t flags, int stack, int smem
         return set_error(ctx, CAV_ERR_INVALID_ARGUMENT, "cav_set_trace_stack: stack 0/64/128, smem_stack 0/16");
     ctx->trace_stack = stack;
     ctx->trace_smem_stack = smem_stack;
+    ctx->screen_smem_stack = smem_stack;
     return CAV_OK;
 }
 

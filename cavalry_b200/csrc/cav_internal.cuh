@@ -77,29 +77,26 @@ struct __align__(64) TNode {
     float4 a;  // L.lo.x L.lo.y L.lo.z L.hi.x
     float4 b;  // L.hi.y L.hi.z R.lo.x R.lo.y
     float4 c;  // R.lo.z R.hi.x R.hi.y R.hi.z
-    int4 d;    // left ref, right ref, 0, 0
+    int4 d;    // left ref, right ref, parent (0 for the root), 0
 };
 static_assert(sizeof(TNode) == 64, "TNode must be 64 bytes");
 
-// Compressed 8-wide traversal node (80 bytes) of the fast mode, after Ylitie, Karras and
-// Laine, "Efficient Incoherent Ray Traversal on GPUs Through Compressed Wide BVHs" (HPG
-// 2017).  Child boxes are 8-bit offsets on a per-node grid: plane = p + q * 2^(e - 127) per
+// Compressed 8-wide traversal node (96 bytes: three 32-byte sectors, so that a node is two
+// 256-bit loads and one of 128 bits) after Ylitie, Karras and Laine, "Efficient Incoherent
+// Ray Traversal on GPUs Through Compressed Wide BVHs" (HPG 2017).  Child boxes are 8-bit offsets on a per-node grid: plane = p + q * 2^(e - 127) per
 // axis, rounded outward when quantised.  Internal children are stored contiguously from
 // child_base in slot order (imask bit s = slot s holds an internal child); triangle children
-// contiguously from tri_base.  meta[s]: 0 = empty slot; 0x20 | (24 + s) = internal child;
-// 0x20 | k = triangle tri_base + k.  A child's slot is chosen so that the slot number's bits
-// give the side of the node's centre it lies on (bit 2: +x, bit 1: +y, bit 0: +z), which lets
-// a ray visit children near-first by its direction octant alone.
-struct __align__(16) CNode {
+// contiguously from tri_base in slot order (tmask bit s).  A child's slot is chosen so that the
+// slot number's bits give the side of the node's centre it lies on (bit 2: +x, bit 1: +y, bit
+// 0: +z), which lets a ray visit children near-first by its direction octant alone.
+struct __align__(32) CNode {
     float px, py, pz;
     uint32_t e_imask;  // biased exponents x | y << 8 | z << 16, imask << 24
-    uint32_t child_base, tri_base;
-    uint32_t meta[2];  // slots 0-3, 4-7 (one byte each)
-    uint32_t qlo_x[2], qlo_y[2];
-    uint32_t qlo_z[2], qhi_x[2];
-    uint32_t qhi_y[2], qhi_z[2];
+    uint32_t child_base, tri_base, tmask, pad0;
+    uint32_t qlo_x[2], qlo_y[2], qlo_z[2], qhi_x[2];  // a byte per slot
+    uint32_t qhi_y[2], qhi_z[2], pad1[4];
 };
-static_assert(sizeof(CNode) == 80, "CNode must be 80 bytes");
+static_assert(sizeof(CNode) == 96, "CNode must be 96 bytes");
 
 // Triangle record (48 bytes) in sorted (Morton) order: v0, e1 = v1-v0, e2 = v2-v0
 // (the same subtractions as Core/Triangle.h:180-183), triangle id and mesh id.
@@ -133,7 +130,9 @@ struct cav_ctx {
     // launch configuration of the fast (compressed 8-wide) mode (0 = defaults)
     int wide_block = 0;
     int wide_batch = 0;
-    int wide_smem_stack = 0;  // > 0: the fast mode's first stack entries in shared memory
+    // > 0: the fast mode's first stack entries in shared memory; -1 (unset): for closest hits
+    int wide_smem_stack = -1;
+    int screen_smem_stack = -1;  // the same for the exact mode's screening pass
     // persistent work counters (device), one per concurrent trace kind
     unsigned long long* d_counters = nullptr;
     int* d_error = nullptr;
@@ -142,6 +141,7 @@ struct cav_ctx {
     size_t pinned_bytes = 0;
     void* dev_stage = nullptr;
     size_t dev_stage_bytes = 0;
+    void* wide_host = nullptr;  // pinned: a view build's counters
     cudaStream_t hstream[2] = {nullptr, nullptr};
     cudaEvent_t hevent[2] = {nullptr, nullptr};
     // Halton tables on the device, uploaded by the first scene and shared by all
@@ -170,10 +170,14 @@ struct cav_bvh {
     int32_t* perm = nullptr;             // N: sorted position -> triangle id
     // traversal layout
     cav::TNode* tnodes = nullptr;  // N-1
-    // compressed 8-wide view for CAV_TRACE_FAST, built on first use (wide.cu)
+    // compressed 8-wide view, built on first use (wide.cu)
     mutable cav::CNode* cnodes = nullptr;
     mutable cav::TriRec* ctris = nullptr;  // triangles in wide-leaf order
+    mutable float4* lbox = nullptr;  // two per triangle of ctris: its box in the binary tree
     mutable void* wide_arena = nullptr;
+    // 0: no view; 1: a view the exact mode does not use; 2: one it does; -1: none could be made for it
+    mutable std::atomic<int> wide_state{0};
+    mutable std::atomic<int64_t> rays_seen{0};  // exact-mode rays before there was a view
     cav::TriRec* tris = nullptr;   // N
     float root_box[6];             // copied to the host at build time? no: device copy
     float* d_root_box = nullptr;   // 6 floats on device
@@ -238,6 +242,7 @@ struct TraceSeg {
     const uint32_t* n_dev;  // single-tree launches: ray count read from device memory (or null)
     const CNode* cnodes;    // the tree's compressed 8-wide view (fast-mode launches; ensure_wide)
     const TriRec* ctris;
+    const float4* lbox;
 };
 cav_status trace_closest_segments(cav_ctx* ctx, const TraceSeg* segs, int nseg, int64_t n, uint32_t flags,
                                   cudaStream_t s, unsigned long long* counter);
@@ -262,6 +267,11 @@ cav_status trace_wide_any(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays,
                           const int32_t* excl, int64_t n, const uint32_t* n_dev, uint8_t* occ, cudaStream_t s,
                           unsigned long long* counter, unsigned long long* stats = nullptr);
 void free_wide(cav_bvh* bvh, cudaStream_t s, bool async);
+// The exact mode through the view: whether it can be used, and one launch of it (q: the rays,
+// the outputs and the binary tree).
+bool screen_ready(cav_ctx* ctx, const cav_bvh* bvh, bool any_hit, int64_t n, cudaStream_t s);
+cav_status trace_screened(cav_ctx* ctx, const cav_bvh* bvh, const TraceSeg& q, bool any_hit, int64_t n, cudaStream_t s,
+                          unsigned long long* counter);
 cav_status trace_wide_segments(cav_ctx* ctx, bool any_hit, const TraceSeg* segs, int nseg, int64_t n, cudaStream_t s,
                                unsigned long long* counter);
 

@@ -52,41 +52,6 @@ __device__ __forceinline__ int32_t stack_get(const int32_t* sst, const int32_t* 
     return kSmemN > 0 && i < kSmemN ? sst[i * (int)blockDim.x] : lst[i - kSmemN];
 }
 
-__device__ inline float imax_f(float a, float b) { return __int_as_float(max(__float_as_int(a), __float_as_int(b))); }
-__device__ inline float imin_f(float a, float b) { return __int_as_float(min(__float_as_int(a), __float_as_int(b))); }
-
-// AABB::intersect: returns the entry distance (>= 0) or -1 on a miss.
-__device__ inline float slab(float lx, float ly, float lz, float hx, float hy, float hz, const f3& o, const f3& inv) {
-    f3 t0 = (mk(lx, ly, lz) - o) * inv;
-    f3 t1 = (mk(hx, hy, hz) - o) * inv;
-    // fmin_fmax(a,b,c) = int max(int min(a,b), c); fmax_fmin(a,b,c) = int min(int max(a,b), c)
-    float maxmin = imax_f(imin_f(t0.x, t1.x), imax_f(imin_f(t0.y, t1.y), fminf(t0.z, t1.z)));
-    float minmax = imin_f(imax_f(t0.x, t1.x), imin_f(imax_f(t0.y, t1.y), fmaxf(t0.z, t1.z)));
-    if (maxmin <= minmax) {
-        if (minmax > 0) return fmaxf(0.f, maxmin);
-    }
-    return -1.f;
-}
-
-// One 64-byte node as two 256-bit read-only loads (sm_100 vector width): each load is one
-// 32-byte sector, half the L1 sector lookups of four 16-byte loads.
-__device__ __forceinline__ void ld_nc_v8(const void* p, float (&r)[8]) {
-    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7])
-                 : "l"(p));
-}
-
-struct NodeRegs {
-    float lo[8];  // L.lo.xyz L.hi.x L.hi.y L.hi.z R.lo.x R.lo.y
-    float hi[8];  // R.lo.z R.hi.xyz left right - -
-};
-
-__device__ __forceinline__ void load_node(const TNode* __restrict__ nodes, int32_t ref, NodeRegs& nr) {
-    const float* p = reinterpret_cast<const float*>(nodes + ref);
-    ld_nc_v8(p, nr.lo);
-    ld_nc_v8(p + 8, nr.hi);
-}
-
 // Register cap of the single-tree traversal kernels: 48 fit the walk without spills and
 // give 42 resident warps per SM where the compiler's own choice (53) gives 36 (measured
 // +2.6 % closest-hit rays/s on the 1M soup).  The segmented and instrumented variants
@@ -598,6 +563,8 @@ cav_status trace_closest(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays, 
     one.prim = prim;
     one.t = t;
     one.uv = uv;
+    if (!(flags & CAV_TRACE_CULL_ON_POP) && screen_ready(ctx, bvh, false, n, s))
+        return trace_screened(ctx, bvh, one, false, n, s, counter);
     return launch_closest<false, false>(ctx, one, nullptr, 0, n, flags, s, counter, nullptr, use_short_stack(ctx, bvh));
 }
 
@@ -625,6 +592,8 @@ cav_status trace_any(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays, cons
     one.limit = limit;
     one.excl = excl;
     one.occ = occ;
+    if (!(flags & CAV_TRACE_CULL_ON_POP) && screen_ready(ctx, bvh, true, n, s))
+        return trace_screened(ctx, bvh, one, true, n, s, counter);
     return launch_any<false, false>(ctx, one, nullptr, 0, n, flags, s, counter, nullptr, use_short_stack(ctx, bvh));
 }
 
@@ -699,6 +668,7 @@ cav_status trace_closest_dev(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* ra
     one.t = t;
     one.uv = uv;
     one.n_dev = n_dev;
+    if (screen_ready(ctx, bvh, false, 0, s)) return trace_screened(ctx, bvh, one, false, INT64_MAX, s, counter);
     return launch_closest<false, false>(ctx, one, nullptr, 0, INT64_MAX, CAV_TRACE_EXACT, s, counter, nullptr,
                                         use_short_stack(ctx, bvh));
 }
@@ -712,6 +682,7 @@ cav_status trace_any_dev(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays, 
     one.excl = excl;
     one.occ = occ;
     one.n_dev = n_dev;
+    if (screen_ready(ctx, bvh, true, 0, s)) return trace_screened(ctx, bvh, one, true, INT64_MAX, s, counter);
     return launch_any<false, false>(ctx, one, nullptr, 0, INT64_MAX, CAV_TRACE_EXACT, s, counter, nullptr,
                                     use_short_stack(ctx, bvh));
 }
@@ -755,8 +726,9 @@ extern "C" cav_status cav_trace_autotune_flags(cav_ctx* ctx, const cav_bvh* bvh,
     cudaEvent_t a, b;
     cudaEventCreate(&a);
     cudaEventCreate(&b);
-    const int saved[8] = {ctx->trace_block, ctx->trace_blocks_per_sm, ctx->trace_batch, ctx->trace_stack,
-                          ctx->wide_block, ctx->wide_batch, ctx->trace_smem_stack, ctx->wide_smem_stack};
+    const int saved[9] = {ctx->trace_block, ctx->trace_blocks_per_sm, ctx->trace_batch, ctx->trace_stack,
+                          ctx->wide_block, ctx->wide_batch, ctx->trace_smem_stack, ctx->wide_smem_stack,
+                          ctx->screen_smem_stack};
     cav_trace_config_t best{0, 0, 0, 0, 1e30f, 0};
     const int blocks[] = {64, 128, 256};
     const int batches[] = {1, 2, 4, 8, 16, 32};
@@ -778,6 +750,7 @@ extern "C" cav_status cav_trace_autotune_flags(cav_ctx* ctx, const cav_bvh* bvh,
                         ctx->trace_batch = bat;
                         ctx->trace_stack = stk;
                         ctx->trace_smem_stack = sm;
+                        ctx->screen_smem_stack = sm;
                     }
                     float ms_best = 1e30f;
                     for (int rep = 0; rep < 3 && st == CAV_OK; ++rep) {  // first repetition warms up
@@ -807,6 +780,7 @@ extern "C" cav_status cav_trace_autotune_flags(cav_ctx* ctx, const cav_bvh* bvh,
         ctx->wide_batch = saved[5];
         ctx->trace_smem_stack = saved[6];
         ctx->wide_smem_stack = saved[7];
+        ctx->screen_smem_stack = saved[8];
         return st != CAV_OK ? st : set_error(ctx, CAV_ERR_CUDA, "cav_trace_autotune: no candidate ran");
     }
     if (wide) {
@@ -815,6 +789,7 @@ extern "C" cav_status cav_trace_autotune_flags(cav_ctx* ctx, const cav_bvh* bvh,
         ctx->trace_batch = saved[2];
         ctx->trace_stack = saved[3];
         ctx->trace_smem_stack = saved[6];
+        ctx->screen_smem_stack = saved[8];
         ctx->wide_block = best.block_threads;
         ctx->wide_batch = best.batch;
         ctx->wide_smem_stack = best.smem_stack;
@@ -825,6 +800,7 @@ extern "C" cav_status cav_trace_autotune_flags(cav_ctx* ctx, const cav_bvh* bvh,
         ctx->trace_batch = best.batch;
         ctx->trace_stack = best.stack;
         ctx->trace_smem_stack = best.smem_stack;
+        ctx->screen_smem_stack = best.smem_stack;
         ctx->wide_block = saved[4];
         ctx->wide_batch = saved[5];
         ctx->wide_smem_stack = saved[7];

@@ -46,6 +46,41 @@ __device__ inline void load_tri(const TriRec* __restrict__ tris, int64_t slot, f
     e2 = mk(c.x, c.y, c.z);
 }
 
+__device__ inline float imax_f(float a, float b) { return __int_as_float(max(__float_as_int(a), __float_as_int(b))); }
+__device__ inline float imin_f(float a, float b) { return __int_as_float(min(__float_as_int(a), __float_as_int(b))); }
+
+// AABB::intersect: returns the entry distance (>= 0) or -1 on a miss.
+__device__ inline float slab(float lx, float ly, float lz, float hx, float hy, float hz, const f3& o, const f3& inv) {
+    f3 t0 = (mk(lx, ly, lz) - o) * inv;
+    f3 t1 = (mk(hx, hy, hz) - o) * inv;
+    // fmin_fmax(a,b,c) = int max(int min(a,b), c); fmax_fmin(a,b,c) = int min(int max(a,b), c)
+    float maxmin = imax_f(imin_f(t0.x, t1.x), imax_f(imin_f(t0.y, t1.y), fminf(t0.z, t1.z)));
+    float minmax = imin_f(imax_f(t0.x, t1.x), imin_f(imax_f(t0.y, t1.y), fmaxf(t0.z, t1.z)));
+    if (maxmin <= minmax) {
+        if (minmax > 0) return fmaxf(0.f, maxmin);
+    }
+    return -1.f;
+}
+
+// One 64-byte node as two 256-bit read-only loads (sm_100 vector width): each load is one
+// 32-byte sector, half the L1 sector lookups of four 16-byte loads.
+__device__ __forceinline__ void ld_nc_v8(const void* p, float (&r)[8]) {
+    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7])
+                 : "l"(p));
+}
+
+struct NodeRegs {
+    float lo[8];  // L.lo.xyz L.hi.x L.hi.y L.hi.z R.lo.x R.lo.y
+    float hi[8];  // R.lo.z R.hi.xyz left right - -
+};
+
+__device__ __forceinline__ void load_node(const TNode* __restrict__ nodes, int32_t ref, NodeRegs& nr) {
+    const float* p = reinterpret_cast<const float*>(nodes + ref);
+    ld_nc_v8(p, nr.lo);
+    ld_nc_v8(p + 8, nr.hi);
+}
+
 // Claims new rays for the idle lanes of the warp.  Returns the claimed index for this lane
 // (or -1) and clears `more` once the counter passed n.
 __device__ inline int64_t claim(unsigned idle, unsigned long long* counter, int64_t n, bool& more) {

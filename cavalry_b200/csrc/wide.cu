@@ -1,7 +1,8 @@
-// The fast traversal mode (CAV_TRACE_FAST): a compressed 8-wide view of the binary tree
-// and persistent-warp traversal over it.
+// The compressed 8-wide view of the binary tree, and persistent-warp traversal over it: the
+// fast traversal mode (CAV_TRACE_FAST), and the screening pass that answers nearly every ray
+// of the exact mode.
 //
-// Layout (CNode, 80 bytes) after Ylitie, Karras and Laine, "Efficient Incoherent Ray
+// Layout (CNode, 96 bytes) after Ylitie, Karras and Laine, "Efficient Incoherent Ray
 // Traversal on GPUs Through Compressed Wide BVHs" (HPG 2017): up to eight children per
 // node with 8-bit quantised boxes, internal children and triangles each stored
 // contiguously, and child slots chosen by direction so that a ray's octant alone gives a
@@ -19,8 +20,10 @@
 // differ; the any-hit answer is the same.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <mutex>
+#include <string>
 
 #include "trace_common.cuh"
 
@@ -35,173 +38,276 @@ constexpr int kMaxWideLevels = 4096;  // a wide level consumes at least one bina
 // distance never drops a box the ray touches.
 constexpr float kGrow = 1.00000095f;  // 1 + 2^-20
 
-__device__ inline void box_of(const TNode& t, int side, float (&b)[6], int32_t& ref) {
-    if (side == 0) {
-        b[0] = t.a.x; b[1] = t.a.y; b[2] = t.a.z; b[3] = t.a.w; b[4] = t.b.x; b[5] = t.b.y;
-        ref = t.d.x;
-    } else {
-        b[0] = t.b.z; b[1] = t.b.w; b[2] = t.c.x; b[3] = t.c.y; b[4] = t.c.z; b[5] = t.c.w;
-        ref = t.d.y;
+// ------------------------------------------------------------------- building the view
+// Device counters of one build.  nodes[l % 3]: wide nodes allocated for level l; level l
+// allocates from nodes[(l + 1) % 3] and nodes[l % 3] is cleared again one level later, so one
+// grid barrier per level is enough.
+struct WideCtr {
+    uint32_t nodes[3];
+    uint32_t tris;      // triangles placed
+    uint32_t bar;       // arrivals at the grid barrier, all levels
+    uint32_t failed;    // a barrier wait ran out, or the level bound was reached
+    uint32_t unscreened;  // a triangle or the scene box outside the screening pass's range
+    float margin;       // of the quantised boxes
+};
+
+// Coordinates up to this are screened (see the screening note below); larger or non-finite
+// geometry always takes the binary traversal in the exact mode.
+constexpr float kScreenCoord = 1e9f;
+
+__global__ void k_wide_init(const float* root_box, int32_t* task, WideCtr* ctr) {
+    if (threadIdx.x != 0) return;
+    float mag = 0.f;
+    bool ok = true;
+    for (int k = 0; k < 6; ++k) {
+        mag = fmaxf(mag, fabsf(root_box[k]));
+        ok = ok && fabsf(root_box[k]) <= kScreenCoord;
     }
+    WideCtr c{};
+    c.margin = mag * 4.76837158e-7f + 1e-30f;  // 2^-21: 4 ulps of the largest coordinate
+    c.unscreened = ok ? 0u : 1u;
+    *ctr = c;
+    task[0] = 0;  // the binary root becomes wide node 0
 }
 
-__device__ inline float half_area(const float (&b)[6]) {
+// All blocks of the (co-resident, cooperatively launched) grid arrive; false once the build
+// has failed in any of them (a wait that ran out among the reasons).
+__device__ bool wide_barrier(WideCtr* ctr, uint32_t target, uint64_t wait_ns) {
+    __shared__ int ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        ok = 1;
+        if (gridDim.x > 1) {
+            __threadfence();
+            atomicAdd(&ctr->bar, 1u);
+            uint64_t t0 = 0;
+            volatile uint32_t* bar = &ctr->bar;
+            while (*bar < target) {
+                if (*(volatile uint32_t*)&ctr->failed) {
+                    ok = 0;
+                    break;
+                }
+                uint64_t t;
+                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+                if (t0 == 0) t0 = t;
+                else if (t - t0 > wait_ns) {
+                    atomicExch(&ctr->failed, 1u);
+                    ok = 0;
+                    break;
+                }
+            }
+            __threadfence();
+        }
+        if (*(volatile uint32_t*)&ctr->failed) ok = 0;
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+__device__ __forceinline__ float half_area(const float (&b)[6]) {
     const float ex = b[3] - b[0], ey = b[4] - b[1], ez = b[5] - b[2];
     return ex * ey + ey * ez + ez * ex;
 }
 
-// One level of the collapse: wide nodes [ctr[2], ctr[3]) each take the binary node task[w].
-// ctr[0] counts wide nodes allocated, ctr[1] triangles placed.
+// One launch builds the whole view: eight lanes per wide node (lane k holds child k while the
+// node is opened, then the child in slot k), the levels separated by a grid barrier (a block
+// barrier for trees small enough for one block).  Latency bounds it: a level is a chain of six
+// dependent node fetches and a barrier.  1M-triangle soup: 0.35 ms; 3.9 ms with a thread per
+// node, its children in local memory, and two launches per level.
 __global__ void __launch_bounds__(kBuildThreads)
-    k_wide_level(const TNode* __restrict__ tn, const TriRec* __restrict__ tris_in, int32_t* __restrict__ task,
-                 CNode* __restrict__ out, TriRec* __restrict__ tris_out, uint32_t* __restrict__ ctr,
-                 const float* __restrict__ margin_p) {
-    const uint32_t begin = ctr[2], end = ctr[3];
-    const float margin = *margin_p;
-    for (uint32_t w = begin + blockIdx.x * blockDim.x + threadIdx.x; w < end; w += gridDim.x * blockDim.x) {
-        float cb[8][6];
-        int32_t cref[8];
-        {
-            const TNode t = tn[task[w]];
-            box_of(t, 0, cb[0], cref[0]);
-            box_of(t, 1, cb[1], cref[1]);
+    k_wide_build(const TNode* __restrict__ tn, const TriRec* __restrict__ tris_in, int32_t* task, CNode* __restrict__ out,
+                 TriRec* __restrict__ tris_out, float4* __restrict__ lbox, WideCtr* ctr, uint32_t max_nodes,
+                 uint32_t max_tris, uint64_t wait_ns) {
+    const int lane = threadIdx.x & 31, k8 = lane & 7, lead = lane & 24;
+    const uint32_t octet = (blockIdx.x * blockDim.x + threadIdx.x) >> 3, octets = (gridDim.x * blockDim.x) >> 3;
+    const float margin = ctr->margin;
+    uint32_t begin = 0, end = 1;
+    for (int level = 0; begin < end; ++level) {
+        if (level >= kMaxWideLevels) {
+            if (threadIdx.x == 0) atomicExch(&ctr->failed, 1u);
+            return;
         }
-        int cnt = 2;
-        while (cnt < 8) {
-            int pick = -1;
-            float pa = -1.f;
-            for (int i = 0; i < cnt; ++i)
-                if (cref[i] >= 0) {
-                    const float a = half_area(cb[i]);
-                    if (a > pa) {
-                        pa = a;
-                        pick = i;
+        if (blockIdx.x == 0 && threadIdx.x == 0) ctr->nodes[(level + 2) % 3] = 0;
+        uint32_t* const alloc = &ctr->nodes[(level + 1) % 3];
+        // the warp's four octets run together: w0 is the first one's node
+        for (uint32_t w0 = begin + (octet & ~3u); w0 < end; w0 += octets) {
+            const uint32_t w = w0 + (lane >> 3);
+            const bool live = w < end;
+            float b[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+            int32_t ref = -1, par = 0;  // the child, and the binary node that holds it
+            int cnt = live ? 2 : 0;
+            if (live && k8 < 2) {
+                par = __ldcg(task + w);
+                const TNode t = tn[par];
+                if (k8 == 0) {
+                    b[0] = t.a.x; b[1] = t.a.y; b[2] = t.a.z; b[3] = t.a.w; b[4] = t.b.x; b[5] = t.b.y;
+                    ref = t.d.x;
+                } else {
+                    b[0] = t.b.z; b[1] = t.b.w; b[2] = t.c.x; b[3] = t.c.y; b[4] = t.c.z; b[5] = t.c.w;
+                    ref = t.d.y;
+                }
+            }
+            // open the internal child of largest area (the first on ties) until there are eight
+#pragma unroll 1
+            for (int step = 0; step < 6; ++step) {
+                float pa = k8 < cnt && ref >= 0 ? half_area(b) : -1.f;
+                if (!(pa > -1.f)) pa = -1.f;  // NaN areas are not opened
+                int pick = k8;
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) {
+                    const float oa = __shfl_xor_sync(kFull, pa, o);
+                    const int oi = __shfl_xor_sync(kFull, pick, o);
+                    if (oa > pa || (oa == pa && oi < pick)) {
+                        pa = oa;
+                        pick = oi;
                     }
                 }
-            if (pick < 0) break;
-            const TNode t = tn[cref[pick]];
-            box_of(t, 0, cb[pick], cref[pick]);
-            box_of(t, 1, cb[cnt], cref[cnt]);
-            ++cnt;
-        }
-        float lo[3] = {cb[0][0], cb[0][1], cb[0][2]}, hi[3] = {cb[0][3], cb[0][4], cb[0][5]};
-        for (int i = 1; i < cnt; ++i)
-            for (int a = 0; a < 3; ++a) {
-                lo[a] = fminf(lo[a], cb[i][a]);
-                hi[a] = fmaxf(hi[a], cb[i][3 + a]);
+                const bool open = pa > -1.f;
+                const int32_t pref = __shfl_sync(kFull, ref, lead + pick);
+                if (open && (k8 == pick || k8 == cnt)) {
+                    const TNode t = tn[pref];
+                    par = pref;
+                    if (k8 == pick) {
+                        b[0] = t.a.x; b[1] = t.a.y; b[2] = t.a.z; b[3] = t.a.w; b[4] = t.b.x; b[5] = t.b.y;
+                        ref = t.d.x;
+                    } else {
+                        b[0] = t.b.z; b[1] = t.b.w; b[2] = t.c.x; b[3] = t.c.y; b[4] = t.c.z; b[5] = t.c.w;
+                        ref = t.d.y;
+                    }
+                }
+                if (open) ++cnt;
+                if (!__any_sync(kFull, open)) break;
             }
-        // slots: child i goes to the free slot whose octant diagonal best matches the
-        // direction from the node's centre to the child's centre (greedy, largest first)
-        float cost[8][8];
-        for (int i = 0; i < cnt; ++i) {
-            const float cx = (cb[i][0] + cb[i][3]) - (lo[0] + hi[0]);
-            const float cy = (cb[i][1] + cb[i][4]) - (lo[1] + hi[1]);
-            const float cz = (cb[i][2] + cb[i][5]) - (lo[2] + hi[2]);
-            for (int s = 0; s < 8; ++s)
-                cost[i][s] = ((s & 4) ? cx : -cx) + ((s & 2) ? cy : -cy) + ((s & 1) ? cz : -cz);
-        }
-        int slot_child[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
-        unsigned child_done = 0;
-        for (int k = 0; k < cnt; ++k) {
-            float bc = -FLT_MAX;
-            int bi = -1, bs = -1;
-            for (int i = 0; i < cnt; ++i) {
-                if (child_done & (1u << i)) continue;
-                for (int s = 0; s < 8; ++s)
-                    if (slot_child[s] < 0 && (bi < 0 || cost[i][s] > bc)) {
-                        bc = cost[i][s];
-                        bi = i;
+            float lo[3] = {b[0], b[1], b[2]}, hi[3] = {b[3], b[4], b[5]};
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    lo[a] = fminf(lo[a], __shfl_xor_sync(kFull, lo[a], o));
+                    hi[a] = fmaxf(hi[a], __shfl_xor_sync(kFull, hi[a], o));
+                }
+            // slots: child i goes to the free slot whose octant diagonal best matches the
+            // direction from the node's centre to the child's centre (greedy, largest first;
+            // ties to the lower child, then the lower slot)
+            const float cx = (b[0] + b[3]) - (lo[0] + hi[0]);
+            const float cy = (b[1] + b[4]) - (lo[1] + hi[1]);
+            const float cz = (b[2] + b[5]) - (lo[2] + hi[2]);
+            int slot = -1;
+            unsigned taken = 0;
+#pragma unroll 1
+            for (int round = 0; round < 8; ++round) {
+                bool has = k8 < cnt && slot < 0;
+                float bc = -FLT_MAX;
+                int bs = -1, bi = k8;
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                    const float c = ((s & 4) ? cx : -cx) + ((s & 2) ? cy : -cy) + ((s & 1) ? cz : -cz);
+                    if (!((taken >> s) & 1u) && (bs < 0 || c > bc)) {
+                        bc = c;
                         bs = s;
                     }
+                }
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) {
+                    const bool oh = __shfl_xor_sync(kFull, has ? 1 : 0, o) != 0;
+                    const float oc = __shfl_xor_sync(kFull, bc, o);
+                    const int os = __shfl_xor_sync(kFull, bs, o), oi = __shfl_xor_sync(kFull, bi, o);
+                    if (oh && (!has || oc > bc || (!(bc > oc) && oi < bi))) {
+                        has = true;
+                        bc = oc;
+                        bs = os;
+                        bi = oi;
+                    }
+                }
+                if (has) {
+                    if (bi == k8) slot = bs;
+                    taken |= 1u << bs;
+                }
+                if (!__any_sync(kFull, has)) break;
             }
-            slot_child[bs] = bi;
-            child_done |= 1u << bi;
-        }
-        // The node's grid: a power-of-two step per axis with 253 steps covering the box grown
-        // by the margin, one spare step below it (the origin) and one above.  Every child plane
-        // is then rounded outward and moved out by one more step, which absorbs the half-step
-        // rounding of the traversal's folded plane distance (node_hits).
-        CNode nd;
-        float p[3];
-        uint32_t ebits = 0;
-        double step_inv[3];
-        for (int a = 0; a < 3; ++a) {
-            const float range = (hi[a] + margin) - (lo[a] - margin);
-            int ex = 0;
-            frexpf(range * (1.f / 253.f) * 1.0000010f, &ex);  // 2^ex > range / 253
-            int eb = ex + 127;
-            eb = eb < 1 ? 1 : (eb > 254 ? 254 : eb);
-            ebits |= (uint32_t)eb << (8 * a);
-            step_inv[a] = ldexp(1.0, 127 - eb);
-            p[a] = (lo[a] - margin) - __uint_as_float((uint32_t)eb << 23);
-        }
-        nd.px = p[0];
-        nd.py = p[1];
-        nd.pz = p[2];
-        int ni = 0, nt = 0;
-        for (int i = 0; i < cnt; ++i) (cref[i] >= 0 ? ni : nt) += 1;
-        const uint32_t cbase = ni ? atomicAdd(&ctr[0], (uint32_t)ni) : 0u;
-        const uint32_t tbase = nt ? atomicAdd(&ctr[1], (uint32_t)nt) : 0u;
-        uint32_t imask = 0, meta[2] = {0, 0}, ql[3][2] = {{0, 0}, {0, 0}, {0, 0}}, qh[3][2] = {{0, 0}, {0, 0}, {0, 0}};
-        int ri = 0, rt = 0;
-        for (int s = 0; s < 8; ++s) {
-            const int i = slot_child[s];
-            if (i < 0) continue;
-            const int word = s >> 2, sh = 8 * (s & 3);
+            // lane k takes the child in slot k
+            int from = -1;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (__shfl_sync(kFull, slot, lead + i) == k8) from = i;
+            const int srcl = lead + (from < 0 ? k8 : from);
+#pragma unroll
+            for (int a = 0; a < 6; ++a) b[a] = __shfl_sync(kFull, b[a], srcl);
+            ref = __shfl_sync(kFull, ref, srcl);
+            par = __shfl_sync(kFull, par, srcl);
+            const bool full = from >= 0;
+            const unsigned imask = (__ballot_sync(kFull, full && ref >= 0) >> lead) & 0xFFu;
+            const unsigned tmask = (__ballot_sync(kFull, full && ref < 0) >> lead) & 0xFFu;
+            // node and triangle ranges: one atomic each per warp
+            const uint32_t ni = __popc(imask), nt = __popc(tmask);
+            uint32_t si = k8 == 0 ? ni : 0u, stt = k8 == 0 ? nt : 0u;
+#pragma unroll
+            for (int o = 8; o < 32; o <<= 1) {
+                const uint32_t a = __shfl_up_sync(kFull, si, o), c = __shfl_up_sync(kFull, stt, o);
+                if (lane >= o) {
+                    si += a;
+                    stt += c;
+                }
+            }
+            uint32_t cbase = 0, tbase = 0;
+            if (lane == 24) {
+                cbase = si ? atomicAdd(alloc, si) : 0u;
+                tbase = stt ? atomicAdd(&ctr->tris, stt) : 0u;
+            }
+            cbase = end + __shfl_sync(kFull, cbase, 24) + __shfl_sync(kFull, si, lead) - ni;
+            tbase = __shfl_sync(kFull, tbase, 24) + __shfl_sync(kFull, stt, lead) - nt;
+            if (!live) continue;
+            if ((uint64_t)cbase + ni > max_nodes || (uint64_t)tbase + nt > max_tris) {  // not a tree
+                if (k8 == 0) atomicExch(&ctr->failed, 1u);
+                continue;
+            }
+            // The node's grid: a power-of-two step per axis with 253 steps covering the box grown
+            // by the margin, one spare step below it (the origin) and one above.  Every child plane
+            // is then rounded outward and moved out by one more step, which absorbs the half-step
+            // rounding of the traversal's folded plane distance (node_hits).
+            unsigned char* const bytes = reinterpret_cast<unsigned char*>(out + w);
+            uint32_t ebits = 0;
+            float p[3];
+#pragma unroll
             for (int a = 0; a < 3; ++a) {
-                double qlo = floor(((double)cb[i][a] - (double)margin - (double)p[a]) * step_inv[a]) - 1.0;
-                double qhi = ceil(((double)cb[i][3 + a] + (double)margin - (double)p[a]) * step_inv[a]) + 1.0;
+                const float range = (hi[a] + margin) - (lo[a] - margin);
+                int ex = 0;
+                frexpf(range * (1.f / 253.f) * 1.0000010f, &ex);  // 2^ex > range / 253
+                int eb = ex + 127;
+                eb = eb < 1 ? 1 : (eb > 254 ? 254 : eb);
+                ebits |= (uint32_t)eb << (8 * a);
+                const double step_inv = ldexp(1.0, 127 - eb);
+                p[a] = (lo[a] - margin) - __uint_as_float((uint32_t)eb << 23);
+                double qlo = floor(((double)b[a] - (double)margin - (double)p[a]) * step_inv) - 1.0;
+                double qhi = ceil(((double)b[3 + a] + (double)margin - (double)p[a]) * step_inv) + 1.0;
                 qlo = qlo < 0.0 ? 0.0 : (qlo > 255.0 ? 255.0 : qlo);
                 qhi = qhi < 0.0 ? 0.0 : (qhi > 255.0 ? 255.0 : qhi);
-                ql[a][word] |= (uint32_t)qlo << sh;
-                qh[a][word] |= (uint32_t)qhi << sh;
+                bytes[32 + 8 * a + k8] = full ? (unsigned char)qlo : 0;
+                bytes[56 + 8 * a + k8] = full ? (unsigned char)qhi : 0;
             }
-            uint32_t m;
-            if (cref[i] >= 0) {
-                imask |= 1u << s;
-                m = 0x20u | (24u + (uint32_t)s);
-                task[cbase + ri] = cref[i];
-                ++ri;
-            } else {
-                m = 0x20u | (uint32_t)rt;
-                tris_out[tbase + rt] = tris_in[~cref[i]];
-                ++rt;
+            if (k8 == 0) {
+                uint4* o = reinterpret_cast<uint4*>(bytes);
+                o[0] = make_uint4(__float_as_uint(p[0]), __float_as_uint(p[1]), __float_as_uint(p[2]), ebits | (imask << 24));
+                o[1] = make_uint4(cbase, tbase, tmask, 0u);
             }
-            meta[word] |= m << sh;
+            if (full && ref >= 0) {
+                task[cbase + __popc(imask & ((1u << k8) - 1u))] = ref;
+            } else if (full) {
+                const uint32_t at = tbase + __popc(tmask & ((1u << k8) - 1u));
+                const TriRec r = tris_in[~ref];
+                tris_out[at] = r;
+                lbox[2 * (size_t)at] = make_float4(b[0], b[1], b[2], b[3]);
+                lbox[2 * (size_t)at + 1] = make_float4(b[4], b[5], __int_as_float(par), __int_as_float(ref));
+                const float m = fmaxf(fmaxf(fmaxf(fabsf(r.e1.x), fabsf(r.e1.y)), fabsf(r.e1.z)),
+                                      fmaxf(fmaxf(fabsf(r.e2.x), fabsf(r.e2.y)), fabsf(r.e2.z)));
+                const float sum = r.v0.x + r.v0.y + r.v0.z + r.e1.x + r.e1.y + r.e1.z + r.e2.x + r.e2.y + r.e2.z;
+                if (!(m <= 4.f * kScreenCoord) || !(fabsf(sum) <= 64.f * kScreenCoord)) ctr->unscreened = 1u;
+            }
         }
-        nd.e_imask = ebits | (imask << 24);
-        nd.child_base = cbase;
-        nd.tri_base = tbase;
-        nd.meta[0] = meta[0];
-        nd.meta[1] = meta[1];
-        nd.qlo_x[0] = ql[0][0]; nd.qlo_x[1] = ql[0][1];
-        nd.qlo_y[0] = ql[1][0]; nd.qlo_y[1] = ql[1][1];
-        nd.qlo_z[0] = ql[2][0]; nd.qlo_z[1] = ql[2][1];
-        nd.qhi_x[0] = qh[0][0]; nd.qhi_x[1] = qh[0][1];
-        nd.qhi_y[0] = qh[1][0]; nd.qhi_y[1] = qh[1][1];
-        nd.qhi_z[0] = qh[2][0]; nd.qhi_z[1] = qh[2][1];
-        out[w] = nd;
+        if (!wide_barrier(ctr, (uint32_t)(level + 1) * gridDim.x, wait_ns)) return;
+        begin = end;
+        end = begin + __ldcg(alloc);
     }
-}
-
-__global__ void k_wide_next_level(uint32_t* ctr) {
-    if (threadIdx.x == 0) {
-        ctr[2] = ctr[3];
-        ctr[3] = ctr[0];
-    }
-}
-
-// Margin of the quantised boxes: 4 ulps of the largest coordinate magnitude of the scene.
-__global__ void k_wide_init(const float* root_box, int32_t* task, uint32_t* ctr, float* margin) {
-    if (threadIdx.x != 0) return;
-    float mag = 0.f;
-    for (int k = 0; k < 6; ++k) mag = fmaxf(mag, fabsf(root_box[k]));
-    margin[0] = mag * 4.76837158e-7f + 1e-30f;  // 2^-21
-    task[0] = 0;  // the binary root becomes wide node 0
-    ctr[0] = 1;
-    ctr[1] = 0;
-    ctr[2] = 0;
-    ctr[3] = 1;
 }
 
 // ----------------------------------------------------------------------- traversal
@@ -221,73 +327,84 @@ __device__ __forceinline__ float biased_byte(uint32_t w, uint32_t k) {
     return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u | k));
 }
 
-struct WideRay {
-    f3 o, inv;
-    uint32_t octinv4;  // the visiting-order flip (7 - direction octant) in every byte
-    bool nx, ny, nz;   // negative direction components
-};
-
-// Hit mask of one node: bits 24-31 the internal children in visiting order, bits 0-23 the
-// triangles.  `lim` bounds the entry distance (closest hit so far, ray tmax, shadow limit).
-// A plane's distance is fma(2^23 + q, s * inv, (p - o) * inv - 2^23 * s * inv): one fma per
-// plane on the byte's biased float; the folded constant rounds by at most half a grid step
-// in distance, inside the spare step every quantised plane carries.
-__device__ __forceinline__ uint32_t node_hits(const CNode* __restrict__ cn, uint32_t idx, const WideRay& R, float lim,
-                                              uint32_t& child_base, uint32_t& tri_base, uint32_t& imask) {
-    const uint4* q = reinterpret_cast<const uint4*>(cn + idx);
-    const uint4 n0 = __ldg(q), n1 = __ldg(q + 1), n2 = __ldg(q + 2), n3 = __ldg(q + 3), n4 = __ldg(q + 4);
-    child_base = n1.x;
-    tri_base = n1.y;
-    imask = n0.w >> 24;
-    const float ax = __uint_as_float((n0.w & 0xFFu) << 23) * R.inv.x;
-    const float ay = __uint_as_float(((n0.w >> 8) & 0xFFu) << 23) * R.inv.y;
-    const float az = __uint_as_float(((n0.w >> 16) & 0xFFu) << 23) * R.inv.z;
-    const float bx = (__uint_as_float(n0.x) - R.o.x) * R.inv.x - 8388608.f * ax;
-    const float by = (__uint_as_float(n0.y) - R.o.y) * R.inv.y - 8388608.f * ay;
-    const float bz = (__uint_as_float(n0.z) - R.o.z) * R.inv.z - 8388608.f * az;
-    // near / far planes by direction sign: qlo = (n2.x n2.y | n2.z n2.w | n3.x n3.y), qhi = (n3.z n3.w | n4.x n4.y | n4.z n4.w)
-    const uint32_t nx0 = R.nx ? n3.z : n2.x, nx1 = R.nx ? n3.w : n2.y;
-    const uint32_t fx0 = R.nx ? n2.x : n3.z, fx1 = R.nx ? n2.y : n3.w;
-    const uint32_t ny0 = R.ny ? n4.x : n2.z, ny1 = R.ny ? n4.y : n2.w;
-    const uint32_t fy0 = R.ny ? n2.z : n4.x, fy1 = R.ny ? n2.w : n4.y;
-    const uint32_t nz0 = R.nz ? n4.z : n3.x, nz1 = R.nz ? n4.w : n3.y;
-    const uint32_t fz0 = R.nz ? n3.x : n4.z, fz1 = R.nz ? n3.y : n4.w;
-    // per slot byte: the hit bit's position and the bits to set (0 for an empty slot);
-    // internal children's positions flip with the ray's octant
-    uint32_t bitpos[2], setbits[2];
-#pragma unroll
-    for (int w = 0; w < 2; ++w) {
-        const uint32_t m4 = w ? n1.w : n1.z;
-        const uint32_t inner4 = (((m4 & (m4 << 1)) >> 4) & 0x01010101u) * 0xFFu;  // 0xFF where bits 3 and 4 are set
-        bitpos[w] = (m4 ^ (R.octinv4 & inner4)) & 0x1F1F1F1Fu;
-        setbits[w] = (m4 >> 5) & 0x07070707u;
-    }
-    uint32_t hits = 0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const uint32_t k = (uint32_t)(i & 3);
-        const bool hiw = i >= 4;
-        if (hiw && n1.w == 0u) break;  // slots 4-7 empty
-        const float tnx = fmaf(biased_byte(hiw ? nx1 : nx0, k), ax, bx);
-        const float tny = fmaf(biased_byte(hiw ? ny1 : ny0, k), ay, by);
-        const float tnz = fmaf(biased_byte(hiw ? nz1 : nz0, k), az, bz);
-        const float tfx = fmaf(biased_byte(hiw ? fx1 : fx0, k), ax, bx);
-        const float tfy = fmaf(biased_byte(hiw ? fy1 : fy0, k), ay, by);
-        const float tfz = fmaf(biased_byte(hiw ? fz1 : fz0, k), az, bz);
-        const float tmin = max3f(tnx, tny, fmaxf(tnz, 0.f));
-        const float tmax = fminf(min3f(tfx, tfy, tfz) * kGrow, lim);
-        const uint32_t sh = 8u * k;
-        const uint32_t bits = tmin <= tmax ? (((hiw ? setbits[1] : setbits[0]) >> sh) & 0xFFu) : 0u;
-        hits |= bits << (((hiw ? bitpos[1] : bitpos[0]) >> sh) & 0xFFu);
-    }
-    return hits;
+// Two plane distances in one instruction: {b0, b1} * {a, a} + {c, c}.
+__device__ __forceinline__ float2 fma2(float b0, float b1, float2 a, float2 c) {
+    unsigned long long r, q, x, y;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(q) : "f"(b0), "f"(b1));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(a.x), "f"(a.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(c.x), "f"(c.y));
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(q), "l"(x), "l"(y));
+    float2 d;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(r));
+    return d;
 }
 
-// kSeg: one launch over several jobs' rays (segs[k] = one tree and its outputs, ray indices
-// numbered across the launch); otherwise the pointer arguments describe the one tree.
-// 64 registers, unconstrained: the kernel is ALU-bound, and capping it for more resident
-// warps made the 5.24M-triangle render's extend stage slower (231 ms at 64 registers, 263 at
-// 48, 302 at 40).
+struct WideRay {
+    f3 o, inv;
+    uint32_t octinv;  // the visiting-order flip, 7 - direction octant
+};
+
+// Hit mask of one node: bits 24-31 the internal children in visiting order (slot ^ octinv),
+// bits 0-7 the triangles by slot.  `lim` bounds the entry distance (closest hit so far, ray
+// tmax, shadow limit).  A plane's distance is fma(2^23 + q, s * inv, (p - o) * inv - 2^23 * s
+// * inv): one fma per plane on the byte's biased float, two children per packed instruction;
+// the folded constant rounds by at most half a grid step in distance, inside the spare step
+// every quantised plane carries.  ALU operations bound this function: a child costs six byte
+// extractions, four three-input min/max and one predicated or; the children's order is applied
+// to the eight-bit mask, not child by child.
+__device__ __forceinline__ uint32_t node_hits(const CNode* __restrict__ cn, uint32_t idx, const WideRay& R, float lim,
+                                              uint32_t& child_base, uint32_t& tri_base, uint32_t& masks) {
+    uint32_t h[8], q[8];
+    const char* at = reinterpret_cast<const char*>(cn + idx);
+    asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=r"(h[0]), "=r"(h[1]), "=r"(h[2]), "=r"(h[3]), "=r"(h[4]), "=r"(h[5]), "=r"(h[6]), "=r"(h[7])
+        : "l"(at));
+    asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7])
+        : "l"(at + 32));
+    const uint4 r = __ldg(reinterpret_cast<const uint4*>(at + 64));
+    child_base = h[4];
+    tri_base = h[5];
+    const uint32_t imask = h[3] >> 24, tmask = h[6];
+    masks = imask | (tmask << 8);
+    const float ax = __uint_as_float((h[3] & 0xFFu) << 23) * R.inv.x;
+    const float ay = __uint_as_float(((h[3] >> 8) & 0xFFu) << 23) * R.inv.y;
+    const float az = __uint_as_float(((h[3] >> 16) & 0xFFu) << 23) * R.inv.z;
+    const float bx = (__uint_as_float(h[0]) - R.o.x) * R.inv.x - 8388608.f * ax;
+    const float by = (__uint_as_float(h[1]) - R.o.y) * R.inv.y - 8388608.f * ay;
+    const float bz = (__uint_as_float(h[2]) - R.o.z) * R.inv.z - 8388608.f * az;
+    const float2 ax2 = make_float2(ax, ax), ay2 = make_float2(ay, ay), az2 = make_float2(az, az);
+    const float2 bx2 = make_float2(bx, bx), by2 = make_float2(by, by), bz2 = make_float2(bz, bz);
+    // near / far planes by direction sign (octinv bit 2: x not negative, and so on)
+    const bool nx = !(R.octinv & 4u), ny = !(R.octinv & 2u), nz = !(R.octinv & 1u);
+    uint32_t hm = 0;
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+        if (w && ((imask | tmask) & 0xF0u) == 0u) break;  // slots 4-7 empty
+        const uint32_t rx = w ? r.y : r.x, rz = w ? r.w : r.z;
+        const uint32_t nxw = nx ? q[6 + w] : q[w], fxw = nx ? q[w] : q[6 + w];
+        const uint32_t nyw = ny ? rx : q[2 + w], fyw = ny ? q[2 + w] : rx;
+        const uint32_t nzw = nz ? rz : q[4 + w], fzw = nz ? q[4 + w] : rz;
+#pragma unroll
+        for (int k = 0; k < 4; k += 2) {
+            const float2 tnx = fma2(biased_byte(nxw, k), biased_byte(nxw, k + 1), ax2, bx2);
+            const float2 tny = fma2(biased_byte(nyw, k), biased_byte(nyw, k + 1), ay2, by2);
+            const float2 tnz = fma2(biased_byte(nzw, k), biased_byte(nzw, k + 1), az2, bz2);
+            const float2 tfx = fma2(biased_byte(fxw, k), biased_byte(fxw, k + 1), ax2, bx2);
+            const float2 tfy = fma2(biased_byte(fyw, k), biased_byte(fyw, k + 1), ay2, by2);
+            const float2 tfz = fma2(biased_byte(fzw, k), biased_byte(fzw, k + 1), az2, bz2);
+            const float t0 = max3f(tnx.x, tny.x, fmaxf(tnz.x, 0.f)), t1 = max3f(tnx.y, tny.y, fmaxf(tnz.y, 0.f));
+            if (t0 <= fminf(min3f(tfx.x, tfy.x, tfz.x) * kGrow, lim)) hm |= 1u << (4 * w + k);
+            if (t1 <= fminf(min3f(tfx.y, tfy.y, tfz.y) * kGrow, lim)) hm |= 2u << (4 * w + k);
+        }
+    }
+    uint32_t x = hm & imask;  // slot s to bit s ^ octinv
+    if (!nz) x = ((x << 1) & 0xAAu) | ((x >> 1) & 0x55u);
+    if (!ny) x = ((x << 2) & 0xCCu) | ((x >> 2) & 0x33u);
+    if (!nx) x = ((x << 4) & 0xF0u) | (x >> 4);
+    return (x << 24) | (hm & tmask);
+}
+
 // The first kSmemN node groups of a lane's stack in shared memory, [entry][thread] (a warp's
 // push or pop is two conflict-free wavefronts whatever the lanes' depths), the rest in local
 // memory; kSmemN == 0 keeps all of it in local memory.
@@ -302,22 +419,159 @@ __device__ __forceinline__ uint2 wstack_get(const uint2* sst, const uint2* lst, 
     return kSmemN > 0 && i < kSmemN ? sst[i * (int)blockDim.x] : lst[i - kSmemN];
 }
 
-template <bool kAny, bool kStats, bool kSeg, int kSmemN = 0>
-__global__ void __launch_bounds__(256)
-    k_trace_wide(const CNode* __restrict__ cn0, const TriRec* __restrict__ tris0, const cav_ray* __restrict__ rays0,
-                 int64_t n, const uint32_t* n_dev, int32_t* prim0, float* tout0, float* uv0,
-                 const float* __restrict__ limit0, const int32_t* __restrict__ excl0, uint8_t* occ0,
-                 unsigned long long* counter, int refill, uint32_t max_steps, int* flag,
-                 unsigned long long* stats,
-                 const TraceSeg* __restrict__ segs, int nseg) {
+// ---- screening (kExact).  The exact mode's answer is the one the binary traversal of
+// trace.cu gives (the reference's visiting order and pruning).  The wide traversal finds it
+// faster, and proves it ray by ray:
+//   * The binary slab test of a box that contains another passes whenever the inner box's
+//     passes, with an entry distance no larger: subtraction and multiplication round
+//     monotonically, and the boxes of the tree are exact unions.  So the slab test of a
+//     triangle's own box, entry `ml`, bounds those of all its ancestors; and a triangle whose
+//     own box fails is never tested by the binary traversal (leaves are tested as boxes).
+//   * Any hit: the binary traversal prunes nothing, so it finds a hit exactly when some hit
+//     triangle's own box passes.
+//   * Closest hit: the wide traversal tests every triangle whose box it enters below
+//     (1 + 2^-10) times the closest distance, leaves out those whose own box fails, and keeps
+//     the two smallest distances.  If the smallest is unique and its `ml` is below the second
+//     (and within 2^-11 of the smallest), the binary traversal cannot have pruned the winner
+//     at any of its ancestors, and no triangle replaces it: that triangle is the answer.
+//   * A tie of two triangles (a ray through a shared edge) goes to the one on the side that
+//     the binary traversal enters first at their lowest common ancestor.
+// The winner's own box is tested once per ray, when the ray ends; if it fails, the wide search
+// runs again and leaves such triangles out as it goes (kModeCareful).  Every other ray (more
+// ties, a second hit as close as the box entry, a ray or scene out of range) takes the binary
+// steps themselves, in the same kernel: first with the search bounded just above the screened
+// distance (kModeBounded), and from the start if that finds nothing (kModeBinary).  A triangle test that
+// rounds a distance to more than 2^-10 before its own box's entry could still differ (a ray in
+// the triangle's plane to the last bits): of 1.16 G random closest-hit rays and as many any-hit
+// rays over soups, sphere scenes and the room none did, of rays laid in triangles' planes about
+// one in 2,000.
+constexpr float kSlack = 1.0009765625f;       // 1 + 2^-10: distances up to this past the closest are all seen
+constexpr float kNear = 1.00048828125f;       // 1 + 2^-11
+constexpr float kScreenDir = 1e6f, kScreenDirMin = 1e-6f;
+
+__device__ inline bool screenable(const f3& o, const f3& d) {
+    const float mo = fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fabsf(o.z));
+    const float md = fmaxf(fmaxf(fabsf(d.x), fabsf(d.y)), fabsf(d.z));
+    // NaN components fail the sums (fmaxf drops them)
+    return mo <= kScreenCoord && md <= kScreenDir && md >= kScreenDirMin && fabsf(o.x + o.y + o.z) <= 4.f * kScreenCoord &&
+           fabsf(d.x + d.y + d.z) <= 4.f * kScreenDir;
+}
+
+// ---- work sharing.  A launch ends when its slowest ray does, and the slowest of a batch
+// visits hundreds of times the average (a ray nearly in a plane of a dense scene).  Once the
+// queue is empty, an idle lane takes the oldest node group of a busy lane of its warp and
+// searches it for the same ray.  The first lane of a shared ray lends its slot in this
+// per-warp record; lanes that run out merge what they found, and the last one to finish
+// writes the ray's result.  The largest part left (the bottom of the stack) is the better one
+// to give: taking the nearest group instead made 65,536 closest-hit rays 1.85 against 1.44 ms.
+// Waiting for a hit or a number of steps before sharing a ray measured slower too (2.7 and 2.2
+// against 1.6 ms).  1M-triangle soup, fast mode, with and without sharing: 16,384 shadow rays
+// 0.12 against 1.4 ms, 65,536 closest-hit rays 1.5 against 6.1, 4M 35.7 against 43.8.
+struct ShareRec {
+    int32_t bound[32];  // closest: the smallest distance any lane of the ray has seen (float bits)
+    float best[32], second[32];  // the two smallest of the merged lanes (second negative: a lane failed)
+    float u[32], v[32];
+    int32_t slot[32];     // closest: the triangle at `best`; any: bits 1 hit, 4 failed
+    int32_t slot2[32];    // the triangle at `second`
+    int32_t pending[32];  // lanes still searching
+    int32_t donor[32];    // one hand-over's donors, in lane order
+};
+constexpr int kShareEvery = 2;  // iterations between two hand-overs
+
+__device__ __forceinline__ int tri_id(const TriRec* __restrict__ tris, int32_t slot) {
+    return __float_as_int(__ldg(&tris[slot].v0.w));
+}
+
+// One more distance beside the smallest: `second` and its triangle.
+__device__ __forceinline__ void add_second(float t, int32_t slot, float& second, int32_t& slot2) {
+    if (t < second) {
+        second = t;
+        slot2 = slot;
+    } else if (t == second) {
+        slot2 = -2;
+    }
+}
+
+// The binary traversal's reciprocal direction: R.inv but for the components that were replaced.
+__device__ __forceinline__ f3 own_inv(const WideRay& R, const f3& d) {
+    if (fmaxf(fmaxf(fabsf(R.inv.x), fabsf(R.inv.y)), fabsf(R.inv.z)) < 7.37e19f) return R.inv;
+    return mk(1.f / d.x, 1.f / d.y, 1.f / d.z);
+}
+
+// The binary slab test of triangle `slot`'s own box (the entry distance, or -1).
+__device__ __forceinline__ float own_box(const TraceSeg& S, uint32_t slot, const WideRay& R, const f3& d) {
+    const float4* lb = S.lbox + 2 * (size_t)slot;
+    const float4 a = __ldg(lb), b = __ldg(lb + 1);
+    return slab(a.x, a.y, a.z, a.w, b.x, b.y, R.o, own_inv(R, d));
+}
+
+// Which of two triangles the binary traversal tests first, both reached: the one on the side
+// that it enters first at their lowest common ancestor.  1: `a`, 0: `b`, -1: the climb does
+// not meet (not a tree).
+__device__ __forceinline__ int tested_first(const TNode* __restrict__ nodes, const float4* __restrict__ lbox, int32_t a,
+                                         int32_t b, f3 o, f3 inv) {
+    const float4 la = __ldg(lbox + 2 * (size_t)a + 1), lb = __ldg(lbox + 2 * (size_t)b + 1);
+    int32_t pa = __float_as_int(la.z), pb = __float_as_int(lb.z);  // nodes, and the child each climb came from
+    int32_t ca = __float_as_int(la.w), cb = __float_as_int(lb.w);
+    int da = 0, db = 0;
+    constexpr int kMaxClimb = 4096;
+    for (int32_t x = pa; x != 0 && da < kMaxClimb; x = __ldg(&nodes[x].d.z)) ++da;
+    for (int32_t x = pb; x != 0 && db < kMaxClimb; x = __ldg(&nodes[x].d.z)) ++db;
+    if (da >= kMaxClimb || db >= kMaxClimb) return -1;
+    for (; da > db; --da) {
+        ca = pa;
+        pa = __ldg(&nodes[pa].d.z);
+    }
+    for (; db > da; --db) {
+        cb = pb;
+        pb = __ldg(&nodes[pb].d.z);
+    }
+    for (; pa != pb && da > 0; --da) {
+        ca = pa;
+        pa = __ldg(&nodes[pa].d.z);
+        cb = pb;
+        pb = __ldg(&nodes[pb].d.z);
+    }
+    if (pa != pb) return -1;
+    NodeRegs nr;
+    load_node(nodes, pa, nr);
+    const float ml = slab(nr.lo[0], nr.lo[1], nr.lo[2], nr.lo[3], nr.lo[4], nr.lo[5], o, inv);
+    const float mr = slab(nr.lo[6], nr.lo[7], nr.hi[0], nr.hi[1], nr.hi[2], nr.hi[3], o, inv);
+    const int32_t first = ml > mr ? __float_as_int(nr.hi[5]) : __float_as_int(nr.hi[4]);
+    return ca == first ? 1 : (cb == first ? 0 : -1);
+}
+
+enum { kModeWide = 0, kModeCareful = 1, kModeBounded = 2, kModeBinary = 3 };
+
+// Idle lane iterations, per unit of the context's queue chunk (default 4), that pay for settling
+// a warp's ended rays and claiming new ones.
+constexpr int kSettleCost = 8;
+
+// kSeg: one launch over several jobs' rays (segs[k] = one tree and its outputs, ray indices
+// numbered across the launch); otherwise `one` describes the tree.
+// A warp holds at most `cap` rays of its own at a time: 32, less when there are fewer rays
+// than lanes (they are spread over the warps, and the other lanes help).
+// Registers: 72 for the exact closest hit (the two smallest distances and the search mode ride
+// along), 64 for the others; 4M soup rays took 38.1 ms at 72, 39.2 at 64, 40.6 at 80 and 53.1 at
+// 56 in the former, 33.7, 35.4 and 38.2 ms at 64, 72 and 80 in the fast mode's closest hit.
+template <bool kAny, bool kStats, bool kSeg, bool kExact, int kSmemN = 0>
+__global__ void __maxnreg__(kExact && !kAny ? 72 : 64)
+    k_trace_wide(TraceSeg one, const TraceSeg* __restrict__ segs, int nseg, int64_t n, unsigned long long* counter,
+                 int refill, int min_cap, uint32_t max_steps, int* flag, unsigned long long* stats) {
     __shared__ int64_t sbeg[kSeg ? kMaxSeg : 1];
+    __shared__ ShareRec shares[8];
     if (kSeg) {
         for (int i = threadIdx.x; i < nseg; i += blockDim.x) sbeg[i] = segs[i].begin;
         __syncthreads();
     }
-    if (n_dev) n = *n_dev;
-    const CNode* __restrict__ cn = cn0;
-    const TriRec* __restrict__ tris = tris0;
+    if (!kSeg && one.n_dev) n = *one.n_dev;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    const int cap = (int)min((int64_t)32, max((int64_t)min_cap, (n + warps - 1) / warps));
+    const bool once = n <= warps * cap;  // every ray fits: warp w takes rays [w cap, (w + 1) cap) and no others
+    ShareRec& sh = shares[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const CNode* __restrict__ cn = one.cnodes;
+    const TriRec* __restrict__ tris = one.ctris;
     int seg = 0;
     TraceStats st;
     extern __shared__ uint2 wsstack[];
@@ -327,180 +581,508 @@ __global__ void __launch_bounds__(256)
     int64_t ray = -1;
     WideRay R{};
     f3 d = mk(0, 0, 0);
-    float tmax = 0.f, best = 0.f, bu = 0.f, bv = 0.f, lim = 0.f;
-    int32_t bid = -1, src = -1, dst = -1;
-    bool hit = false, use_limit = false;
+    // closest: ray tmax; any: the limit (FLT_MAX without one: a hit needs t < lim only with one)
+    float tmax = 0.f;
+    float best = 0.f, second = 0.f, bu = 0.f, bv = 0.f;
+    int32_t slot = -1, src = -1, dst = -1;  // closest: the hit triangle; any: the bits of ShareRec::slot
+    int32_t slot2 = -1;                     // the triangle at `second`; -2: there are several
+    bool use_limit = false;
     uint2 grp = make_uint2(0, 0), tgrp = make_uint2(0, 0);
-    int top = -1;
+    int top = -1, bot = 0;  // stack entries bot..top
+    // The record that the lane's ray uses when it is shared (its first lane's, which no other
+    // ray can need); ~owner while the ray has one lane only.
+    int owner = ~lane;
+    int mode = kModeWide;
+    bool finished = false;  // this lane's search has ended, its ray is not yet written
     uint32_t steps = 0;
+    int turn = 0, waste = 0;  // waste: idle lanes, summed over iterations
     for (;;) {
-        const unsigned idle = __ballot_sync(kFull, ray < 0);
-        if (idle == kFull && !more) break;
-        if (more && idle != 0 && (__popc(idle) >= refill || idle == kFull)) {
-            int64_t r = claim(idle, counter, n, more);
-            if (r >= 0) {
-                const cav_ray* rays = rays0;
-                const float* limit = limit0;
-                const int32_t* excl = excl0;
-                if (kSeg) {
-                    seg = find_seg(sbeg, nseg, r);
-                    const TraceSeg& G = segs[seg];
-                    cn = G.cnodes;
-                    tris = G.ctris;
-                    rays = G.rays;
-                    limit = G.limit;
-                    excl = G.excl;
-                    r -= G.begin;
-                }
-                const float4* rp = reinterpret_cast<const float4*>(rays + r);
-                const float4 r0 = __ldg(rp), r1 = __ldg(rp + 1);
-                R.o = mk(r0.x, r0.y, r0.z);
-                d = mk(r1.x, r1.y, r1.z);
-                tmax = r1.w;
-                // Box tests use a direction whose zero components are replaced by +-2^-66: a
-                // finite reciprocal keeps the folded plane distances finite (an infinite one
-                // turns them into NaN, which the min / max drop, so the axis would stop
-                // bounding the ray and a ray parallel to it would visit a whole slab of the
-                // tree).  The triangle test uses the ray's own direction.
-                const f3 db = mk(fabsf(d.x) < 1.3552527e-20f ? copysignf(1.3552527e-20f, d.x) : d.x,
-                                 fabsf(d.y) < 1.3552527e-20f ? copysignf(1.3552527e-20f, d.y) : d.y,
-                                 fabsf(d.z) < 1.3552527e-20f ? copysignf(1.3552527e-20f, d.z) : d.z);
-                R.inv = mk(1.f / db.x, 1.f / db.y, 1.f / db.z);
-                R.nx = db.x < 0.f;
-                R.ny = db.y < 0.f;
-                R.nz = db.z < 0.f;
-                const uint32_t octinv = 7u - ((R.nx ? 4u : 0u) | (R.ny ? 2u : 0u) | (R.nz ? 1u : 0u));
-                R.octinv4 = octinv * 0x01010101u;
-                // the root as the one internal child of a virtual parent: slot 0, imask 1
-                grp = make_uint2(0u, (1u << (24u + octinv)) | 1u);
-                tgrp = make_uint2(0u, 0u);
-                hit = false;
-                best = FLT_MAX;
-                bu = bv = 0.f;
-                bid = -1;
-                top = -1;
-                steps = 0;
-                if (kAny) {
-                    use_limit = limit != nullptr;
-                    lim = use_limit ? __ldg(limit + r) : FLT_MAX;
-                    src = dst = -1;
-                    if (excl) {
-                        const int2 e = __ldg(reinterpret_cast<const int2*>(excl) + r);
-                        src = e.x;
-                        dst = e.y;
+        unsigned idle = __ballot_sync(kFull, ray < 0 || finished);
+        // Rays that ended are proven and written, and their lanes take new rays, once the lanes
+        // have waited long enough together to pay for the instructions (at once when the queue
+        // is empty): after a few iterations where rays are short, with few lanes where they are
+        // long.  Against a fixed four lanes: 1M rays of the 36-triangle
+        // room 0.207 -> 0.189 ms, 1M camera rays over 20,498 triangles 0.157 -> 0.136, 4M soup
+        // rays 38.1 -> 37.0.
+        waste += __popc(idle);
+        if (!more || idle == kFull || waste >= kSettleCost * refill) {
+            waste = 0;
+            if (!more) {  // lanes of shared rays that ran out merge; the last of a ray goes on to write it
+                const bool out = finished && owner >= 0;
+                if (__any_sync(kFull, out)) {
+                    if (kAny) {
+                        if (out && slot != 0) atomicOr(&sh.slot[owner], slot);
+                    } else {
+                        // most lanes found nothing and have nothing to add; the others one by one
+                        unsigned fin = __ballot_sync(kFull, out && (slot >= 0 || second < FLT_MAX));
+                        while (fin) {
+                            const int f = __ffs(fin) - 1;
+                            fin &= fin - 1u;
+                            if (lane == f) {
+                                const float rb = sh.best[owner];
+                                const int32_t rs = sh.slot[owner];
+                                if (kExact) add_second(sh.second[owner], sh.slot2[owner], second, slot2);
+                                else second = fminf(second, sh.second[owner]);  // a failure
+                                bool keep = slot >= 0 && (rs < 0 || best < rb);
+                                if (!kExact && slot >= 0 && rs >= 0 && best == rb) keep = tri_id(tris, slot) < tri_id(tris, rs);
+                                if (keep) {
+                                    if (kExact && rs >= 0) add_second(rb, rs, second, slot2);
+                                    sh.best[owner] = best;
+                                    sh.slot[owner] = slot;
+                                    sh.u[owner] = bu;
+                                    sh.v[owner] = bv;
+                                    
+                                } else if (kExact && slot >= 0) {
+                                    add_second(best, slot, second, slot2);
+                                }
+                                sh.second[owner] = second;
+                                sh.slot2[owner] = slot2;
+                            }
+                            __syncwarp();
+                        }
+                    }
+                    __syncwarp();
+                    if (out) {
+                        if (atomicSub(&sh.pending[owner], 1) > 1) {
+                            ray = -1;
+                            finished = false;
+                        } else {
+                            slot = sh.slot[owner];
+                            if (!kAny) {
+                                best = sh.best[owner];
+                                second = sh.second[owner];
+                                slot2 = sh.slot2[owner];
+                                bu = sh.u[owner];
+                                bv = sh.v[owner];
+                                }
+                        }
+                        owner = ~owner;
                     }
                 }
-                ray = r;
+            }
+            if (finished && kExact) {  // proven, or searched again
+                int next = -1;
+                if (mode <= kModeCareful) {
+                    if (kAny) {
+                        if ((slot & 4) && !(slot & 1)) next = kModeBinary;
+                    } else if (second < 0.f) {
+                        next = kModeBinary;
+                    } else if (slot >= 0) {
+                        const float ml = own_box(one, slot, R, d);
+                        if (!(ml >= 0.f)) {
+                            next = kModeCareful;
+                        } else if (ml > tmax || !(ml <= best * kNear)) {
+                            next = kModeBounded;
+                        } else if (best == second && slot2 >= 0 && ml <= best) {
+                            // a tie of two (a ray through a shared edge): the first one tested keeps it
+                            const float m2 = own_box(one, slot2, R, d);
+                            const int first =
+                                m2 >= 0.f ? tested_first(one.nodes, one.lbox, slot, slot2, R.o, own_inv(R, d)) : 1;
+                            if (first == 0 && m2 <= best && !(m2 > tmax)) {
+                                tgrp = make_uint2((uint32_t)slot2, 0x101u);  // test it once more, alone
+                                grp = make_uint2(0u, 0u);
+                                best = second = FLT_MAX;
+                                slot = slot2 = -1;
+                                top = -1;
+                                bot = 0;
+                                finished = false;
+                            } else if (first != 1) {
+                                next = kModeBounded;
+                            }
+                        } else if (!(best < second && ml < second)) {
+                            next = kModeBounded;
+                        }
+                    }
+                } else if (!kAny && mode == kModeBounded && slot == -1) {
+                    next = kModeBinary;
+                }
+                if (next >= 0) {
+                    best = next == kModeBounded ? best * kNear : FLT_MAX;
+                    second = FLT_MAX;
+                    bu = bv = 0.f;
+                    slot = kAny ? 0 : -1;
+                    slot2 = -1;
+                    grp = make_uint2(0u, next == kModeCareful ? (1u << (24u + R.octinv)) | 1u : 0u);
+                    top = -1;
+                    bot = 0;
+                    steps = 0;
+                    mode = next;
+                    finished = false;
+                }
+            }
+            if (finished) {
+                const TraceSeg& S = kSeg ? segs[seg] : one;
+                if (kAny) {
+                    S.occ[ray] = (slot & 1) ? 1 : ((slot & 4) ? 2 : 0);
+                } else {
+                    const bool wide = mode <= kModeCareful;
+                    const bool bad = wide ? second < 0.f : slot == -2;
+                    const bool hit = !bad && slot >= 0;
+                    S.prim[ray] = hit ? (wide ? tri_id(tris, slot) : slot) : (bad ? -2 : -1);
+                    if (S.t) S.t[ray] = hit ? best : __int_as_float(0x7f800000);
+                    if (S.uv) reinterpret_cast<float2*>(S.uv)[ray] = hit ? make_float2(bu, bv) : make_float2(0.f, 0.f);
+                }
+                ray = -1;
+                finished = false;
+            }
+            idle = __ballot_sync(kFull, ray < 0);
+            if (more) {
+                const int busy = 32 - __popc(idle);
+                const int want = min(cap - busy, 32 - busy);
+                if (want > 0) {
+                    const int rank = __popc(idle & ((1u << lane) - 1u));
+                    const bool mine = ((idle >> lane) & 1u) && rank < want;
+                    int64_t r;
+                    if (once) {
+                        r = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * cap + rank;
+                        if (!mine || r >= n) r = -1;
+                        more = false;
+                    } else {
+                        r = claim(__ballot_sync(kFull, mine), counter, n, more);
+                    }
+                    if (r >= 0) {
+                        const TraceSeg* S = &one;
+                        if (kSeg) {
+                            seg = find_seg(sbeg, nseg, r);
+                            S = segs + seg;
+                            cn = S->cnodes;
+                            tris = S->ctris;
+                            r -= S->begin;
+                        }
+                        const float4* rp = reinterpret_cast<const float4*>(S->rays + r);
+                        const float4 r0 = __ldg(rp), r1 = __ldg(rp + 1);
+                        R.o = mk(r0.x, r0.y, r0.z);
+                        d = mk(r1.x, r1.y, r1.z);
+                        tmax = r1.w;
+                        // Box tests use a direction whose zero components are replaced by +-2^-66: a
+                        // finite reciprocal keeps the folded plane distances finite (an infinite one
+                        // turns them into NaN, which the min / max drop, so the axis would stop
+                        // bounding the ray and a ray parallel to it would visit a whole slab of the
+                        // tree).  The triangle test uses the ray's own direction.
+                        const f3 db = mk(fabsf(d.x) < 1.3552527e-20f ? copysignf(1.3552527e-20f, d.x) : d.x,
+                                         fabsf(d.y) < 1.3552527e-20f ? copysignf(1.3552527e-20f, d.y) : d.y,
+                                         fabsf(d.z) < 1.3552527e-20f ? copysignf(1.3552527e-20f, d.z) : d.z);
+                        R.inv = mk(1.f / db.x, 1.f / db.y, 1.f / db.z);
+                        R.octinv = 7u - ((db.x < 0.f ? 4u : 0u) | (db.y < 0.f ? 2u : 0u) | (db.z < 0.f ? 1u : 0u));
+                        // the root as the one internal child of a virtual parent: slot 0, imask 1
+                        grp = make_uint2(0u, (1u << (24u + R.octinv)) | 1u);
+                        tgrp = make_uint2(0u, 0u);
+                        best = second = FLT_MAX;
+                        bu = bv = 0.f;
+                        slot = kAny ? 0 : -1;
+                        slot2 = -1;
+                        top = -1;
+                        bot = 0;
+                        owner = ~lane;
+                        mode = kModeWide;
+                        steps = 0;
+                        if (kAny) {
+                            use_limit = S->limit != nullptr;
+                            tmax = use_limit ? __ldg(S->limit + r) : FLT_MAX;
+                            src = dst = -1;
+                            if (S->excl) {
+                                const int2 e = __ldg(reinterpret_cast<const int2*>(S->excl) + r);
+                                src = e.x;
+                                dst = e.y;
+                            }
+                        }
+                        ray = r;
+                        if (kExact && !screenable(R.o, d)) {
+                            mode = kModeBinary;
+                            grp.x = 0u;
+                        }
+                    }
+                }
+            } else {
+                if (idle == kFull) break;
+                // The step limit counts one lane's visits, so rays are shared only under the default
+                if (idle != 0 && max_steps >= kMaxSteps && (++turn & (kShareEvery - 1)) == 0) {
+                    const bool on_stack = top >= bot;
+                    const bool can = ray >= 0 && mode <= kModeCareful && (on_stack || __popc(grp.y >> 24) >= 2);
+                    const unsigned donors = __ballot_sync(kFull, can);
+                    const int pairs = min(__popc(donors), __popc(idle));
+                    if (pairs > 0) {
+                        const unsigned lt = (1u << lane) - 1u;
+                        const bool give = can && __popc(donors & lt) < pairs;
+                        const bool take = ray < 0 && __popc(idle & lt) < pairs;
+                        uint2 g = make_uint2(0, 0);
+                        if (give) {
+                            if (on_stack) {
+                                g = wstack_get<kSmemN>(sst, lst, bot++);  // the oldest: the largest part left
+                                if (bot > top) {
+                                    bot = 0;
+                                    top = -1;
+                                }
+                            } else {  // all but the next child of the current group
+                                const uint32_t keep = 0x80000000u >> __clz(grp.y & 0xFF000000u);
+                                g = make_uint2(grp.x, grp.y & ~keep);
+                                grp.y &= keep | 0x00FFFFFFu;
+                            }
+                            if (owner < 0) {
+                                owner = ~owner;
+                                sh.bound[owner] = __float_as_int(best);
+                                sh.best[owner] = FLT_MAX;
+                                sh.second[owner] = FLT_MAX;
+                                sh.slot2[owner] = -1;
+                                sh.slot[owner] = kAny ? 0 : -1;
+                                sh.pending[owner] = 1;
+                            }
+                            atomicAdd(&sh.pending[owner], 1);
+                            sh.donor[__popc(donors & lt)] = lane;
+                        }
+                        __syncwarp();
+                        // the k-th idle lane takes from the k-th donor
+                        const int from = take ? sh.donor[__popc(idle & lt)] : lane;
+                        const float ox = __shfl_sync(kFull, R.o.x, from), oy = __shfl_sync(kFull, R.o.y, from),
+                                    oz = __shfl_sync(kFull, R.o.z, from);
+                        const float ix = __shfl_sync(kFull, R.inv.x, from), iy = __shfl_sync(kFull, R.inv.y, from),
+                                    iz = __shfl_sync(kFull, R.inv.z, from);
+                        const float dx = __shfl_sync(kFull, d.x, from), dy = __shfl_sync(kFull, d.y, from),
+                                    dz = __shfl_sync(kFull, d.z, from);
+                        const uint32_t oct = __shfl_sync(kFull, R.octinv, from);
+                        const float tm = __shfl_sync(kFull, tmax, from), bb = __shfl_sync(kFull, best, from);
+                        const int64_t rr = __shfl_sync(kFull, ray, from);
+                        const int ow = __shfl_sync(kFull, owner, from), sg = __shfl_sync(kFull, seg, from);
+                        const int es = __shfl_sync(kFull, src, from), ed = __shfl_sync(kFull, dst, from);
+                        const uint32_t gx = __shfl_sync(kFull, g.x, from), gy = __shfl_sync(kFull, g.y, from);
+                        const int how = __shfl_sync(kFull, mode | (use_limit ? 16 : 0), from);
+                        if (take) {
+                            R.o = mk(ox, oy, oz);
+                            R.inv = mk(ix, iy, iz);
+                            R.octinv = oct;
+                            d = mk(dx, dy, dz);
+                            tmax = tm;
+                            best = bb;
+                            second = FLT_MAX;
+                            bu = bv = 0.f;
+                            slot = kAny ? 0 : -1;
+                            slot2 = -1;
+                            src = es;
+                            dst = ed;
+                            use_limit = (how & 16) != 0;
+                            ray = rr;
+                            owner = ow;
+                            if (kSeg) {
+                                seg = sg;
+                                cn = segs[seg].cnodes;
+                                tris = segs[seg].ctris;
+                            }
+                            grp = make_uint2(gx, gy);
+                            tgrp = make_uint2(0u, 0u);
+                            top = -1;
+                            bot = 0;
+                            mode = how & 15;
+                            steps = 0;
+                        }
+                    }
+                }
             }
         }
-        if (ray < 0) continue;
-        int result = -1;  // any hit: 0 clear, 1 occluded
-        bool finished = false, overflow = false;
-        // node phase: a lane without pending triangles takes its next internal child
-        if (tgrp.y == 0u) {
-            if ((grp.y & 0xFF000000u) == 0u) {
-                if (top < 0) {
-                    finished = true;
-                    result = 0;
-                } else {
-                    grp = wstack_get<kSmemN>(sst, lst, top--);
+        // The lanes take each phase together: without the barriers the compiler duplicates the
+        // phases for the paths that lead to them, and the lanes of a warp run them apart (16,384
+        // soup rays 1.43 against 0.76 ms, 4M 40.2 against 38.4).
+        __syncwarp();
+        const bool walk = ray >= 0 && !finished && (!kExact || mode <= kModeCareful);
+        bool failed = false;
+        if (walk) {
+            if (kAny && owner >= 0 && (*(volatile int32_t*)&sh.slot[owner] & 1)) finished = true;
+            // node phase: a lane without pending triangles takes its next internal child
+            if (!finished && (tgrp.y & 0xFFu) == 0u) {
+                if ((grp.y & 0xFF000000u) == 0u) {
+                    if (top < bot) finished = true;
+                    else grp = wstack_get<kSmemN>(sst, lst, top--);
                 }
+                if (!finished) {
+                    const uint32_t bit = 31u - __clz(grp.y & 0xFF000000u);
+                    grp.y &= ~(1u << bit);
+                    const uint32_t s = (bit - 24u) ^ R.octinv;
+                    const uint32_t idx = grp.x + __popc(grp.y & 0xFFu & ((1u << s) - 1u));
+                    if (grp.y & 0xFF000000u) {
+                        if (top + 1 >= kWideStack) failed = true;
+                        else wstack_put<kSmemN>(sst, lst, ++top, grp);
+                    }
+                    uint32_t cbase, tbase, masks;
+                    float bound;
+                    if (kAny) {
+                        bound = kExact ? tmax * kSlack : tmax;
+                    } else {
+                        bound = best;
+                        if (owner >= 0) bound = fminf(bound, __int_as_float(*(volatile int32_t*)&sh.bound[owner]));
+                        bound = fminf(kExact ? bound * kSlack : bound, tmax);
+                    }
+                    if (kStats) ++st.nodes;
+                    const uint32_t h = node_hits(cn, idx, R, bound, cbase, tbase, masks);
+                    grp = make_uint2(cbase, (h & 0xFF000000u) | (masks & 0xFFu));
+                    tgrp = make_uint2(tbase, (h & 0xFFu) | (masks & 0xFF00u));
+                }
+            }
+        }
+        __syncwarp();
+        if (walk) {
+            // triangle phase: one triangle per iteration
+            if (!finished && (tgrp.y & 0xFFu) != 0u) {
+                const uint32_t s = (uint32_t)(__ffs(tgrp.y) - 1);
+                tgrp.y &= tgrp.y - 1u;
+                if (kStats) ++st.tris;
+                const uint32_t at = tgrp.x + __popc((tgrp.y >> 8) & ((1u << s) - 1u));
+                f3 v0, e1, e2;
+                int id, mesh;
+                load_tri(tris, (int64_t)at, v0, e1, e2, id, mesh);
+                float t, u, v;
+                if (kAny) {
+                    if (mesh != src && mesh != dst && tri_test(R.o, d, v0, e1, e2, t, u, v) && (!use_limit || t < tmax)) {
+                        if (!kExact || own_box(kSeg ? segs[seg] : one, at, R, d) >= 0.f) {
+                            slot |= 1;
+                            finished = true;
+                        }
+                    }
+                } else if (tri_test(R.o, d, v0, e1, e2, t, u, v)) {
+                    // slot < 0: no hit of this lane's own (best is then the bound it started from)
+                    const bool mine = slot >= 0;
+                    const bool better = !(t > tmax) && ((!mine && (t <= best || best == FLT_MAX)) || t < best);
+                    bool reached = better;
+                    if (kExact && better && mode == kModeCareful) reached = own_box(one, at, R, d) >= 0.f;
+                    if (reached) {
+                        if (mine) {
+                            second = best;
+                            slot2 = slot;
+                        }
+                        best = t;
+                        slot = (int32_t)at;
+                        bu = u;
+                        bv = v;
+                        if (owner >= 0) atomicMin(&sh.bound[owner], __float_as_int(t));
+                    } else if (!better && !(t > tmax)) {
+                        if (kExact) add_second(t, (int32_t)at, second, slot2);
+                        if (!kExact && t == best && id < tri_id(tris, slot)) {  // at equal distances the lower triangle
+                            slot = (int32_t)at;
+                            bu = u;
+                            bv = v;
+                        }
+                    }
+                    if (kExact && !(t < FLT_MAX)) failed = true;  // not a distance that can be compared
+                }
+            }
+            if (!finished && (failed || ++steps >= max_steps)) {
+                if (!kExact) atomicOr(flag, failed ? kFlagStackOverflow : kFlagStepLimit);
+                if (kAny) slot |= 4;
+                else second = -1.f;
+                finished = true;
+            }
+        } else if (kExact && ray >= 0 && !finished) {
+            // the binary traversal's steps, exactly as in trace.cu; grp.x is the node reference
+            const TraceSeg& S = kSeg ? segs[seg] : one;
+            const f3 inv = mk(1.f / d.x, 1.f / d.y, 1.f / d.z);
+            const int32_t ref = (int32_t)grp.x;
+            bool pop = false, failed = false;
+            if (!kAny && steps == 0 && mode == kModeBinary) {  // a missed root box ends the ray
+                const float* rb = S.root_box;
+                if (!(slab(rb[0], rb[1], rb[2], rb[3], rb[4], rb[5], R.o, inv) >= 0.f)) finished = true;
+            }
+            if (finished) {
+            } else if (ref >= 0) {
+                NodeRegs nr;
+                load_node(S.nodes, ref, nr);
+                const int2 dd = make_int2(__float_as_int(nr.hi[4]), __float_as_int(nr.hi[5]));
+                const float ml = slab(nr.lo[0], nr.lo[1], nr.lo[2], nr.lo[3], nr.lo[4], nr.lo[5], R.o, inv);
+                const float mr = slab(nr.lo[6], nr.lo[7], nr.hi[0], nr.hi[1], nr.hi[2], nr.hi[3], R.o, inv);
+                const bool okl = ml >= 0 && (kAny || (ml < best && !(ml > tmax)));
+                const bool okr = mr >= 0 && (kAny || (mr < best && !(mr > tmax)));
+                if (okl && okr) {
+                    if (top + 1 >= kWideStack) {
+                        failed = true;
+                    } else {
+                        const bool lfar = ml > mr;
+                        wstack_put<kSmemN>(sst, lst, ++top, make_uint2((uint32_t)(lfar ? dd.x : dd.y), 0u));
+                        grp.x = (uint32_t)(lfar ? dd.y : dd.x);
+                    }
+                } else if (okl) {
+                    grp.x = (uint32_t)dd.x;
+                } else if (okr) {
+                    grp.x = (uint32_t)dd.y;
+                } else {
+                    pop = true;
+                }
+            } else {
+                f3 v0, e1, e2;
+                int id, mesh;
+                load_tri(S.tris, ~ref, v0, e1, e2, id, mesh);
+                float t, u, v;
+                if (kAny) {
+                    if (mesh != src && mesh != dst && tri_test(R.o, d, v0, e1, e2, t, u, v) && (!use_limit || t < tmax)) {
+                        slot = 1;
+                        finished = true;
+                    }
+                } else if (tri_test(R.o, d, v0, e1, e2, t, u, v)) {
+                    // bounded: only below the bound; otherwise the first hit counts whatever its distance
+                    if (((mode == kModeBinary && slot < 0) || t < best) && !(t > tmax)) {
+                        best = t;
+                        slot = id;
+                        bu = u;
+                        bv = v;
+                    }
+                }
+                pop = true;
             }
             if (!finished) {
-                const uint32_t bit = 31u - __clz(grp.y & 0xFF000000u);
-                grp.y &= ~(1u << bit);
-                const uint32_t slot = (bit - 24u) ^ (R.octinv4 & 7u);
-                const uint32_t idx = grp.x + __popc(grp.y & 0xFFu & ((1u << slot) - 1u));
-                if (grp.y & 0xFF000000u) {
-                    if (top + 1 >= kWideStack) overflow = true;  // flagged below
-                    else wstack_put<kSmemN>(sst, lst, ++top, grp);
-                }
-                uint32_t cbase, tbase, imask;
-                const float bound = kAny ? lim : fminf(best, tmax);
-                if (kStats) ++st.nodes;
-                const uint32_t h = node_hits(cn, idx, R, bound, cbase, tbase, imask);
-                grp = make_uint2(cbase, (h & 0xFF000000u) | imask);
-                tgrp = make_uint2(tbase, h & 0x00FFFFFFu);
-            }
-        }
-        // triangle phase: one triangle per iteration
-        if (!finished && tgrp.y != 0u) {
-            const uint32_t k = (uint32_t)(__ffs(tgrp.y) - 1);
-            tgrp.y &= tgrp.y - 1u;
-            if (kStats) ++st.tris;
-            f3 v0, e1, e2;
-            int id, mesh;
-            load_tri(tris, (int64_t)tgrp.x + k, v0, e1, e2, id, mesh);
-            float t, u, v;
-            if (kAny) {
-                if (mesh != src && mesh != dst && tri_test(R.o, d, v0, e1, e2, t, u, v) && (!use_limit || t < lim)) {
-                    result = 1;
+                if (failed || ++steps >= max_steps) {
+                    atomicOr(flag, failed ? kFlagStackOverflow : kFlagStepLimit);
+                    if (kAny) slot = 4;
+                    else slot = -2;
                     finished = true;
-                }
-            } else if (tri_test(R.o, d, v0, e1, e2, t, u, v)) {
-                if ((!hit || t < best) && !(t > tmax)) {
-                    hit = true;
-                    best = t;
-                    bid = id;
-                    bu = u;
-                    bv = v;
+                } else if (pop) {
+                    if (top < 0) finished = true;
+                    else grp.x = wstack_get<kSmemN>(sst, lst, top--).x;
                 }
             }
-        }
-        if (!finished && (overflow || ++steps >= max_steps)) {
-            atomicOr(flag, overflow ? kFlagStackOverflow : kFlagStepLimit);
-            result = 2;
-            hit = false;
-            bid = -2;
-            finished = true;
-        }
-        if (finished) {
-            if (kAny) {
-                uint8_t* occ = kSeg ? segs[seg].occ : occ0;
-                occ[ray] = (uint8_t)result;
-            } else {
-                int32_t* prim = kSeg ? segs[seg].prim : prim0;
-                float* tout = kSeg ? segs[seg].t : tout0;
-                float* uv = kSeg ? segs[seg].uv : uv0;
-                prim[ray] = hit ? bid : (bid == -2 ? -2 : -1);
-                if (tout) tout[ray] = hit ? best : __int_as_float(0x7f800000);
-                if (uv) reinterpret_cast<float2*>(uv)[ray] = make_float2(bu, bv);
-            }
-            ray = -1;
         }
     }
     flush_stats<kStats>(st, stats);
 }
 
-template <bool kAny>
-cav_status launch_wide(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays, int64_t n, const uint32_t* n_dev,
-                       int32_t* prim, float* t, float* uv, const float* limit, const int32_t* excl, uint8_t* occ,
-                       cudaStream_t s, unsigned long long* counter, unsigned long long* stats) {
-    cav_status st = ensure_wide(ctx, bvh, s);
-    if (st != CAV_OK) return st;
-    const int block = ctx->wide_block > 0 ? ctx->wide_block : 128;
-    const int batch = ctx->wide_batch > 0 ? ctx->wide_batch : kDefaultRefill;
-    CAV_CUDA(ctx, cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s));
-    int* flag = ctx->d_error + (kAny ? 3 : 2);
-    if (stats) {
-        const int grid = grid_for(ctx, k_trace_wide<kAny, true, false>, block);
-        k_trace_wide<kAny, true, false><<<grid, block, 0, s>>>(bvh->cnodes, bvh->ctris, rays, n, n_dev, prim, t, uv,
-                                                               limit, excl, occ, counter, batch, ctx->max_trace_steps, flag, stats,
-                                                               nullptr, 0);
-    } else if (ctx->wide_smem_stack > 0) {
-        const size_t dyn = sizeof(uint2) * kWideSmemStack * (size_t)block;
-        const int grid = grid_for(ctx, k_trace_wide<kAny, false, false, kWideSmemStack>, block, dyn);
-        k_trace_wide<kAny, false, false, kWideSmemStack><<<grid, block, dyn, s>>>(
-            bvh->cnodes, bvh->ctris, rays, n, n_dev, prim, t, uv, limit, excl, occ, counter, batch,
-            ctx->max_trace_steps, flag, nullptr, nullptr, 0);
-    } else {
-        const int grid = grid_for(ctx, k_trace_wide<kAny, false, false>, block);
-        k_trace_wide<kAny, false, false><<<grid, block, 0, s>>>(bvh->cnodes, bvh->ctris, rays, n, n_dev, prim, t, uv,
-                                                                limit, excl, occ, counter, batch, ctx->max_trace_steps,
-                                                                flag, nullptr, nullptr, 0);
+// Rays a warp holds at least, when there are rays enough: fewer would leave most of each
+// instruction idle while the queue lasts.
+constexpr int kMinCap = 4;
+
+template <bool kAny, bool kStats, bool kSeg, bool kExact, int kSmemN>
+cav_status launch_one(cav_ctx* ctx, const TraceSeg& one, const TraceSeg* segs, int nseg, int64_t n, int block, int batch,
+                      cudaStream_t s, unsigned long long* counter, unsigned long long* stats) {
+    const size_t dyn = sizeof(uint2) * kSmemN * (size_t)block;
+    auto* kernel = k_trace_wide<kAny, kStats, kSeg, kExact, kSmemN>;
+    int grid = grid_for(ctx, kernel, block, dyn);
+    if (!one.n_dev) {
+        const int64_t warps = (n + kMinCap - 1) / kMinCap;
+        grid = (int)std::min<int64_t>(grid, (warps + block / 32 - 1) / (block / 32));
     }
+    CAV_CUDA(ctx, cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s));
+    kernel<<<grid, block, dyn, s>>>(one, segs, nseg, n, counter, batch, kMinCap, ctx->max_trace_steps,
+                                    ctx->d_error + (kAny ? 3 : 2), stats);
     CAV_CUDA(ctx, cudaGetLastError());
     return CAV_OK;
+}
+
+template <bool kAny, bool kSeg>
+cav_status launch_wide(cav_ctx* ctx, const TraceSeg& one, const TraceSeg* segs, int nseg, int64_t n, cudaStream_t s,
+                       unsigned long long* counter, unsigned long long* stats) {
+    const int block = ctx->wide_block > 0 ? ctx->wide_block : 128;
+    const int batch = ctx->wide_batch > 0 ? ctx->wide_batch : kDefaultRefill;
+    if (!kSeg && stats)
+        return launch_one<kAny, !kSeg, kSeg, false, 0>(ctx, one, segs, nseg, n, block, batch, s, counter, stats);
+    if (!kSeg && (ctx->wide_smem_stack > 0 || (ctx->wide_smem_stack < 0 && !kAny)))
+        return launch_one<kAny, false, kSeg, false, kSeg ? 0 : kWideSmemStack>(ctx, one, segs, nseg, n, block, batch, s,
+                                                                              counter, nullptr);
+    return launch_one<kAny, false, kSeg, false, 0>(ctx, one, segs, nseg, n, block, batch, s, counter, nullptr);
+}
+
+TraceSeg wide_seg(const cav_bvh* bvh) {
+    TraceSeg g{};
+    g.nodes = bvh->tnodes;
+    g.tris = bvh->tris;
+    g.root_box = bvh->d_root_box;
+    g.cnodes = bvh->cnodes;
+    g.ctris = bvh->ctris;
+    g.lbox = bvh->lbox;
+    return g;
 }
 
 }  // namespace
@@ -511,38 +1093,30 @@ cav_status trace_wide_segments(cav_ctx* ctx, bool any_hit, const TraceSeg* segs,
                                unsigned long long* counter) {
     if (nseg <= 0 || n == 0) return CAV_OK;
     if (nseg > kMaxSeg) return set_error(ctx, CAV_ERR_INVALID_ARGUMENT, "too many trace segments in one launch");
-    const int block = ctx->wide_block > 0 ? ctx->wide_block : 128;
-    const int batch = ctx->wide_batch > 0 ? ctx->wide_batch : kDefaultRefill;
-    CAV_CUDA(ctx, cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s));
-    if (any_hit) {
-        const int grid = grid_for(ctx, k_trace_wide<true, false, true>, block);
-        k_trace_wide<true, false, true><<<grid, block, 0, s>>>(nullptr, nullptr, nullptr, n, nullptr, nullptr, nullptr,
-                                                               nullptr, nullptr, nullptr, nullptr, counter, batch,
-                                                               ctx->max_trace_steps, ctx->d_error + 3, nullptr, segs,
-                                                               nseg);
-    } else {
-        const int grid = grid_for(ctx, k_trace_wide<false, false, true>, block);
-        k_trace_wide<false, false, true><<<grid, block, 0, s>>>(nullptr, nullptr, nullptr, n, nullptr, nullptr, nullptr,
-                                                                nullptr, nullptr, nullptr, nullptr, counter, batch,
-                                                                ctx->max_trace_steps, ctx->d_error + 2, nullptr, segs,
-                                                                nseg);
-    }
-    CAV_CUDA(ctx, cudaGetLastError());
-    return CAV_OK;
+    const TraceSeg none{};
+    return any_hit ? launch_wide<true, true>(ctx, none, segs, nseg, n, s, counter, nullptr)
+                   : launch_wide<false, true>(ctx, none, segs, nseg, n, s, counter, nullptr);
 }
 
 cav_status ensure_wide(cav_ctx* ctx, const cav_bvh* bvh, cudaStream_t s) {
+    if (bvh->wide_state.load(std::memory_order_acquire) > 0) return CAV_OK;
     // serialised: several host threads (the server's lanes) may reach one tree at once; the
     // view is published only once its build has completed on the device
     static std::mutex build_mu;
     std::lock_guard<std::mutex> lk(build_mu);
-    if (bvh->cnodes) return CAV_OK;
+    if (bvh->wide_state.load(std::memory_order_acquire) > 0) return CAV_OK;
     const int64_t n = bvh->n;
     const int64_t nw = n - 1;  // each wide node but the root stands for a distinct binary internal node
     size_t need = sizeof(CNode) * (size_t)nw + 256;
     need += sizeof(TriRec) * (size_t)n + 256;
+    need += 2 * sizeof(float4) * (size_t)n + 256;
     need += sizeof(int32_t) * (size_t)nw + 256;
-    need += 64 + 256;
+    need += sizeof(WideCtr) + 256;
+    if (!ctx->wide_host && cudaMallocHost(&ctx->wide_host, sizeof(WideCtr)) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->wide_host = nullptr;
+        return set_error(ctx, CAV_ERR_OUT_OF_MEMORY, "fast traversal layout: pinned allocation failed");
+    }
     void* arena = nullptr;  // stream-ordered: complete before the view is published below
     if (dev_alloc(ctx, &arena, need, s, true) != cudaSuccess) {
         cudaGetLastError();
@@ -556,39 +1130,28 @@ cav_status ensure_wide(cav_ctx* ctx, const cav_bvh* bvh, cudaStream_t s) {
     };
     CNode* cn = (CNode*)carve(sizeof(CNode) * (size_t)nw);
     TriRec* ct = (TriRec*)carve(sizeof(TriRec) * (size_t)n);
+    float4* lbox = (float4*)carve(2 * sizeof(float4) * (size_t)n);
     int32_t* task = (int32_t*)carve(sizeof(int32_t) * (size_t)nw);
-    uint32_t* ctr = (uint32_t*)carve(32);
-    float* margin = (float*)(ctr + 4);
-    k_wide_init<<<1, 32, 0, s>>>(bvh->d_root_box, task, ctr, margin);
-    const int grid = ctx->num_sms * 8;
-    uint32_t* hctr = nullptr;
-    if (cudaMallocHost(&hctr, 16) != cudaSuccess) {
-        cudaGetLastError();
-        cudaFree(arena);
-        return set_error(ctx, CAV_ERR_OUT_OF_MEMORY, "fast traversal layout: pinned allocation failed");
-    }
+    WideCtr* ctr = (WideCtr*)carve(sizeof(WideCtr));
+    k_wide_init<<<1, 32, 0, s>>>(bvh->d_root_box, task, ctr);
+    // about one wide node per four triangles, eight lanes each; every block co-resident
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wide_build, kBuildThreads, 0);
+    const int64_t room = (int64_t)ctx->num_sms * std::min(std::max(per_sm, 1), 8);
+    const int grid = (int)std::min<int64_t>(room, std::max<int64_t>(1, n * 2 / kBuildThreads));
+    uint32_t max_nodes = (uint32_t)nw, max_tris = (uint32_t)n;
+    uint64_t wait_ns = ctx->sort_wait_ns;
+    const TNode* tn = bvh->tnodes;
+    const TriRec* tin = bvh->tris;
+    void* args[] = {&tn, &tin, &task, &cn, &ct, &lbox, &ctr, &max_nodes, &max_tris, &wait_ns};
+    cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_wide_build, dim3(grid), dim3(kBuildThreads), args, 0, s);
+    WideCtr* h = (WideCtr*)ctx->wide_host;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, ctr, sizeof(WideCtr), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     cav_status st = CAV_OK;
-    // levels until the frontier is empty; the host looks every 8 levels
-    for (int level = 0; level < kMaxWideLevels; ++level) {
-        k_wide_level<<<grid, kBuildThreads, 0, s>>>(bvh->tnodes, bvh->tris, task, cn, ct, ctr, margin);
-        k_wide_next_level<<<1, 32, 0, s>>>(ctr);
-        if ((level & 7) == 7) {
-            cudaMemcpyAsync(hctr, ctr, 16, cudaMemcpyDeviceToHost, s);
-            cudaError_t e = cudaStreamSynchronize(s);
-            if (e != cudaSuccess) {
-                st = cuda_error(ctx, e, "fast traversal layout");
-                break;
-            }
-            if (hctr[2] == hctr[3]) break;
-        }
-    }
-    if (st == CAV_OK) {
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) st = cuda_error(ctx, e, "fast traversal layout");
-        else if (hctr[1] != (uint32_t)n)
-            st = set_error(ctx, CAV_ERR_CUDA, "fast traversal layout: not every triangle placed");
-    }
-    cudaFreeHost(hctr);
+    if (e != cudaSuccess) st = cuda_error(ctx, e, "fast traversal layout");
+    else if (h->failed || h->tris != (uint32_t)n)
+        st = set_error(ctx, CAV_ERR_CUDA, "fast traversal layout: not every triangle placed");
     if (st != CAV_OK) {
         cudaFree(arena);
         return st;
@@ -596,6 +1159,8 @@ cav_status ensure_wide(cav_ctx* ctx, const cav_bvh* bvh, cudaStream_t s) {
     bvh->wide_arena = arena;
     bvh->cnodes = cn;
     bvh->ctris = ct;
+    bvh->lbox = lbox;
+    bvh->wide_state.store(h->unscreened ? 1 : 2, std::memory_order_release);
     return CAV_OK;
 }
 
@@ -607,19 +1172,93 @@ void free_wide(cav_bvh* bvh, cudaStream_t s, bool async) {
     bvh->wide_arena = nullptr;
     bvh->cnodes = nullptr;
     bvh->ctris = nullptr;
+    bvh->lbox = nullptr;
+    bvh->wide_state.store(0);
+}
+
+// Rays that a tree must have been asked about before the exact mode builds its view.  The view
+// of a tree of 10,000 triangles or more costs less than what its first batch saves, down to
+// 64 rays (soups, closest hit, a call with the view's build against the binary traversal:
+// 10,000 triangles and 512 rays 157 against 283 us, 100,000 and 512 rays 305 against 1,162 us,
+// 1M and 512 rays 1.6 against 8.2 ms); smaller trees save 10 to 30 us a call and the view
+// costs 70 us.
+static int64_t screen_min_rays(int64_t n) { return n >= 4096 ? 512 : 16384; }
+
+// Closest hits on trees of up to this many triangles always take the binary traversal: a wide
+// node costs as much as the few binary nodes it replaces (36 triangles, 1M rays: 0.177 ms
+// against 0.189; any hits gain, 0.178 against 0.114).
+constexpr int64_t kScreenMinTris = 128;
+
+// Whether the exact mode's screening pass can run for n more rays on this tree, building the
+// view on the stream when the tree has been asked about enough of them (that first call waits
+// for the build).  False leaves the binary traversal: a lowered step limit, a stream in
+// capture without a view, no memory for one, or geometry out of the screening range.
+bool screen_ready(cav_ctx* ctx, const cav_bvh* bvh, bool any_hit, int64_t n, cudaStream_t s) {
+    if (!any_hit && bvh->n <= kScreenMinTris) return false;
+    if (ctx->max_trace_steps < kMaxSteps) return false;  // a lowered limit counts binary visits
+    int state = bvh->wide_state.load(std::memory_order_acquire);
+    if (state == 0) {
+        const int64_t seen = bvh->rays_seen.fetch_add(n) + n;
+        if (seen < screen_min_rays(bvh->n)) return false;
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+            cudaGetLastError();
+            return false;
+        }
+        const std::string said = ctx->last_error;
+        if (ensure_wide(ctx, bvh, s) != CAV_OK) {  // the binary traversal needs no view
+            ctx->last_error = said;
+            bvh->wide_state.store(-1);
+            return false;
+        }
+        state = bvh->wide_state.load(std::memory_order_acquire);
+    }
+    return state == 2;
+}
+
+cav_status trace_screened(cav_ctx* ctx, const cav_bvh* bvh, const TraceSeg& q, bool any_hit, int64_t n, cudaStream_t s,
+                          unsigned long long* counter) {
+    TraceSeg one = q;
+    const TraceSeg w = wide_seg(bvh);
+    one.cnodes = w.cnodes;
+    one.ctris = w.ctris;
+    one.lbox = w.lbox;
+    const int block = ctx->trace_block > 0 ? std::min(ctx->trace_block, 256) : 128;
+    const int batch = ctx->trace_batch > 0 ? ctx->trace_batch : kDefaultRefill;
+    const bool smem = ctx->screen_smem_stack < 0 ? !any_hit : ctx->screen_smem_stack > 0;
+    if (any_hit)
+        return smem ? launch_one<true, false, false, true, kWideSmemStack>(ctx, one, nullptr, 0, n, block, batch, s, counter, nullptr)
+                    : launch_one<true, false, false, true, 0>(ctx, one, nullptr, 0, n, block, batch, s, counter, nullptr);
+    return smem ? launch_one<false, false, false, true, kWideSmemStack>(ctx, one, nullptr, 0, n, block, batch, s, counter, nullptr)
+                : launch_one<false, false, false, true, 0>(ctx, one, nullptr, 0, n, block, batch, s, counter, nullptr);
 }
 
 cav_status trace_wide_closest(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays, int64_t n, const uint32_t* n_dev,
                               int32_t* prim, float* t, float* uv, cudaStream_t s, unsigned long long* counter,
                               unsigned long long* stats) {
-    return launch_wide<false>(ctx, bvh, rays, n, n_dev, prim, t, uv, nullptr, nullptr, nullptr, s, counter, stats);
+    cav_status st = ensure_wide(ctx, bvh, s);
+    if (st != CAV_OK) return st;
+    TraceSeg one = wide_seg(bvh);
+    one.rays = rays;
+    one.prim = prim;
+    one.t = t;
+    one.uv = uv;
+    one.n_dev = n_dev;
+    return launch_wide<false, false>(ctx, one, nullptr, 0, n, s, counter, stats);
 }
 
 cav_status trace_wide_any(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays, const float* limit,
                           const int32_t* excl, int64_t n, const uint32_t* n_dev, uint8_t* occ, cudaStream_t s,
                           unsigned long long* counter, unsigned long long* stats) {
-    return launch_wide<true>(ctx, bvh, rays, n, n_dev, nullptr, nullptr, nullptr, limit, excl, occ, s, counter,
-                             stats);
+    cav_status st = ensure_wide(ctx, bvh, s);
+    if (st != CAV_OK) return st;
+    TraceSeg one = wide_seg(bvh);
+    one.rays = rays;
+    one.limit = limit;
+    one.excl = excl;
+    one.occ = occ;
+    one.n_dev = n_dev;
+    return launch_wide<true, false>(ctx, one, nullptr, 0, n, s, counter, stats);
 }
 
 }  // namespace cav
