@@ -35,15 +35,18 @@ __host__ __device__ inline f3 cross3(f3 a, f3 b) {
 }
 __host__ __device__ inline float dot3(f3 a, f3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 
-// AABB::computeSurfaceArea, Core/BoundingBox.h:77-80 (same expression).
+// AABB::computeSurfaceArea, Core/BoundingBox.h:77-80.  The contraction is written out, so that
+// the areas, and through ties the trees, do not depend on how the code around is compiled.
 __device__ inline float surface_area(f3 lo, f3 hi) {
     f3 e = hi - lo;
-    return 2.f * (e.x * e.y + e.y * e.z + e.x * e.z);
+    return 2.f * fmaf(e.x, e.z, fmaf(e.x, e.y, __fmul_rn(e.y, e.z)));
 }
 // BVH/SAH.h:4-22: FP64 literals, float results.
 __device__ inline float leaf_cost(float area, int n) { return area * 1.0 * n; }
-__device__ inline float internal_cost(float area, float l, float r) { return area * 1.2 + l + r; }
-__device__ inline float internal_cost(float area, float c) { return area * 1.2 + c; }
+__device__ inline float internal_cost(float area, float l, float r) {
+    return (float)__dadd_rn(fma((double)area, 1.2, (double)l), (double)r);
+}
+__device__ inline float internal_cost(float area, float c) { return (float)fma((double)area, 1.2, (double)c); }
 
 // Build error bits, or-ed into the context's first error word by a build and mapped to a
 // cav_status by cav_sync_check.  Every bit but kErrBadIndex means the tree's structure is not

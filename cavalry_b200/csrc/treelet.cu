@@ -53,13 +53,15 @@ constexpr SubsetTable make_table() {
 
 __constant__ SubsetTable kSubsets = make_table();
 
-struct WarpSmem {
+struct __align__(16) WarpSmem {
     float area[128];
     float cost[128];
-    signed char part[128];
-    int leaf_lane[8];
-    float lbox[7][6];  // the treelet leaves' boxes (read by every lane: broadcast)
+    float lbox[7][8];    // the treelet leaves' boxes (lo, hi, two unused: 16-byte loads, broadcast)
     int32_t lrec[7][4];  // and their left, right, prim, is_leaf
+    float carea[8];      // and their areas as stored
+    float pcost[64];     // partial minima of subsets whose partitions are split over lanes
+    signed char ppart[64];
+    signed char part[128];
 };
 
 struct Rec {
@@ -124,110 +126,201 @@ __device__ inline void reduce_partition(float& tc, int& p) {
     p = __shfl_sync(kFull, p, (int)win);
 }
 
-// optimizeTreelet semantics for the subtree rooted at `root`.  Returns false only on
-// an internal inconsistency (recorded in *err by the caller).
-__device__ bool optimize_treelet(BNode* nodes, int32_t root, int32_t count, WarpSmem& S) {
+// The area of a union of treelet leaves, rounded as this pass always has (the other order of
+// the contraction than surface_area).
+__device__ __forceinline__ float subset_area(f3 lo, f3 hi) {
+    const f3 e = hi - lo;
+    return 2.f * fmaf(e.x, e.z, fmaf(e.y, e.z, __fmul_rn(e.x, e.y)));
+}
+
+__device__ __forceinline__ void load_box(const WarpSmem& S, int k, f3& lo, f3& hi) {
+    const float4 a = *reinterpret_cast<const float4*>(S.lbox[k]);
+    const float2 b = *reinterpret_cast<const float2*>(S.lbox[k] + 4);
+    lo = mk(a.x, a.y, a.z);
+    hi = mk(a.w, b.x, b.y);
+}
+
+__device__ __forceinline__ void unite_box(const WarpSmem& S, int k, f3& lo, f3& hi) {
+    f3 blo, bhi;
+    load_box(S, k, blo, bhi);
+    lo = vmin3(lo, blo);
+    hi = vmax3(hi, bhi);
+}
+
+// The cost of subset `s` split into p and the rest.
+__device__ __forceinline__ float split_cost(const WarpSmem& S, int s, int p) { return S.cost[p] + S.cost[s ^ p]; }
+
+// Partitions first..last of subset s in the reference's order (Optimization.cu:180-216: the
+// j-th is the j-th subset of s without its lowest bit, in increasing order), from partition p
+// on; the first smallest wins.
+__device__ __forceinline__ void best_of(const WarpSmem& S, int s, int p, int count, float& best, int& bestp) {
+    const int cleared = (s - 1) & s;
+    best = split_cost(S, s, p);
+    bestp = p;
+#pragma unroll 1
+    for (int k = 1; k < count; ++k) {
+        p = (p - cleared) & s;
+        const float c = split_cost(S, s, p);
+        if (c < best) {
+            best = c;
+            bestp = p;
+        }
+    }
+}
+
+// The j-th subset of `m` in increasing order (bit i of j to the i-th bit of m), m of at most
+// four bits.
+__device__ __forceinline__ int nth_subset(int m, int j) {
+    int r = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int low = m & -m;
+        if ((j >> i) & 1) r |= low;
+        m ^= low;
+    }
+    return r;
+}
+
+__device__ __forceinline__ void put_subset(WarpSmem& S, int s, float best, int bestp) {
+    S.cost[s] = internal_cost(S.area[s], best);
+    S.part[s] = (signed char)bestp;
+}
+
+// The best partition of every subset of 2..7 leaves, with the reference's choice among equal
+// costs (the first smallest in its order).  Subsets of 2 and 3 leaves take a lane each; the
+// last three of the 35 of 4 leaves and all 21 of 5 leaves are split over lanes, whose partial
+// minima are then taken in order; the 7 of 6 leaves take four lanes each: the reference's
+// bracket keeps, among equal costs, the partition whose 5-bit number read backwards is
+// smallest, so lane c of a subset takes the numbers 8 c .. 8 c + 7 in that reading.  21
+// steps of a cost sum and a comparison, where a lane per subset and a warp reduction per
+// 6-leaf subset took 36 and seven reductions.  With the boxes and records
+// taken from the subsets (below) a round over the 1M-triangle soup executes 644 M warp
+// instructions, 795 M before, and three rounds take 4.13 ms, 4.47 before; issue slots (57 %
+// used) and the waits for node fetches bound the walk.
+__device__ __forceinline__ void split_subsets(WarpSmem& S) {
     const int lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
-
-    // ---- formation (Optimization.cu:59-107)
-    int32_t nid = -1;
-    Rec rec{};
-    if (lane == 0) {
-        nid = root;
-        rec = load_rec(nodes, root);
+    float best;
+    int bestp;
+    // 2 leaves: one partition each
+    if (lane < 21) {
+        const int s = kSubsets.s[lane], p = (s - 1) & s;
+        put_subset(S, s, split_cost(S, s, p), p);
     }
-    bool expanded = false;
-    int size = 1;
-    while (size < 13) {
-        // the first of lanes 0..size-1 with the largest area above -1 (lane 0 when none):
-        // areas are non-negative, so their bit patterns order like their values
-        const bool cand = lane < size && !(rec.is_leaf || expanded) && rec.area > -1.f;
-        int max_lane = 0;
-        if (__any_sync(kFull, cand && !(rec.area >= 0.f))) {  // a negative area: a plain scan
-            float my_area = rec.area;
-            if (rec.is_leaf || expanded) my_area = -1.f;
-            float max_area = -1.f;
-            for (int i = 0; i < size; ++i) {
-                float a = __shfl_sync(kFull, my_area, i);
-                if (a > max_area) {
-                    max_area = a;
-                    max_lane = i;
+    __syncwarp();
+    // 3 leaves: three partitions each, 35 subsets
+#pragma unroll 1
+    for (int k = lane; k < 35; k += 32) {
+        const int s = kSubsets.s[kSubsets.off[1] + k];
+        best_of(S, s, -((s - 1) & s) & s, 3, best, bestp);
+        put_subset(S, s, best, bestp);
+    }
+    __syncwarp();
+    // 4 leaves: seven partitions each; the last three subsets one partition per lane
+    {
+        const int s = kSubsets.s[kSubsets.off[2] + lane];
+        best_of(S, s, -((s - 1) & s) & s, 7, best, bestp);
+        put_subset(S, s, best, bestp);
+        if (lane < 21) {
+            const int k = lane / 7;
+            const int s3 = kSubsets.s[kSubsets.off[2] + 32 + k];
+            const int p = nth_subset((s3 - 1) & s3, lane - 7 * k + 1);
+            S.pcost[lane] = split_cost(S, s3, p);
+            S.ppart[lane] = (signed char)p;
+        }
+        __syncwarp();
+        if (lane < 3) {
+            best = S.pcost[7 * lane];
+            int at = 7 * lane;
+#pragma unroll
+            for (int j = 1; j < 7; ++j)
+                if (S.pcost[7 * lane + j] < best) {
+                    best = S.pcost[7 * lane + j];
+                    at = 7 * lane + j;
                 }
+            put_subset(S, kSubsets.s[kSubsets.off[2] + 32 + lane], best, S.ppart[at]);
+        }
+    }
+    __syncwarp();
+    // 5 leaves: fifteen partitions each, in three parts of five
+    {
+#pragma unroll 1
+        for (int k = lane; k < 63; k += 32) {
+            const int q = k / 3;
+            const int s = kSubsets.s[kSubsets.off[3] + q];
+            best_of(S, s, nth_subset((s - 1) & s, 5 * (k - 3 * q) + 1), 5, best, bestp);
+            S.pcost[k] = best;
+            S.ppart[k] = (signed char)bestp;
+        }
+        __syncwarp();
+        if (lane < 21) {
+            best = S.pcost[3 * lane];
+            int at = 3 * lane;
+#pragma unroll
+            for (int j = 1; j < 3; ++j)
+                if (S.pcost[3 * lane + j] < best) {
+                    best = S.pcost[3 * lane + j];
+                    at = 3 * lane + j;
+                }
+            put_subset(S, kSubsets.s[kSubsets.off[3] + lane], best, S.ppart[at]);
+        }
+    }
+    __syncwarp();
+    // 6 leaves (Optimization.cu:224-266): partition number l of the subset without leaf eb
+    // (lane l's in the reference) is l with a zero bit put in at eb, for eb = 6 with its upper
+    // bits dropped (the reference's shift by -1)
+    {
+        const int eb = min(lane >> 2, 6), c = lane & 3;
+        const int s = 0x7f ^ (1 << eb);
+        best = INFINITY;
+        bestp = 0;
+        bool none = true;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {  // l = bit-reversed (8 c + r)
+            const int l = ((r & 1) << 4) | ((r & 2) << 2) | (r & 4) | ((c & 1) << 1) | (c >> 1);
+            const int hi = eb <= 5 ? ((l << 1) & (((1 << (5 - eb)) - 1) << (eb + 1))) : 0;
+            const int p = (l & ((1 << eb) - 1)) | hi;
+            const float t = split_cost(S, s, p);
+            if (p != 0 && (none || t < best)) {
+                best = t;
+                bestp = p;
+                none = false;
             }
-        } else {
-            const unsigned key = cand ? __float_as_uint(rec.area + 0.f) + 1u : 0u;
-            const unsigned top = __reduce_max_sync(kFull, key);
-            if (top != 0u) max_lane = __ffs(__ballot_sync(kFull, key == top)) - 1;
         }
-        int stop = __shfl_sync(kFull, (int)(expanded || rec.is_leaf), max_lane);
-        if (stop) return true;  // fewer than 7 leaves reachable: leave the subtree as it is
-        int32_t cl = __shfl_sync(kFull, rec.left, max_lane);
-        int32_t cr = __shfl_sync(kFull, rec.right, max_lane);
-        if (cl < 0 || cr < 0 || cl >= count || cr >= count) return false;
-        if (lane == max_lane) expanded = true;
-        if (lane == size) {
-            nid = cl;
-            rec = load_rec(nodes, cl);
+#pragma unroll
+        for (int d = 1; d < 4; d <<= 1) {  // the lower lane keeps equal costs
+            const float ob = __shfl_xor_sync(kFull, best, d);
+            const int op = __shfl_xor_sync(kFull, bestp, d);
+            const bool on = __shfl_xor_sync(kFull, none ? 1 : 0, d) != 0;
+            const bool upper = (c & d) != 0;
+            if (!on && (none || ob < best || (ob == best && upper))) {
+                best = ob;
+                bestp = op;
+                none = false;
+            }
         }
-        if (lane == size + 1) {
-            nid = cr;
-            rec = load_rec(nodes, cr);
-        }
-        size += 2;
+        if (c == 0 && lane < 28) put_subset(S, s, best, bestp);
     }
-    const bool in_treelet = lane < 13;
-    const unsigned leaf_mask = __ballot_sync(kFull, in_treelet && !expanded);
-    const int my_leaf = __popc(leaf_mask & lt);
-    if (in_treelet && !expanded) S.leaf_lane[my_leaf] = lane;
     __syncwarp();
+    // all 7 leaves (Optimization.cu:271-324)
+    {
+        int p = lane;
+        float tc = -1.f;
+        if (p != 0) tc = split_cost(S, 0x7f, p);
+        const int op = lane | 32;
+        const float otc = split_cost(S, 0x7f, op);
+        if (tc == -1.f || otc < tc) {
+            tc = otc;
+            p = op;
+        }
+        reduce_partition(tc, p);
+        if (lane == 0) put_subset(S, 0x7f, tc, p);
+    }
+    __syncwarp();
+}
 
-    // ---- subset areas (Optimization.cu:126-163)
-    // the leaves' records go through shared memory rather than registers (the walk's
-    // occupancy is set by its registers)
-    if (in_treelet && !expanded) {
-        float* b = S.lbox[my_leaf];
-        b[0] = rec.lo_x; b[1] = rec.lo_y; b[2] = rec.lo_z;
-        b[3] = rec.hi_x; b[4] = rec.hi_y; b[5] = rec.hi_z;
-        int32_t* r = S.lrec[my_leaf];
-        r[0] = rec.left; r[1] = rec.right; r[2] = rec.prim; r[3] = rec.is_leaf;
-    }
-    __syncwarp();
-    const float(&lbox)[7][6] = S.lbox;
-#pragma unroll
-    // Subset s = (q << 5) | lane: the union of the lane's leaves 0-4 (its low five bits) is
-    // taken once, then leaves 5 and 6 per quarter q (min/max unions are exact in any order).
-    bool any = false;
-    f3 lo = mk(0, 0, 0), hi = mk(0, 0, 0);
-    auto unite = [&](int k, bool& a, f3& l, f3& h) {
-        const f3 blo = mk(lbox[k][0], lbox[k][1], lbox[k][2]);
-        const f3 bhi = mk(lbox[k][3], lbox[k][4], lbox[k][5]);
-        if (!a) {
-            l = blo;
-            h = bhi;
-            a = true;
-        } else {
-            l = vmin3(l, blo);
-            h = vmax3(h, bhi);
-        }
-    };
-#pragma unroll
-    for (int k = 0; k < 5; ++k)
-        if ((lane >> k) & 1) unite(k, any, lo, hi);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        bool qany = any;
-        f3 qlo = lo, qhi = hi;
-        if (q & 1) unite(5, qany, qlo, qhi);
-        if (q & 2) unite(6, qany, qlo, qhi);
-        const int s = (q << 5) | lane;
-        S.area[s] = qany ? surface_area(qlo, qhi) : 0.f;
-        S.cost[s] = -1.f;
-    }
-    __syncwarp();
-    if (in_treelet && !expanded) S.cost[1 << my_leaf] = rec.cost;
-    __syncwarp();
-
+// The same with the reference's own loops, for costs that do not order (NaN or negative).
+__device__ __noinline__ void plain_subsets(WarpSmem& S) {
+    const int lane = threadIdx.x & 31;
     // ---- subsets of 2..5 leaves (Optimization.cu:180-216), grouped by size
 #pragma unroll 1
     for (int g = 0; g < 4; ++g) {
@@ -292,106 +385,189 @@ __device__ bool optimize_treelet(BNode* nodes, int32_t root, int32_t count, Warp
         }
         __syncwarp();
     }
+}
+
+// optimizeTreelet semantics for the subtree rooted at `root`.  Returns false only on
+// an internal inconsistency (recorded in *err by the caller).
+__device__ bool optimize_treelet(BNode* nodes, int32_t root, int32_t count, WarpSmem& S) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+
+    // ---- formation (Optimization.cu:59-107)
+    int32_t nid = -1;
+    Rec rec{};
+    if (lane == 0) {
+        nid = root;
+        rec = load_rec(nodes, root);
+    }
+    bool expanded = false;
+    int size = 1;
+    while (size < 13) {
+        // the first of lanes 0..size-1 with the largest area above -1 (lane 0 when none):
+        // areas are non-negative, so their bit patterns order like their values
+        const bool cand = lane < size && !(rec.is_leaf || expanded) && rec.area > -1.f;
+        int max_lane = 0;
+        if (__any_sync(kFull, cand && !(rec.area >= 0.f))) {  // a negative area: a plain scan
+            float my_area = rec.area;
+            if (rec.is_leaf || expanded) my_area = -1.f;
+            float max_area = -1.f;
+            for (int i = 0; i < size; ++i) {
+                float a = __shfl_sync(kFull, my_area, i);
+                if (a > max_area) {
+                    max_area = a;
+                    max_lane = i;
+                }
+            }
+        } else {
+            const unsigned key = cand ? __float_as_uint(rec.area + 0.f) + 1u : 0u;
+            const unsigned top = __reduce_max_sync(kFull, key);
+            if (top != 0u) max_lane = __ffs(__ballot_sync(kFull, key == top)) - 1;
+        }
+        int stop = __shfl_sync(kFull, (int)(expanded || rec.is_leaf), max_lane);
+        if (stop) return true;  // fewer than 7 leaves reachable: leave the subtree as it is
+        int32_t cl = __shfl_sync(kFull, rec.left, max_lane);
+        int32_t cr = __shfl_sync(kFull, rec.right, max_lane);
+        if (cl < 0 || cr < 0 || cl >= count || cr >= count) return false;
+        if (lane == max_lane) expanded = true;
+        if (lane == size) {
+            nid = cl;
+            rec = load_rec(nodes, cl);
+        }
+        if (lane == size + 1) {
+            nid = cr;
+            rec = load_rec(nodes, cr);
+        }
+        size += 2;
+    }
+    const bool in_treelet = lane < 13;
+    const unsigned leaf_mask = __ballot_sync(kFull, in_treelet && !expanded);
+    const int my_leaf = __popc(leaf_mask & lt);
+
+    // ---- subset areas (Optimization.cu:126-163)
+    // the leaves' records go through shared memory rather than registers (the walk's
+    // occupancy is set by its registers)
+    if (in_treelet && !expanded) {
+        float4* b = reinterpret_cast<float4*>(S.lbox[my_leaf]);
+        b[0] = make_float4(rec.lo_x, rec.lo_y, rec.lo_z, rec.hi_x);
+        b[1] = make_float4(rec.hi_y, rec.hi_z, 0.f, 0.f);
+        *reinterpret_cast<int4*>(S.lrec[my_leaf]) = make_int4(rec.left, rec.right, rec.prim, rec.is_leaf);
+    }
+    __syncwarp();
+    // Subset s = (q << 5) | lane: the union of the lane's leaves 0-4 (its low five bits) is
+    // taken once, then leaves 5 and 6 per quarter q.
+    f3 lo, hi;
+    load_box(S, lane != 0 ? __ffs(lane) - 1 : 5, lo, hi);
+#pragma unroll
+    for (int k = 1; k < 5; ++k)
+        if ((lane >> k) & 1) unite_box(S, k, lo, hi);
+    S.area[lane] = lane != 0 ? subset_area(lo, hi) : 0.f;
+    {
+        f3 l6, h6;
+        load_box(S, 6, l6, h6);
+        if (lane != 0) {
+            l6 = vmin3(lo, l6);
+            h6 = vmax3(hi, h6);
+            unite_box(S, 5, lo, hi);
+        }
+        S.area[32 | lane] = subset_area(lo, hi);
+        S.area[64 | lane] = subset_area(l6, h6);
+        unite_box(S, 6, lo, hi);
+        S.area[96 | lane] = subset_area(lo, hi);
+    }
+    if (in_treelet && !expanded) {
+        S.cost[1 << my_leaf] = rec.cost;
+        S.carea[my_leaf] = rec.area;
+    }
+    __syncwarp();
+
+    // costs are finite or infinite but never NaN or negative, or the reference's own loops run
+    bool plain = in_treelet && !expanded && !(rec.cost >= 0.f);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) plain = plain || !(S.area[(q << 5) | lane] >= 0.f);
+    if (__any_sync(kFull, plain)) plain_subsets(S);
+    else split_subsets(S);
 
     // ---- reconstruction (Optimization.cu:330-394): lane i keeps node nid and takes a role
     int my_subset = lane == 0 ? 0x7f : -1;
-    int32_t my_parent = lane == 0 ? rec.parent : -1;
     bool exp_r = false;
-    int cl_lane = lane, cr_lane = lane;
+    int par_lane = 0, cl_lane = lane, cr_lane = lane;
     int rsize = 1;
     while (rsize < 13) {
-        bool prop = lane < rsize && !exp_r && !is_pow2(my_subset);
-        unsigned m = __ballot_sync(kFull, prop);
+        const bool prop = lane < rsize && !exp_r && !is_pow2(my_subset);
+        const unsigned m = __ballot_sync(kFull, prop);
         if (m == 0) return false;
-        int sel_lane = __ffs(m) - 1;
-        int sel = __shfl_sync(kFull, my_subset, sel_lane);
-        int32_t parent_node = __shfl_sync(kFull, nid, sel_lane);
-        int pp = S.part[sel];
-        if (sel <= 0 || sel > 127 || is_pow2(sel) || pp <= 0 || (pp & ~sel) != 0) return false;
+        const int sel_lane = __ffs(m) - 1;
+        const int sel = __shfl_sync(kFull, my_subset, sel_lane);
+        if (sel <= 0 || sel > 127 || is_pow2(sel)) return false;
+        const int pp = S.part[sel];
+        if (pp <= 0 || (pp & ~sel) != 0) return false;
         if (lane == sel_lane) {
             exp_r = true;
             cl_lane = rsize;
             cr_lane = rsize + 1;
         }
-        if (lane == rsize) {
-            my_parent = parent_node;
-            my_subset = pp;
-        }
-        if (lane == rsize + 1) {
-            my_parent = parent_node;
-            my_subset = sel ^ pp;
-        }
+        if (lane == rsize) my_subset = pp;
+        if (lane == rsize + 1) my_subset = sel ^ pp;
+        if (lane == rsize || lane == rsize + 1) par_lane = sel_lane;
         rsize += 2;
     }
 
-    // ---- new records (Optimization.cu:400-461)
-    int leaf_id = (in_treelet && !exp_r) ? __ffs(my_subset) - 1 : 0;
-    Rec o;
-    o.lo_x = lbox[leaf_id][0];
-    o.lo_y = lbox[leaf_id][1];
-    o.lo_z = lbox[leaf_id][2];
-    o.hi_x = lbox[leaf_id][3];
-    o.hi_y = lbox[leaf_id][4];
-    o.hi_z = lbox[leaf_id][5];
-    o.left = S.lrec[leaf_id][0];
-    o.right = S.lrec[leaf_id][1];
-    o.prim = S.lrec[leaf_id][2];
-    o.is_leaf = S.lrec[leaf_id][3];
-    int32_t child_l = __shfl_sync(kFull, nid, cl_lane);
-    int32_t child_r = __shfl_sync(kFull, nid, cr_lane);
-
+    // ---- new records (Optimization.cu:400-461).  A node's box is the union of its leaves'
+    // (min and max do not depend on the order), its area the subset's; a treelet leaf keeps
+    // the cost it was stored with, which is what computing it again gives: its own treelet was
+    // finished, and its children's costs final, before this root was reached.
     Rec nr;
-    nr.parent = my_parent;
-    float ocl = 0.f, ocr = 0.f;
-    if (!exp_r) {
-        nr.lo_x = o.lo_x; nr.lo_y = o.lo_y; nr.lo_z = o.lo_z;
-        nr.hi_x = o.hi_x; nr.hi_y = o.hi_y; nr.hi_z = o.hi_z;
-        nr.left = o.left;
-        nr.right = o.right;
-        nr.prim = o.prim;
-        nr.is_leaf = o.is_leaf;
-        if (in_treelet && !o.is_leaf && o.left >= 0 && o.right >= 0 && o.left < count && o.right < count) {
-            ocl = __ldcg(&nodes[o.left].cost);
-            ocr = __ldcg(&nodes[o.right].cost);
-        }
-    } else {
-        nr.lo_x = nr.lo_y = nr.lo_z = 0.f;
-        nr.hi_x = nr.hi_y = nr.hi_z = 0.f;
+    {
+        const int32_t up = __shfl_sync(kFull, nid, par_lane);
+        nr.parent = lane == 0 ? rec.parent : up;
+    }
+    const int32_t child_l = __shfl_sync(kFull, nid, cl_lane);
+    const int32_t child_r = __shfl_sync(kFull, nid, cr_lane);
+    const int subset = in_treelet ? my_subset : 1;
+    const int leaf_id = __ffs(subset) - 1;
+    f3 nlo, nhi;
+    load_box(S, leaf_id, nlo, nhi);
+#pragma unroll
+    for (int k = 1; k < 7; ++k)
+        if ((subset >> k) & 1) unite_box(S, k, nlo, nhi);
+    nr.lo_x = nlo.x; nr.lo_y = nlo.y; nr.lo_z = nlo.z;
+    nr.hi_x = nhi.x; nr.hi_y = nhi.y; nr.hi_z = nhi.z;
+    nr.area = S.area[subset];
+    int32_t old_l = 0, old_r = 0;
+    if (exp_r) {
         nr.left = child_l;
         nr.right = child_r;
         nr.prim = -1;
         nr.is_leaf = 0;
-    }
-    // bottom-up boxes: children sit at higher lanes, the treelet is at most 6 deep
-#pragma unroll
-    for (int it = 0; it < 6; ++it) {
-        float a0 = __shfl_sync(kFull, nr.lo_x, cl_lane), b0 = __shfl_sync(kFull, nr.lo_x, cr_lane);
-        float a1 = __shfl_sync(kFull, nr.lo_y, cl_lane), b1 = __shfl_sync(kFull, nr.lo_y, cr_lane);
-        float a2 = __shfl_sync(kFull, nr.lo_z, cl_lane), b2 = __shfl_sync(kFull, nr.lo_z, cr_lane);
-        float a3 = __shfl_sync(kFull, nr.hi_x, cl_lane), b3 = __shfl_sync(kFull, nr.hi_x, cr_lane);
-        float a4 = __shfl_sync(kFull, nr.hi_y, cl_lane), b4 = __shfl_sync(kFull, nr.hi_y, cr_lane);
-        float a5 = __shfl_sync(kFull, nr.hi_z, cl_lane), b5 = __shfl_sync(kFull, nr.hi_z, cr_lane);
-        if (exp_r) {
-            f3 lo = vmin3(mk(a0, a1, a2), mk(b0, b1, b2));
-            f3 hi = vmax3(mk(a3, a4, a5), mk(b3, b4, b5));
-            nr.lo_x = lo.x; nr.lo_y = lo.y; nr.lo_z = lo.z;
-            nr.hi_x = hi.x; nr.hi_y = hi.y; nr.hi_z = hi.z;
+        nr.cost = 0.f;
+    } else {
+        const int4 o = *reinterpret_cast<const int4*>(S.lrec[leaf_id]);
+        nr.left = old_l = o.x;
+        nr.right = old_r = o.y;
+        nr.prim = o.z;
+        nr.is_leaf = o.w;
+        nr.cost = S.cost[1 << leaf_id];
+        // where the stored area was rounded another way (a node that the refit wrote), the cost
+        // follows the area; the children's costs are final
+        if (in_treelet && nr.area != S.carea[leaf_id]) {
+            if (nr.is_leaf) nr.cost = leaf_cost(nr.area, 1);
+            else if (old_l >= 0 && old_r >= 0 && old_l < count && old_r < count)
+                nr.cost = internal_cost(nr.area, __ldcg(&nodes[old_l].cost), __ldcg(&nodes[old_r].cost));
         }
     }
-    nr.area = surface_area(mk(nr.lo_x, nr.lo_y, nr.lo_z), mk(nr.hi_x, nr.hi_y, nr.hi_z));
-    if (!exp_r) nr.cost = nr.is_leaf ? leaf_cost(nr.area, 1) : internal_cost(nr.area, ocl, ocr);
-    else nr.cost = 0.f;
+    // costs from the last pair of children to the first: lanes 2 k + 1 and 2 k + 2 hang
+    // under the lane that took them, always a lower one
 #pragma unroll
-    for (int it = 0; it < 6; ++it) {
-        float ca = __shfl_sync(kFull, nr.cost, cl_lane);
-        float cb = __shfl_sync(kFull, nr.cost, cr_lane);
-        if (exp_r) nr.cost = internal_cost(nr.area, ca, cb);
+    for (int k = 11; k >= 1; k -= 2) {
+        const float ca = __shfl_sync(kFull, nr.cost, k);
+        const float cb = __shfl_sync(kFull, nr.cost, k + 1);
+        if (cl_lane == k && lane != k) nr.cost = internal_cost(nr.area, ca, cb);
     }
     if (in_treelet) {
         store_rec(nodes, nid, nr);
-        if (!exp_r && !o.is_leaf && o.left >= 0 && o.right >= 0 && o.left < count && o.right < count) {
-            __stcg(&nodes[o.left].parent, nid);
-            __stcg(&nodes[o.right].parent, nid);
+        if (!exp_r && !nr.is_leaf && old_l >= 0 && old_r >= 0 && old_l < count && old_r < count) {
+            __stcg(&nodes[old_l].parent, nid);
+            __stcg(&nodes[old_r].parent, nid);
         }
     }
     __syncwarp();

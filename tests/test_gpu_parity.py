@@ -317,3 +317,25 @@ def test_host_buffer_path_over_several_chunks(cuda_ctx):
     assert np.array_equal(out[0].numpy(), prim_d) and np.array_equal(out[1].numpy().view(np.uint32), t_d.view(np.uint32))
     assert np.array_equal(occ_p.numpy(), occ_d)
     bvh.free()
+
+
+@pytest.mark.parametrize("n", [7, 8, 50, 1000, 5000])
+@pytest.mark.parametrize("rounds", [1, 3])
+def test_treelets_on_ties_match_oracle(cuda_ctx, n, rounds):
+    """Vertices on a small integer lattice: areas are exact, so partitions tie everywhere and the
+    choice among equal costs (in every subset size) decides the tree."""
+    import torch
+
+    from oracle import pyoracle as po
+
+    rng = np.random.default_rng(n + rounds)
+    pos = rng.integers(0, 9, (3 * n, 3)).astype(np.float32)
+    pos[::5] = pos[0]
+    idx = np.arange(3 * n, dtype=np.int32).reshape(n, 3)
+    bvh = cuda_ctx.build(torch.from_numpy(pos).cuda(), torch.from_numpy(idx).cuda(), rounds=rounds)
+    mu, ms, perm = bvh.export_stages()
+    o = po.build(pos, idx, codes=mu, rounds=rounds)
+    assert np.array_equal(ms, o["sorted"]) and np.array_equal(perm, o["perm"])
+    nodes_equal(bvh.export_nodes(), o["final"], f"lattice {n} rounds {rounds}")
+    cuda_ctx.sync_check()
+    bvh.free()
