@@ -229,15 +229,17 @@ static cav_status ctx_halton(cav_ctx* ctx, cav_scene* sc) {
     std::lock_guard<std::mutex> lk(ctx->halton_mu);
     if (!ctx->d_halton_perms) {
         const HaltonTables& t = halton_tables();
+        std::vector<uint32_t> primes = t.primes;  // with the digits' multipliers behind them
+        for (uint32_t p : t.primes) primes.push_back((uint32_t)(((uint64_t)1 << 32) / p));
         void *a = nullptr, *b = nullptr, *c = nullptr;
-        if (cudaMalloc(&a, t.primes.size() * 4) != cudaSuccess || cudaMalloc(&b, t.start.size() * 4) != cudaSuccess ||
+        if (cudaMalloc(&a, primes.size() * 4) != cudaSuccess || cudaMalloc(&b, t.start.size() * 4) != cudaSuccess ||
             cudaMalloc(&c, t.perms.size() * 2) != cudaSuccess) {
             cudaGetLastError();
             cudaFree(a);
             cudaFree(b);
             return set_error(ctx, CAV_ERR_OUT_OF_MEMORY, "Halton tables: device allocation failed");
         }
-        CAV_CUDA(ctx, cudaMemcpy(a, t.primes.data(), t.primes.size() * 4, cudaMemcpyHostToDevice));
+        CAV_CUDA(ctx, cudaMemcpy(a, primes.data(), primes.size() * 4, cudaMemcpyHostToDevice));
         CAV_CUDA(ctx, cudaMemcpy(b, t.start.data(), t.start.size() * 4, cudaMemcpyHostToDevice));
         CAV_CUDA(ctx, cudaMemcpy(c, t.perms.data(), t.perms.size() * 2, cudaMemcpyHostToDevice));
         ctx->d_halton_primes = (uint32_t*)a;

@@ -41,23 +41,37 @@ __device__ inline f3 ld3(const float* p) { return mk(p[0], p[1], p[2]); }
 
 // ------------------------------------------------------------------------ Halton
 struct Halton {
-    const uint32_t* primes;
+    const uint32_t* primes;  // kPrimes primes, then floor(2^32 / prime) of each
     const uint32_t* perm_start;
     const uint16_t* perms;
 };
 
-// runHalton + HaltonSampler::rand1 (Samplers/HaltonSampler.h:13-23, :59-66)
+// runHalton + HaltonSampler::rand1 (Samplers/HaltonSampler.h:13-23, :59-66).  The digits are
+// exact: with m = floor(2^32 / base), the high word of i m is i / base or one less.  A bounce's
+// dimensions take 30 to 80 digits; with a 64-bit division for each (the reference's index type)
+// shading took 89 us a bounce of the 256x256, 16-sample room and generation 60, now 76 and 37.
 __device__ inline float halton(const Halton& h, uint64_t index, int& dim) {
     const int d = dim < kPrimes ? dim : kPrimes - 1;
     dim += 1;
-    const uint32_t base = h.primes[d];
+    const uint32_t base = h.primes[d], m = h.primes[kPrimes + d];
     const uint16_t* perm = h.perms + h.perm_start[d];
     float r = 0, f = 1;
-    uint64_t i = index;
+    uint64_t big = index;
+    while (big >> 32) {
+        f = f / base;
+        r = r + f * (perm[big % base]);
+        big = big / base;
+    }
+    uint32_t i = (uint32_t)big;
     while (i > 0) {
         f = f / base;
-        r = r + f * (perm[i % base]);
-        i = i / base;
+        uint32_t q = __umulhi(i, m), digit = i - q * base;
+        if (digit >= base) {
+            digit -= base;
+            ++q;
+        }
+        r = r + f * (perm[digit]);
+        i = q;
     }
     return r;
 }
