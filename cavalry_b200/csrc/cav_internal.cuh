@@ -217,7 +217,7 @@ size_t sort_status_words(int64_t n, int passes);
 cav_status sort_pairs(cav_ctx* ctx, uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp, uint32_t* vals_tmp, int64_t n,
                       int passes, uint32_t* hist, uint32_t* status, uint32_t* counters, int* err, cudaStream_t s);
 // treelet.cu
-// counters: device words of the caller's scratch ([0]: leaf-list positions, [1]: the walkers' claims)
+// counters: device words of the caller's scratch ([0]: seeds listed, [1]: the walkers' claims)
 cav_status treelet_rounds(cav_ctx* ctx, BNode* nodes, int64_t n, int rounds, int32_t* leaf_list, uint32_t* visited,
                           uint32_t* counters, cudaStream_t s);
 struct TreeletSeg {  // one tree of a batched treelet pass
@@ -272,7 +272,7 @@ cav_status trace_wide_any(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays,
 void free_wide(cav_bvh* bvh, cudaStream_t s, bool async);
 // The exact mode through the view: whether it can be used, and one launch of it (q: the rays,
 // the outputs and the binary tree).
-bool screen_ready(cav_ctx* ctx, const cav_bvh* bvh, bool any_hit, int64_t n, cudaStream_t s);
+bool screen_ready(cav_ctx* ctx, const cav_bvh* bvh, int64_t n, cudaStream_t s);
 cav_status trace_screened(cav_ctx* ctx, const cav_bvh* bvh, const TraceSeg& q, bool any_hit, int64_t n, cudaStream_t s,
                           unsigned long long* counter);
 cav_status trace_wide_segments(cav_ctx* ctx, bool any_hit, const TraceSeg* segs, int nseg, int64_t n, cudaStream_t s,

@@ -1184,17 +1184,12 @@ void free_wide(cav_bvh* bvh, cudaStream_t s, bool async) {
 // costs 70 us.
 static int64_t screen_min_rays(int64_t n) { return n >= 4096 ? 512 : 16384; }
 
-// Closest hits on trees of up to this many triangles always take the binary traversal: a wide
-// node costs as much as the few binary nodes it replaces (36 triangles, 1M rays: 0.177 ms
-// against 0.189; any hits gain, 0.178 against 0.114).
-constexpr int64_t kScreenMinTris = 128;
-
 // Whether the exact mode's screening pass can run for n more rays on this tree, building the
 // view on the stream when the tree has been asked about enough of them (that first call waits
 // for the build).  False leaves the binary traversal: a lowered step limit, a stream in
 // capture without a view, no memory for one, or geometry out of the screening range.
-bool screen_ready(cav_ctx* ctx, const cav_bvh* bvh, bool any_hit, int64_t n, cudaStream_t s) {
-    if (!any_hit && bvh->n <= kScreenMinTris) return false;
+bool screen_ready(cav_ctx* ctx, const cav_bvh* bvh, int64_t n, cudaStream_t s) {
+    if (bvh->n <= kTinyTris) return false;
     if (ctx->max_trace_steps < kMaxSteps) return false;  // a lowered limit counts binary visits
     int state = bvh->wide_state.load(std::memory_order_acquire);
     if (state == 0) {
