@@ -7,9 +7,9 @@
 // node, first lane on ties), same partition enumeration order per subset, the same
 // warp min-reduction tree for the 6- and 7-leaf subsets, and the same reuse of node
 // ids by lane during reconstruction.  It differs in mechanics only:
-//   * the warps that start a round are the nodes that are leaves when the round starts,
-//     listed by a separate pass (the reference tests `isLeaf` inside the same launch
-//     that restructures the tree, Optimization.cu:479);
+//   * a round starts from the nodes that are leaves when it starts (the reference tests
+//     `isLeaf` inside the same launch that restructures the tree, Optimization.cu:479): a
+//     separate pass climbs from them, a thread per leaf, to the lowest nodes with 7 leaves;
 //   * the formation lanes keep their node records in registers, so every read of the
 //     old treelet precedes every write, and the bottom-up box/cost refresh runs on
 //     registers with explicit warp synchronisation (the reference iterates 7 times over
@@ -19,7 +19,7 @@
 //     smaller subsets, so the order between subsets does not change any value);
 //   * a node whose subtree holds fewer than 7 leaves is not visited by the formation at
 //     all (the reference's formation expands such a subtree and gives up without writing);
-//   * the walkers are persistent warps that claim their starting leaves from a counter.
+//   * the walkers are persistent warps that claim their starting nodes from a counter.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -387,9 +387,10 @@ __device__ __noinline__ void plain_subsets(WarpSmem& S) {
     }
 }
 
-// optimizeTreelet semantics for the subtree rooted at `root`.  Returns false only on
+// optimizeTreelet semantics for the subtree rooted at `root`, whose parent it reports (it never
+// changes).  Returns false only on
 // an internal inconsistency (recorded in *err by the caller).
-__device__ bool optimize_treelet(BNode* nodes, int32_t root, int32_t count, WarpSmem& S) {
+__device__ bool optimize_treelet(BNode* nodes, int32_t root, int32_t count, WarpSmem& S, int32_t& root_parent) {
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
 
@@ -400,6 +401,7 @@ __device__ bool optimize_treelet(BNode* nodes, int32_t root, int32_t count, Warp
         nid = root;
         rec = load_rec(nodes, root);
     }
+    root_parent = __shfl_sync(kFull, rec.parent, 0);
     bool expanded = false;
     int size = 1;
     while (size < 13) {
@@ -574,40 +576,65 @@ __device__ bool optimize_treelet(BNode* nodes, int32_t root, int32_t count, Warp
     return true;
 }
 
-__global__ void k_leaf_list(const BNode* __restrict__ nodes, int64_t count, int32_t* __restrict__ list,
-                            uint32_t* __restrict__ counter) {
+// A leaf's climb to the first node with 7 or more leaves under it (a subtree of fewer cannot form
+// a treelet: the reference's formation then expands every internal node of it and gives up
+// without writing anything; with 7 or more an internal node always remains to expand).  Each
+// node's arrival counter holds the leaves of its first child to arrive (saturated at 7); the
+// second arrival goes on, and returns the node once it counts 7.  -1: another leaf goes on.
+__device__ int32_t seed_climb(const BNode* __restrict__ nodes, int32_t curr, int32_t count, uint32_t* visited, int* err) {
+    uint32_t leaves = 1;
+    while (curr != 0) {
+        const int32_t parent = nodes[curr].parent;
+        if (parent < 0 || parent >= count) {
+            atomicExch(err, 2);
+            return -1;
+        }
+        const uint32_t old = atomicAdd(visited + parent, (leaves << 2) | 1u);
+        if ((old & 3u) != 1u) return -1;
+        leaves = min(7u, leaves + (old >> 2));
+        curr = parent;
+        if (leaves >= 7) return curr;
+    }
+    return -1;
+}
+
+// The round's seeds: a thread per leaf climbs the small subtrees.  With a warp per leaf the
+// walkers spent a third of the round on climbs that ended below a treelet (three rounds on the
+// 1M-triangle soup 4.13 ms, 2.92 with this pass).
+__global__ void k_treelet_seeds(const BNode* __restrict__ nodes, int64_t count, int32_t* __restrict__ list,
+                                uint32_t* __restrict__ counter, uint32_t* visited, int* err) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    bool leaf = i < count && nodes[i].is_leaf;
-    unsigned m = __ballot_sync(kFull, leaf);
+    int32_t seed = -1;
+    if (i < count && nodes[i].is_leaf) seed = seed_climb(nodes, (int32_t)i, (int32_t)count, visited, err);
+    __syncwarp();
+    const unsigned m = __ballot_sync(kFull, seed >= 0);
     if (m == 0) return;
-    int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31;
     uint32_t base = 0;
     if (lane == __ffs(m) - 1) base = atomicAdd(counter, (uint32_t)__popc(m));
     base = __shfl_sync(kFull, base, __ffs(m) - 1);
-    uint32_t pos = base + __popc(m & ((1u << lane) - 1u));
-    if (leaf && pos < (uint32_t)((count + 1) / 2)) list[pos] = (int32_t)i;
+    const uint32_t pos = base + __popc(m & ((1u << lane) - 1u));
+    if (seed >= 0 && pos < (uint32_t)((count + 1) / 2)) list[pos] = seed;
 }
 
-// optimizeBVHImpl (Optimization.cu:467-507): one warp per starting leaf; the second
-// arrival at a node optimises the treelet rooted there and continues upwards.
-//
-// Each walker carries the number of leaves under its node (saturated at 7) in the arrival
-// counter: an arrival adds (leaves << 2) | 1, so the second arrival learns its sibling's
-// count.  A subtree of fewer than 7 leaves cannot form a treelet: the reference's formation
-// then expands every internal node of it and gives up without writing anything (with 7 or
-// more leaves an internal node always remains to expand), so such nodes skip formation and
-// the tree is unchanged.  The counter's update is an acquire-release atomic: the lanes'
-// record writes precede it (warp barrier), and the second arrival's reads follow it.
+// optimizeBVHImpl (Optimization.cu:467-507): a warp per seed optimises its treelet and walks up;
+// the second arrival at a node optimises the treelet rooted there and continues.  The
+// counter's update is an acquire-release atomic: the lanes' record writes precede it (warp
+// barrier), and the second arrival's reads follow it.
 __device__ void treelet_walk(BNode* nodes, int32_t curr, int32_t count, uint32_t* visited, WarpSmem& S, int* err) {
     const int lane = threadIdx.x & 31;
     if (curr < 0 || curr >= count) {
         if (lane == 0) atomicExch(err, 2);
         return;
     }
-    uint32_t leaves = 1;  // under curr, saturated at 7
     for (;;) {
-        if (curr == 0) break;
-        int32_t parent = __ldcg(&nodes[curr].parent);
+        int32_t parent = -1;
+        if (!optimize_treelet(nodes, curr, count, S, parent)) {
+            if (lane == 0) atomicExch(err, 2);
+            return;
+        }
+        __syncwarp();
+        if (curr == 0) return;
         if (parent < 0 || parent >= count) {
             if (lane == 0) atomicExch(err, 2);
             return;
@@ -616,43 +643,38 @@ __device__ void treelet_walk(BNode* nodes, int32_t curr, int32_t count, uint32_t
         if (lane == 0)
             asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;"
                          : "=r"(old)
-                         : "l"(visited + parent), "r"((leaves << 2) | 1u)
+                         : "l"(visited + parent), "r"((7u << 2) | 1u)
                          : "memory");
         old = __shfl_sync(kFull, old, 0);
         if ((old & 3u) != 1u) return;  // first arrival stops; the second optimises the parent
         __syncwarp();
-        leaves = min(7u, leaves + (old >> 2));
         curr = parent;
-        if (leaves >= 7 && !optimize_treelet(nodes, curr, count, S)) {
-            if (lane == 0) atomicExch(err, 2);
-            return;
-        }
-        __syncwarp();
     }
 }
 
 // Persistent walkers: a fixed grid of 2-warp blocks, 24 per SM (48 warps at 40 registers),
-// each warp claiming starting leaves from a counter until the list is exhausted.  The walk
+// each warp claiming seeds from a counter until the list is exhausted.  The walk
 // waits on atomics and dependent loads, so resident walkers matter more than registers,
 // and a persistent warp never waits for a block launch after a first arrival ends its walk.
 // Measured on 3 rounds over a 1M-triangle soup: one launched warp per leaf in 1-warp blocks
 // (32 per SM, 64 registers) 7.14 ms; persistent 1-warp blocks at 64 registers 5.67;
 // 2-warp blocks at 48 registers (40 per SM) 5.46; at 40 registers 5.34, 5.00 with the leaf
 // boxes in shared memory, 4.93 with the leaf records there too, 4.72 with the subset boxes
-// built from per-lane partial unions; at 32 registers (64 per SM) 5.99 (spills).  Claiming
-// 4 or 16 leaves per atomic did not help.
+// built from per-lane partial unions; at 32 registers (64 per SM) 5.99 (spills).
 constexpr int kWalkWarps = 2;
 constexpr int kWalkBlocksPerSm = 24;
 __global__ void __launch_bounds__(kWalkWarps * 32, kWalkBlocksPerSm)
-    k_treelet(BNode* nodes, const int32_t* __restrict__ list, int64_t n, uint32_t* visited, int* err, uint32_t* claim) {
+    k_treelet(BNode* nodes, const int32_t* __restrict__ list, int64_t n, uint32_t* visited, int* err,
+              const uint32_t* __restrict__ seeds, uint32_t* claim) {
     __shared__ WarpSmem smem[kWalkWarps];
     WarpSmem& S = smem[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
+    const uint32_t total = min(*seeds, (uint32_t)n);
     for (;;) {
         uint32_t i = 0;
         if (lane == 0) i = atomicAdd(claim, 1u);
         i = __shfl_sync(kFull, i, 0);
-        if (i >= (uint32_t)n) return;
+        if (i >= total) return;
         treelet_walk(nodes, list[i], (int32_t)(2 * n - 1), visited, S, err);
         __syncwarp();
     }
@@ -664,14 +686,13 @@ __global__ void __launch_bounds__(kWalkWarps * 32, kWalkBlocksPerSm)
 // warp finds its tree by binary search over the offsets.
 __device__ inline int64_t node_off(const int64_t* leaf_off, int k) { return 2 * leaf_off[k] - k; }
 
-__global__ void k_leaf_list_batch(const TreeletSeg* __restrict__ segs, const int64_t* __restrict__ leaf_off, int k0,
-                                  int k1, int32_t* __restrict__ list, uint32_t* __restrict__ counters) {
+__global__ void k_treelet_seeds_batch(const TreeletSeg* __restrict__ segs, const int64_t* __restrict__ leaf_off, int k0,
+                                      int k1, int2* __restrict__ list, uint32_t* __restrict__ counter, uint32_t* visited,
+                                      int* err) {
     const int64_t i = node_off(leaf_off, k0) + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool in = i < node_off(leaf_off, k1);
     int k = k0;
-    int64_t local = 0, n = 0;
-    bool leaf = false;
-    if (in) {
+    int32_t seed = -1;
+    if (i < node_off(leaf_off, k1)) {
         int lo = k0, hi = k1 - 1;  // the tree whose node range holds i
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
@@ -679,47 +700,39 @@ __global__ void k_leaf_list_batch(const TreeletSeg* __restrict__ segs, const int
             else hi = mid - 1;
         }
         k = lo;
-        local = i - node_off(leaf_off, k);
-        n = segs[k].n;
-        leaf = local < 2 * n - 1 && segs[k].nodes[local].is_leaf;
+        const int64_t at = node_off(leaf_off, k), local = i - at;
+        const int32_t count = (int32_t)(2 * segs[k].n - 1);
+        if (local < count && segs[k].nodes[local].is_leaf)
+            seed = seed_climb(segs[k].nodes, (int32_t)local, count, visited + at, err);
     }
-    // one atomic per (warp, tree): the lanes of one tree take consecutive list positions in
-    // lane order, as the single-tree pass does
-    const unsigned leaves = __ballot_sync(kFull, leaf);
-    if (!leaf) return;
-    const unsigned peers = __match_any_sync(leaves, k) & leaves;
+    __syncwarp();
+    const unsigned m = __ballot_sync(kFull, seed >= 0);
+    if (m == 0) return;
     const int lane = threadIdx.x & 31;
-    const int first = __ffs(peers) - 1;
     uint32_t base = 0;
-    if (lane == first) base = atomicAdd(counters + k, (uint32_t)__popc(peers));
-    base = __shfl_sync(peers, base, first);
-    const uint32_t pos = base + __popc(peers & ((1u << lane) - 1u));
-    if (pos < (uint32_t)n) list[leaf_off[k] + pos] = (int32_t)local;
+    if (lane == __ffs(m) - 1) base = atomicAdd(counter, (uint32_t)__popc(m));
+    base = __shfl_sync(kFull, base, __ffs(m) - 1);
+    const int64_t pos = (int64_t)base + __popc(m & ((1u << lane) - 1u));
+    // a seed has 7 leaves or more of its own, so two words per seed fit the group's leaves
+    if (seed >= 0 && 2 * pos + 1 < leaf_off[k1] - leaf_off[k0]) list[pos] = make_int2(k, seed);
 }
 
-// The same persistent walkers over a group of trees: a claimed index g of the group's
-// concatenated leaf list belongs to the tree whose leaf range holds it.
+// The same persistent walkers over a group of trees: a seed names its tree.
 __global__ void __launch_bounds__(kWalkWarps * 32, kWalkBlocksPerSm)
-    k_treelet_batch(const TreeletSeg* __restrict__ segs, const int64_t* __restrict__ leaf_off, int k0, int k1,
-                    const int32_t* __restrict__ list, uint32_t* visited, int* err, uint32_t* claim) {
+    k_treelet_batch(const TreeletSeg* __restrict__ segs, const int64_t* __restrict__ leaf_off,
+                    const int2* __restrict__ list, uint32_t* visited, int* err, const uint32_t* __restrict__ seeds,
+                    uint32_t* claim) {
     __shared__ WarpSmem smem[kWalkWarps];
     WarpSmem& S = smem[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
-    const int64_t first = leaf_off[k0], total = leaf_off[k1] - first;
+    const uint32_t total = *seeds;
     for (;;) {
         uint32_t i = 0;
         if (lane == 0) i = atomicAdd(claim, 1u);
         i = __shfl_sync(kFull, i, 0);
-        if ((int64_t)i >= total) return;
-        const int64_t g = first + i;
-        int lo = k0, hi = k1 - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (leaf_off[mid] <= g) lo = mid;
-            else hi = mid - 1;
-        }
-        const int64_t n = segs[lo].n;
-        treelet_walk(segs[lo].nodes, list[g], (int32_t)(2 * n - 1), visited + node_off(leaf_off, lo), S, err);
+        if (i >= total) return;
+        const int2 s = list[i];
+        treelet_walk(segs[s.x].nodes, s.y, (int32_t)(2 * segs[s.x].n - 1), visited + node_off(leaf_off, s.x), S, err);
         __syncwarp();
     }
 }
@@ -730,14 +743,15 @@ cav_status treelet_rounds(cav_ctx* ctx, BNode* nodes, int64_t n, int rounds, int
                           uint32_t* counter, cudaStream_t s) {
     if (rounds <= 0) return CAV_OK;
     const int64_t count = 2 * n - 1;
-    // counter[0]: the leaf list's positions, counter[1]: the walkers' claims; both in the
+    // counter[0]: the seeds listed, counter[1]: the walkers' claims; both in the
     // build's own scratch (builds on different streams, such as a server's lanes, never share it)
-    const int64_t grid = std::min<int64_t>(div_up(n, kWalkWarps), (int64_t)ctx->num_sms * kWalkBlocksPerSm);
+    // at most n / 7 seeds: their subtrees are disjoint
+    const int64_t grid = std::min<int64_t>(div_up(div_up(n, 7) + 1, kWalkWarps), (int64_t)ctx->num_sms * kWalkBlocksPerSm);
     for (int r = 0; r < rounds; ++r) {
         CAV_CUDA(ctx, cudaMemsetAsync(visited, 0, sizeof(uint32_t) * count, s));
         CAV_CUDA(ctx, cudaMemsetAsync(counter, 0, 2 * sizeof(uint32_t), s));
-        k_leaf_list<<<div_up(count, 256), 256, 0, s>>>(nodes, count, leaf_list, counter);
-        k_treelet<<<(unsigned)grid, kWalkWarps * 32, 0, s>>>(nodes, leaf_list, n, visited, ctx->d_error + 1,
+        k_treelet_seeds<<<div_up(count, 256), 256, 0, s>>>(nodes, count, leaf_list, counter, visited, ctx->d_error + 1);
+        k_treelet<<<(unsigned)grid, kWalkWarps * 32, 0, s>>>(nodes, leaf_list, n, visited, ctx->d_error + 1, counter,
                                                              counter + 1);
     }
     CAV_CUDA(ctx, cudaGetLastError());
@@ -745,14 +759,14 @@ cav_status treelet_rounds(cav_ctx* ctx, BNode* nodes, int64_t n, int rounds, int
 }
 
 // Treelet rounds of K trees, a group of consecutive trees at a time: per group and round one
-// leaf-list launch and one treelet launch over all its trees (rather than two per tree).  A
+// seeds launch and one treelet launch over all its trees (rather than two per tree).  A
 // group holds at most kGroupLeaves leaves; a tree that fills a group alone runs the
 // single-tree pass (measured: the grouped kernels were 1.3x slower than it on trees of
 // 0.5-2M triangles, and launch overhead does not matter there).  Each tree's result is the
 // single-tree one: within a tree the walk is the same, and trees share no nodes.  segs /
 // leaf_off: device tables (K trees, K + 1 leaf offsets), segs_host / leaf_off_host the same
 // on the host; leaf_list holds leaf_off[K] entries, visited 2 leaf_off[K] - K, counters K + 2
-// (per tree leaf-list positions, then the two of a tree that runs the single-tree pass).
+// (the last two are used).
 cav_status treelet_rounds_batch(cav_ctx* ctx, const TreeletSeg* segs, const TreeletSeg* segs_host,
                                 const int64_t* leaf_off, const int64_t* leaf_off_host, int K, int rounds,
                                 int32_t* leaf_list, uint32_t* counters, uint32_t* visited, cudaStream_t s) {
@@ -771,14 +785,16 @@ cav_status treelet_rounds_batch(cav_ctx* ctx, const TreeletSeg* segs, const Tree
             k0 = k1;
             continue;
         }
-        const int64_t grid = std::min<int64_t>(div_up(leaves, kWalkWarps), (int64_t)ctx->num_sms * kWalkBlocksPerSm);
+        const int64_t grid =
+            std::min<int64_t>(div_up(div_up(leaves, 7) + 1, kWalkWarps), (int64_t)ctx->num_sms * kWalkBlocksPerSm);
         for (int r = 0; r < rounds; ++r) {
             CAV_CUDA(ctx, cudaMemsetAsync(visited + node_off_h(k0), 0, sizeof(uint32_t) * nodes, s));
-            CAV_CUDA(ctx, cudaMemsetAsync(counters + k0, 0, sizeof(uint32_t) * (k1 - k0), s));
-            CAV_CUDA(ctx, cudaMemsetAsync(counters + K + 1, 0, sizeof(uint32_t), s));  // the walkers' claims
-            k_leaf_list_batch<<<div_up(nodes, 256), 256, 0, s>>>(segs, leaf_off, k0, k1, leaf_list, counters);
-            k_treelet_batch<<<(unsigned)grid, kWalkWarps * 32, 0, s>>>(segs, leaf_off, k0, k1, leaf_list, visited,
-                                                                      ctx->d_error + 1, counters + K + 1);
+            CAV_CUDA(ctx, cudaMemsetAsync(counters + K, 0, 2 * sizeof(uint32_t), s));  // seeds, the walkers' claims
+            int2* list = reinterpret_cast<int2*>(leaf_list);
+            k_treelet_seeds_batch<<<div_up(nodes, 256), 256, 0, s>>>(segs, leaf_off, k0, k1, list, counters + K, visited,
+                                                                     ctx->d_error + 1);
+            k_treelet_batch<<<(unsigned)grid, kWalkWarps * 32, 0, s>>>(segs, leaf_off, list, visited, ctx->d_error + 1,
+                                                                      counters + K, counters + K + 1);
         }
         k0 = k1;
     }
