@@ -141,6 +141,15 @@ __device__ inline uint64_t spread3(uint64_t x) {
     return x;
 }
 
+__device__ __forceinline__ uint64_t morton_code(f3 lo, f3 hi, f3 slo, f3 shi) {
+    f3 centroid = ((lo + hi) * 0.5f - (slo + shi) * 0.5f) / (shi - slo);
+    uint64_t factor = (uint64_t)(1L << 21);
+    uint64_t x = centroid.x * factor;
+    uint64_t y = centroid.y * factor;
+    uint64_t z = centroid.z * factor;
+    return (spread3(x) << 2) | (spread3(y) << 1) | spread3(z);
+}
+
 __global__ void __launch_bounds__(kThreads) k_morton(const float* __restrict__ box, int64_t n, const float* dev_bounds,
                                                      Bounds6 host_bounds, int use_dev, uint64_t* __restrict__ codes,
                                                      uint64_t* __restrict__ codes_copy, uint32_t* __restrict__ vals) {
@@ -155,13 +164,7 @@ __global__ void __launch_bounds__(kThreads) k_morton(const float* __restrict__ b
         shi = mk(host_bounds.v[3], host_bounds.v[4], host_bounds.v[5]);
     }
     const float* b = box + 6 * i;
-    f3 lo = mk(b[0], b[1], b[2]), hi = mk(b[3], b[4], b[5]);
-    f3 centroid = ((lo + hi) * 0.5f - (slo + shi) * 0.5f) / (shi - slo);
-    uint64_t factor = (uint64_t)(1L << 21);
-    uint64_t x = centroid.x * factor;
-    uint64_t y = centroid.y * factor;
-    uint64_t z = centroid.z * factor;
-    uint64_t code = (spread3(x) << 2) | (spread3(y) << 1) | spread3(z);
+    const uint64_t code = morton_code(mk(b[0], b[1], b[2]), mk(b[3], b[4], b[5]), slo, shi);
     codes[i] = code;
     codes_copy[i] = code;
     vals[i] = (uint32_t)i;
@@ -390,8 +393,13 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const uint64_t* __res
 // commonPrefixLength, BVH/BVH.cu:101-120, via count-leading-zeros: codes use bits 0..62,
 // so differing codes give clz(a^b)-1 equal leading bits; equal codes fall back to
 // 63 + the equal leading bits of the 32-bit indices (95 when i == j).
-__device__ inline int cpl(const uint64_t* __restrict__ m, uint64_t mi, uint32_t i, uint32_t j) {
-    uint64_t mj = __ldg(m + j);
+struct GlobalCodes {  // sorted codes that this kernel does not write
+    const uint64_t* __restrict__ m;
+    __device__ __forceinline__ uint64_t operator[](int64_t i) const { return __ldg(m + i); }
+};
+template <typename Codes>
+__device__ inline int cpl(Codes m, uint64_t mi, uint32_t i, uint32_t j) {
+    uint64_t mj = m[j];
     if (mi != mj) return __clzll((long long)(mi ^ mj)) - 1;
     return 63 + __clz((int)(i ^ j));
 }
@@ -401,9 +409,9 @@ __device__ inline int cpl(const uint64_t* __restrict__ m, uint64_t mi, uint32_t 
 // search, and the `rightChild == leavesCount - 1` leaf clause), writing straight into
 // the merged node layout of mergeNodesArray (BVH/BVH.cu:273-302): internal i at i,
 // leaf j at N-1+j.
-__device__ inline void radix_node(const uint64_t* __restrict__ m, int32_t N, BNode* __restrict__ nodes, int32_t i,
-                                  int* err) {
-    const uint64_t mi = __ldg(m + i);
+template <typename Codes>
+__device__ inline void radix_node(Codes m, int32_t N, BNode* __restrict__ nodes, int32_t i, int* err) {
+    const uint64_t mi = m[i];
     int d = 1;
     if (i > 0) d = (cpl(m, mi, i, i + 1) - cpl(m, mi, i, i - 1)) >= 0 ? 1 : -1;
     int minCPL = 0;
@@ -456,7 +464,7 @@ __global__ void __launch_bounds__(kThreads) k_radix_tree(const uint64_t* __restr
                                                          BNode* __restrict__ nodes, int* err) {
     int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N - 1) return;
-    radix_node(m, N, nodes, i, err);
+    radix_node(GlobalCodes{m}, N, nodes, i, err);
 }
 
 // Leaf records (fillLeafBoundingBoxes + copyLeafNode, BVH/BVH.cu:46-56, 261-271) and
@@ -465,7 +473,7 @@ __global__ void __launch_bounds__(kThreads) k_radix_tree(const uint64_t* __restr
 // after an acquire fence; writes are published with a release fence before the
 // arrival counter is bumped (the reference has no fence here).
 // box_index: the leaf's triangle in `box`; prim: the triangle id the leaf records
-__device__ inline void refit_leaf(const float* __restrict__ box, uint32_t box_index, int32_t prim, int32_t N,
+__device__ inline void refit_leaf(const float* box, uint32_t box_index, int32_t prim, int32_t N,
                                   BNode* nodes, uint32_t* visited, int32_t j, int* err) {
     const uint32_t t = box_index;
     const float* b = box + 6 * (size_t)t;
@@ -692,6 +700,153 @@ __global__ void k_poison_tree(const int* err, TNode* tnodes, TriRec* tris) {
     if (threadIdx.x == 0 && (*err & kErrStructural)) poison_tree(tnodes, tris);
 }
 
+// ------------------------------------------------------------ small trees
+// Up to kSmallTris triangles, one block builds the whole LBVH and one more lays it out: the
+// stages above are a few microseconds of work there, and their 24 launches and memsets were
+// latency (36 triangles without treelet rounds 0.165 -> 0.071 ms, 1,000 with three rounds 0.88 ->
+// 0.72).  The codes, their order and the tree are the same: a
+// bitonic sort by (code, index) is the stable sort by code.
+constexpr int kSmallTris = 2048;
+constexpr int kSmallThreads = 1024;
+static_assert(kScanThreads == kSmallThreads, "block_excl_scan's warp count");
+
+struct SmallSmem {
+    uint64_t key[kSmallTris];
+    uint32_t val[kSmallTris];
+    float box[6 * kSmallTris];
+    int32_t bounds[6];
+};
+
+struct SharedCodes {
+    const uint64_t* m;
+    __device__ __forceinline__ uint64_t operator[](int64_t i) const { return m[i]; }
+};
+
+__global__ void __launch_bounds__(kSmallThreads) k_build_small(const float* __restrict__ pos, const int32_t* __restrict__ idx,
+                                                               int32_t n, int64_t nv, Bounds6 host_bounds, int use_dev,
+                                                               BNode* nodes, uint64_t* codes_unsorted,
+                                                               uint64_t* codes_sorted, int32_t* perm, uint32_t* visited,
+                                                               int* err) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    SmallSmem& S = *reinterpret_cast<SmallSmem*>(smem_raw);
+    const int tid = threadIdx.x;
+    if (tid < 6) S.bounds[tid] = tid < 3 ? INT32_MAX : INT32_MIN;
+    if (tid < 8) err[tid] = 0;
+    for (int i = tid; i < n - 1; i += kSmallThreads) visited[i] = 0;
+    __syncthreads();
+    // leaf boxes and the scene's bounds (k_leaf_boxes)
+    for (int i0 = 0; i0 < n; i0 += kSmallThreads) {
+        const int i = i0 + tid;
+        float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+        bool valid = i < n;
+        if (valid) {
+            int32_t a, b, c;
+            valid = load_tri_idx(idx, i, nv, a, b, c, err);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const float v0 = __ldg(pos + 3 * (int64_t)a + k), v1 = __ldg(pos + 3 * (int64_t)b + k),
+                            v2 = __ldg(pos + 3 * (int64_t)c + k);
+                S.box[6 * i + k] = lo[k] = fminf(v0, fminf(v1, v2));
+                S.box[6 * i + 3 + k] = hi[k] = fmaxf(v0, fmaxf(v1, v2));
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int32_t l = __reduce_min_sync(0xffffffffu, valid ? f2ord(lo[k]) : INT32_MAX);
+            const int32_t h = __reduce_max_sync(0xffffffffu, valid ? f2ord(hi[k]) : INT32_MIN);
+            if ((tid & 31) == 0) {
+                atomicMin(&S.bounds[k], l);
+                atomicMax(&S.bounds[3 + k], h);
+            }
+        }
+    }
+    __syncthreads();
+    f3 slo, shi;
+    if (use_dev) {
+        slo = mk(ord2f(S.bounds[0]), ord2f(S.bounds[1]), ord2f(S.bounds[2]));
+        shi = mk(ord2f(S.bounds[3]), ord2f(S.bounds[4]), ord2f(S.bounds[5]));
+    } else {
+        slo = mk(host_bounds.v[0], host_bounds.v[1], host_bounds.v[2]);
+        shi = mk(host_bounds.v[3], host_bounds.v[4], host_bounds.v[5]);
+    }
+    int padded = 2;
+    while (padded < n) padded *= 2;
+    for (int i = tid; i < padded; i += kSmallThreads) {
+        uint64_t code = ~0ull;  // past every code (63 bits)
+        if (i < n) {
+            const float* b = S.box + 6 * i;
+            code = morton_code(mk(b[0], b[1], b[2]), mk(b[3], b[4], b[5]), slo, shi);
+            codes_unsorted[i] = code;
+        }
+        S.key[i] = code;
+        S.val[i] = (uint32_t)i;
+    }
+    // bitonic sort by (code, index): at most one pair per thread and step
+    for (int size = 2; size <= padded; size *= 2)
+        for (int step = size / 2; step > 0; step /= 2) {
+            __syncthreads();
+            if (tid < padded / 2) {
+                const int i = 2 * tid - (tid & (step - 1)), j = i + step;
+                const uint64_t a = S.key[i], b = S.key[j];
+                const uint32_t va = S.val[i], vb = S.val[j];
+                const bool greater = a > b || (a == b && va > vb);
+                if (greater == ((i & size) == 0)) {
+                    S.key[i] = b;
+                    S.key[j] = a;
+                    S.val[i] = vb;
+                    S.val[j] = va;
+                }
+            }
+        }
+    __syncthreads();
+    for (int i = tid; i < n; i += kSmallThreads) {
+        codes_sorted[i] = S.key[i];
+        perm[i] = (int32_t)S.val[i];
+    }
+    for (int i = tid; i < n - 1; i += kSmallThreads) radix_node(SharedCodes{S.key}, n, nodes, i, err);
+    __threadfence();
+    __syncthreads();
+    for (int j = tid; j < n; j += kSmallThreads)
+        refit_leaf(S.box, S.val[j], (int32_t)S.val[j], n, nodes, visited, j, err);
+}
+
+// The traversal layout of a small tree (the kernels above in one block), and the build's end:
+// a tree whose build failed is made safe to trace, the error words join the context's.
+__global__ void __launch_bounds__(kSmallThreads) k_layout_small(const float* __restrict__ pos, int64_t nv,
+                                                                const int32_t* __restrict__ idx,
+                                                                const int32_t* __restrict__ mesh,
+                                                                const uint32_t* __restrict__ perm, int32_t n,
+                                                                const BNode* __restrict__ nodes, TNode* tnodes, TriRec* tris,
+                                                                float* root_box, const int* err, int* ctx_err) {
+    __shared__ int32_t compact[2 * kSmallTris];
+    __shared__ int32_t slot_of[kSmallTris];
+    __shared__ uint32_t wsum[32];
+    const int tid = threadIdx.x, count = 2 * n - 1;
+    constexpr int kItems = 2 * kSmallTris / kSmallThreads;
+    uint32_t c = 0;
+    bool in[kItems];
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+        const int x = tid * kItems + k;
+        in[k] = x < count && !nodes[x].is_leaf;
+        c += in[k];
+    }
+    uint32_t e = block_excl_scan(c, wsum, nullptr);
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+        const int x = tid * kItems + k;
+        if (x < count) compact[x] = in[k] ? (int32_t)(e++) : -1;
+    }
+    for (int j = tid; j < n; j += kSmallThreads) tri_layout(pos, nv, idx, mesh, perm, n, tris, slot_of, j);
+    __syncthreads();
+    for (int x = tid; x < count; x += kSmallThreads) tnode_layout(nodes, count, compact, slot_of, tnodes, root_box, x);
+    __syncthreads();
+    if (tid == 0) {
+        if (*err & kErrStructural) poison_tree(tnodes, tris);
+        if (*err != 0) atomicOr(ctx_err, *err);
+    }
+}
+
 template <typename T>
 T* carve(unsigned char*& p, size_t count) {
     size_t off = ((uintptr_t)p + 255) & ~(uintptr_t)255;
@@ -821,6 +976,28 @@ cav_status build_bvh(cav_ctx* ctx, const float* positions, int64_t nv, const int
     for (int k = 0; k < 7; ++k) cudaEventCreate(&bvh->ev[k]);
     bvh->timed = true;
 
+    Bounds6 hb{};
+    if (bounds)
+        for (int k = 0; k < 6; ++k) hb.v[k] = bounds[k];
+    if (n <= kSmallTris) {
+        CAV_CUDA(ctx, cudaFuncSetAttribute(k_build_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmallSmem)));
+        cudaEventRecord(bvh->ev[0], s);
+        k_build_small<<<1, kSmallThreads, sizeof(SmallSmem), s>>>(positions, indices, (int32_t)n, nv, hb, bounds ? 0 : 1,
+                                                                  bvh->nodes, bvh->codes_unsorted, bvh->codes_sorted,
+                                                                  bvh->perm, visited, err);
+        for (int k = 1; k <= 4; ++k) cudaEventRecord(bvh->ev[k], s);  // one kernel: the first stage's time is all four's
+        CAV_CUDA(ctx, cudaGetLastError());
+        cav_status st = treelet_rounds(ctx, bvh->nodes, n, rounds, leaf_list, visited, counters + 14, s);
+        if (st != CAV_OK) return st;
+        cudaEventRecord(bvh->ev[5], s);
+        k_layout_small<<<1, kSmallThreads, 0, s>>>(positions, nv, indices, mesh_ids, (const uint32_t*)bvh->perm, (int32_t)n,
+                                                   bvh->nodes, bvh->tnodes, bvh->tris, bvh->d_root_box, err, ctx->d_error);
+        cudaEventRecord(bvh->ev[6], s);
+        CAV_CUDA(ctx, cudaGetLastError());
+        CAV_CUDA(ctx, cudaFreeAsync(sbase, s));
+        *out = bvh;
+        return CAV_OK;
+    }
     CAV_CUDA(ctx, cudaMemsetAsync(hist, 0, sizeof(uint32_t) * 8 * 256, s));
     CAV_CUDA(ctx, cudaMemsetAsync(status, 0, sizeof(uint32_t) * 8 * (size_t)tiles * 256, s));
     CAV_CUDA(ctx, cudaMemsetAsync(counters, 0, sizeof(uint32_t) * 16, s));
@@ -831,10 +1008,8 @@ cav_status build_bvh(cav_ctx* ctx, const float* positions, int64_t nv, const int
     cudaEventRecord(bvh->ev[0], s);
     int32_t* bounds_ord = (int32_t*)(counters + 8);
     const int gb = div_up(n, kThreads);
-    Bounds6 hb{};
     int use_dev = bounds ? 0 : 1;
     if (bounds) {
-        for (int k = 0; k < 6; ++k) hb.v[k] = bounds[k];
         k_leaf_boxes<<<gb, kThreads, 0, s>>>(positions, indices, n, nv, leafbox, nullptr, err);
     } else {
         k_bounds_init<<<1, 32, 0, s>>>(bounds_ord);
@@ -990,13 +1165,7 @@ __global__ void __launch_bounds__(kThreads) k_morton_batch(const float* __restri
     const float* bb = S.use_dev ? dev_bounds + 6 * sg : S.bounds;
     f3 slo = mk(bb[0], bb[1], bb[2]), shi = mk(bb[3], bb[4], bb[5]);
     const float* b = box + 6 * g;
-    f3 lo = mk(b[0], b[1], b[2]), hi = mk(b[3], b[4], b[5]);
-    f3 centroid = ((lo + hi) * 0.5f - (slo + shi) * 0.5f) / (shi - slo);  // as k_morton
-    uint64_t factor = (uint64_t)(1L << 21);
-    uint64_t x = centroid.x * factor;
-    uint64_t y = centroid.y * factor;
-    uint64_t z = centroid.z * factor;
-    uint64_t code = (spread3(x) << 2) | (spread3(y) << 1) | spread3(z);
+    const uint64_t code = morton_code(mk(b[0], b[1], b[2]), mk(b[3], b[4], b[5]), slo, shi);
     codes[g] = code;
     codes_copy[g] = code;
     vals[g] = (uint32_t)g;
@@ -1029,7 +1198,7 @@ __global__ void __launch_bounds__(kThreads) k_radix_batch(const BuildSeg* segs, 
     if (g >= total_internal) return;
     const int sg = find_off(int_offs, K, g);
     const BuildSeg& S = segs[sg];
-    radix_node(S.codes_sorted, (int32_t)S.n, S.nodes, (int32_t)(g - int_offs[sg]), err);
+    radix_node(GlobalCodes{S.codes_sorted}, (int32_t)S.n, S.nodes, (int32_t)(g - int_offs[sg]), err);
 }
 
 __global__ void __launch_bounds__(kThreads) k_refit_batch(const float* __restrict__ box, const uint32_t* vals,
