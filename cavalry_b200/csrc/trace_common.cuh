@@ -135,16 +135,49 @@ __device__ inline void flush_stats(const TraceStats& st, unsigned long long* sta
 }
 
 // Blocks of a persistent traversal launch: every SM filled to the kernel's occupancy (or
-// the context's configured blocks per SM).
+// the context's configured blocks per SM).  The occupancy query costs a microsecond or two of
+// the launch, so each host thread remembers its last answers.
 template <typename K>
 int grid_for(cav_ctx* ctx, K kernel, int block, size_t dyn_smem = 0) {
     if (dyn_smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_smem);
     int per_sm = ctx->trace_blocks_per_sm;
     if (per_sm <= 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, dyn_smem);
-        if (per_sm < 1) per_sm = 1;
+        struct Known {
+            const void* kernel;
+            size_t dyn;
+            int block, device, per_sm;
+        };
+        thread_local Known known[16] = {};
+        thread_local int next = 0;
+        for (const Known& k : known)
+            if (k.kernel == (const void*)kernel && k.dyn == dyn_smem && k.block == block && k.device == ctx->device)
+                per_sm = k.per_sm;
+        if (per_sm <= 0) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, dyn_smem);
+            if (per_sm < 1) per_sm = 1;
+            known[next] = Known{(const void*)kernel, dyn_smem, block, ctx->device, per_sm};
+            next = (next + 1) & 15;
+        }
     }
     return ctx->num_sms * per_sm;
+}
+
+// Rays a warp holds at least, when there are rays enough: fewer would leave most of each
+// instruction idle.  With rays for every warp of the grid in one go, warp w takes rays [w cap,
+// (w + 1) cap) and no others, and the work counter is not used (nor cleared by the launch).
+__device__ __forceinline__ int warp_share(int64_t n, int min_cap, bool& once) {
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    const int cap = (int)min((int64_t)32, max((int64_t)min_cap, (n + warps - 1) / warps));
+    once = n <= warps * cap;
+    return cap;
+}
+
+// The launch's side of it: the blocks that n rays need, and whether the counter will be used.
+inline int share_grid(int64_t n, int min_cap, int block, int grid, bool& counted) {
+    const int64_t warps = (n + min_cap - 1) / min_cap, per_block = block / 32;
+    grid = (int)(warps / per_block + 1 < grid ? (warps + per_block - 1) / per_block : grid);
+    counted = n > (int64_t)grid * per_block * 32;
+    return grid;
 }
 
 }  // namespace cav

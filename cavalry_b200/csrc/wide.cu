@@ -565,9 +565,8 @@ __global__ void __maxnreg__(kExact && !kAny ? 72 : 64)
         __syncthreads();
     }
     if (!kSeg && one.n_dev) n = *one.n_dev;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    const int cap = (int)min((int64_t)32, max((int64_t)min_cap, (n + warps - 1) / warps));
-    const bool once = n <= warps * cap;  // every ray fits: warp w takes rays [w cap, (w + 1) cap) and no others
+    bool once;
+    const int cap = warp_share(n, min_cap, once);
     ShareRec& sh = shares[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const CNode* __restrict__ cn = one.cnodes;
@@ -1040,9 +1039,7 @@ __global__ void __maxnreg__(kExact && !kAny ? 72 : 64)
     flush_stats<kStats>(st, stats);
 }
 
-// Rays a warp holds at least, when there are rays enough: fewer would leave most of each
-// instruction idle while the queue lasts.
-constexpr int kMinCap = 4;
+constexpr int kMinCap = 4;  // rays a warp holds at least (fewer leave most of each instruction idle)
 
 template <bool kAny, bool kStats, bool kSeg, bool kExact, int kSmemN>
 cav_status launch_one(cav_ctx* ctx, const TraceSeg& one, const TraceSeg* segs, int nseg, int64_t n, int block, int batch,
@@ -1050,11 +1047,9 @@ cav_status launch_one(cav_ctx* ctx, const TraceSeg& one, const TraceSeg* segs, i
     const size_t dyn = sizeof(uint2) * kSmemN * (size_t)block;
     auto* kernel = k_trace_wide<kAny, kStats, kSeg, kExact, kSmemN>;
     int grid = grid_for(ctx, kernel, block, dyn);
-    if (!one.n_dev) {
-        const int64_t warps = (n + kMinCap - 1) / kMinCap;
-        grid = (int)std::min<int64_t>(grid, (warps + block / 32 - 1) / (block / 32));
-    }
-    CAV_CUDA(ctx, cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s));
+    bool counted = true;
+    if (!one.n_dev) grid = share_grid(n, kMinCap, block, grid, counted);
+    if (counted) CAV_CUDA(ctx, cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s));
     kernel<<<grid, block, dyn, s>>>(one, segs, nseg, n, counter, batch, kMinCap, ctx->max_trace_steps,
                                     ctx->d_error + (kAny ? 3 : 2), stats);
     CAV_CUDA(ctx, cudaGetLastError());
