@@ -902,7 +902,8 @@ cav_status alloc_bvh(cav_ctx* ctx, int64_t n, cudaStream_t s, cav_bvh** out) {
 }
 
 // Releases a tree: its events, its fast-mode view and its arena (or its share of a batch's
-// arena, freed with the last tree of the batch).  async: stream-ordered frees on `s`.
+// arena, freed with the last tree of the batch).  async: stream-ordered frees on `s`; else the
+// device's work so far is waited for, since the tree may be in use on any stream.
 void bvh_release(cav_bvh* bvh, cudaStream_t s, bool async) {
     if (!bvh) return;
     if (bvh->timed)
@@ -916,10 +917,7 @@ void bvh_release(cav_bvh* bvh, cudaStream_t s, bool async) {
             delete bvh->shared;
         }
     }
-    if (mem) {
-        if (async) cudaFreeAsync(mem, s);
-        else cudaFree(mem);
-    }
+    if (mem) release_memory(mem, s, async);
     delete bvh;
 }
 

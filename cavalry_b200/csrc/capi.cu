@@ -27,6 +27,17 @@ cudaError_t dev_alloc(cav_ctx* ctx, void** p, size_t bytes, cudaStream_t s, bool
     return async ? cudaMallocAsync(p, bytes, s) : cudaMalloc(p, bytes);
 }
 
+// cudaFree waits for nothing when the memory came from a pool: the driver takes it as no longer
+// in use and may unmap or reuse it under a kernel that still reads it.
+void release_memory(void* p, cudaStream_t s, bool async) {
+    if (async) {
+        cudaFreeAsync(p, s);
+        return;
+    }
+    cudaDeviceSynchronize();
+    cudaFree(p);
+}
+
 cav_status cuda_error(cav_ctx* ctx, cudaError_t e, const char* what) {
     std::string m = std::string(what) + ": " + cudaGetErrorString(e);
     cudaGetLastError();

@@ -200,6 +200,8 @@ cav_status cuda_error(cav_ctx* ctx, cudaError_t e, const char* what);
 // Fails with cudaErrorMemoryAllocation while the context's injected allocation failures last
 // (cav_ctx_inject), so the error paths of every caller can be tested without exhausting HBM.
 cudaError_t dev_alloc(cav_ctx* ctx, void** p, size_t bytes, cudaStream_t s, bool async);
+// Frees memory of the device's pool: on the stream, or once all of the device's work is done.
+void release_memory(void* p, cudaStream_t s, bool async);
 
 // build.cu
 // Releases a tree (cav_bvh_free); async: stream-ordered frees on `s`, for callers (the

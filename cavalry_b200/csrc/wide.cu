@@ -1148,7 +1148,7 @@ cav_status ensure_wide(cav_ctx* ctx, const cav_bvh* bvh, cudaStream_t s) {
     else if (h->failed || h->tris != (uint32_t)n)
         st = set_error(ctx, CAV_ERR_CUDA, "fast traversal layout: not every triangle placed");
     if (st != CAV_OK) {
-        cudaFree(arena);
+        cudaFreeAsync(arena, s);
         return st;
     }
     bvh->wide_arena = arena;
@@ -1160,10 +1160,7 @@ cav_status ensure_wide(cav_ctx* ctx, const cav_bvh* bvh, cudaStream_t s) {
 }
 
 void free_wide(cav_bvh* bvh, cudaStream_t s, bool async) {
-    if (bvh->wide_arena) {
-        if (async) cudaFreeAsync(bvh->wide_arena, s);
-        else cudaFree(bvh->wide_arena);
-    }
+    if (bvh->wide_arena) release_memory(bvh->wide_arena, s, async);
     bvh->wide_arena = nullptr;
     bvh->cnodes = nullptr;
     bvh->ctris = nullptr;

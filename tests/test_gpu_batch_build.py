@@ -57,3 +57,46 @@ def test_many_small_scenes_with_treelet_rounds():
         assert batch[k].export_nodes().tobytes() == single.export_nodes().tobytes(), (k, sizes[k])
         single.free()
     ctx.sync_check()
+
+
+def test_trees_freed_while_they_are_traced():
+    """Trees freed right after their queries were launched, and others of other sizes built at
+    once, on the default and on a side stream: the memory is given back only once the queries
+    are through, so their hits are those of trees that were kept."""
+    import torch
+
+    import cavalry_b200 as cav
+    from cavalry_b200 import scenes
+
+    ctx = cav.Context(0)
+    rays = torch.from_numpy(scenes.closest_rays(200_000, seed=6)).cuda()
+    groups = []
+    for g, sizes in enumerate([[30000, 2000, 500], [9000, 15000, 700, 41], [60000, 130]]):
+        data = [scenes.soup(n, seed=70 + 10 * g + k) for k, n in enumerate(sizes)]
+        groups.append([(torch.from_numpy(p).cuda(), torch.from_numpy(i).cuda()) for p, i in data])
+    want = []
+    for dev in groups:
+        trees = ctx.build_batch(dev, rounds=1)
+        want.append([t.trace_closest(rays) for t in trees])
+        ctx.sync_check()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    for stream in (torch.cuda.current_stream(), side):
+        with torch.cuda.stream(stream):
+            got = []
+            for _ in range(3):
+                for dev in groups:
+                    trees = ctx.build_batch(dev, rounds=1)
+                    got.append([t.trace_closest(rays) for t in trees])
+                    for t in trees:
+                        t.free()
+                    p, i = dev[0]
+                    one = ctx.build(p, i, rounds=1)
+                    got[-1].append(one.trace_closest(rays))
+                    one.free()
+        torch.cuda.synchronize()
+        for at, hits in enumerate(got):
+            ref = want[at % len(groups)]
+            for a, b in zip(hits, ref + ref[:1]):
+                assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+    ctx.sync_check()
