@@ -908,6 +908,11 @@ void bvh_release(cav_bvh* bvh, cudaStream_t s, bool async) {
     if (!bvh) return;
     if (bvh->timed)
         for (int k = 0; k < 7; ++k) cudaEventDestroy(bvh->ev[k]);
+    if (bvh->shared) {
+        std::lock_guard<std::mutex> lk(bvh->shared->mu);
+        auto& t = bvh->shared->trees;
+        if ((size_t)bvh->shared_at < t.size()) t[bvh->shared_at] = nullptr;
+    }
     free_wide(bvh, s, async);
     void* mem = bvh->arena;
     if (bvh->shared) {
@@ -1329,6 +1334,7 @@ cav_status build_bvh_batch(cav_ctx* ctx, int K, const float* const* positions, c
             p = (unsigned char*)(((uintptr_t)p + 255) & ~(uintptr_t)255);
             bv[k] = carve_bvh(ctx, num_triangles[k], p);
             bv[k]->shared = shared;
+            bv[k]->shared_at = k;
             p += bvh_arena_bytes(num_triangles[k]);
         }
     }
@@ -1484,6 +1490,7 @@ cav_status build_bvh_batch(cav_ctx* ctx, int K, const float* const* positions, c
     CAV_CUDA(ctx, cudaGetLastError());
     k_merge_error<<<1, 32, 0, s>>>(err, ctx->d_error);
     CAV_CUDA(ctx, cudaFreeAsync(sbase, s));
+    shared->trees.assign(bv.begin(), bv.end());  // complete: their views may be built together
     for (int k = 0; k < K; ++k) out[k] = bv[k];
     return CAV_OK;
 }

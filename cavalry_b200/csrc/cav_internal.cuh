@@ -12,6 +12,7 @@
 #include <atomic>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include "../../include/cavalry.h"
 
@@ -113,6 +114,7 @@ static_assert(sizeof(TriRec) == 48, "TriRec must be 48 bytes");
 }  // namespace cav
 
 // ------------------------------------------------------------ host objects
+struct cav_bvh;
 struct cav_ctx {
     int device = 0;
     int num_sms = 148;
@@ -155,10 +157,13 @@ struct cav_ctx {
 };
 
 namespace cav {
-// A device allocation shared by the trees of one batched build; the last tree released frees it.
+// A device allocation shared by trees; the last tree released frees it.
 struct SharedArena {
     void* p = nullptr;
     std::atomic<int> refs{0};
+    // of a batched build: its trees, null once released (their views are built together, wide.cu)
+    std::mutex mu;
+    std::vector<const cav_bvh*> trees;
 };
 }  // namespace cav
 
@@ -178,6 +183,7 @@ struct cav_bvh {
     mutable cav::TriRec* ctris = nullptr;  // triangles in wide-leaf order
     mutable float4* lbox = nullptr;  // two per triangle of ctris: its box in the binary tree
     mutable void* wide_arena = nullptr;
+    mutable cav::SharedArena* wide_shared = nullptr;  // the view's arena when it was built with others
     // 0: no view; 1: a view the exact mode does not use; 2: one it does; -1: none could be made for it
     mutable std::atomic<int> wide_state{0};
     mutable std::atomic<int64_t> rays_seen{0};  // exact-mode rays before there was a view
@@ -190,6 +196,7 @@ struct cav_bvh {
     bool timed = false;
     void* arena = nullptr;  // one allocation holding the arrays above (null when shared)
     cav::SharedArena* shared = nullptr;  // the batch's arena the arrays live in, or null
+    int shared_at = 0;                   // this tree among the batch's
 };
 
 namespace cav {

@@ -100,3 +100,32 @@ def test_trees_freed_while_they_are_traced():
             for a, b in zip(hits, ref + ref[:1]):
                 assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
     ctx.sync_check()
+
+
+@pytest.mark.parametrize("sizes", [[65536, 65537, 2, 300], [129], [65537, 200, 70000], [2, 3, 128, 129, 2000]])
+def test_views_of_a_batch_equal_single_views(sizes):
+    """The 8-wide views of a batch's trees, built together (trees of at most 65,536 triangles
+    that are still there, two or more of them) or alone: hits equal those of the scenes' own
+    trees in both modes."""
+    import torch
+
+    import cavalry_b200 as cav
+    from cavalry_b200 import scenes
+
+    ctx = cav.Context(0)
+    data = [scenes.soup(n, seed=500 + k) for k, n in enumerate(sizes + [400])]
+    dev = [(torch.from_numpy(p).cuda(), torch.from_numpy(i).cuda()) for p, i in data]
+    batch = ctx.build_batch(dev, rounds=1)
+    batch.pop().free()  # before any view was built
+    rays = torch.from_numpy(scenes.closest_rays(3000, seed=7)).cuda()
+    limit = torch.full((3000,), 0.6, device="cuda")
+    for k, tree in enumerate(batch):
+        single = ctx.build(*dev[k], rounds=1)
+        for flags in (cav.TRACE_EXACT, cav.TRACE_FAST):
+            for x, y in zip(tree.trace_closest(rays, flags=flags), single.trace_closest(rays, flags=flags)):
+                assert torch.equal(x, y), (k, flags)
+            assert torch.equal(tree.trace_any(rays, limit, flags=flags), single.trace_any(rays, limit, flags=flags))
+        if k % 2:
+            tree.free()
+        single.free()
+    ctx.sync_check()
