@@ -376,11 +376,22 @@ cav_status cav_trace_stats(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays
 // ------------------------------------------------------------ host-buffer path
 namespace {
 
-// Rays per pipelined chunk.  Every traversal launch ends in a tail while its last, longest
-// rays finish (about 4.7 ms on the 1M-triangle soup), so chunks are large: 4M rays of the
-// soup take 68.4 ms through the host path in one chunk against 76.9 ms in four chunks of 1M
-// (64.9 ms of traversal alone).
+// Rays per pipelined chunk: at most what the staging slots hold.
 constexpr int64_t kChunkRays = (int64_t)1 << 22;
+
+// Of a call that is cut for the sake of its copies, up to four chunks of 2^18 rays or more: the
+// first chunk's copy in and the last one's copy out overlap nothing.  Any-hit calls are (their
+// traversal takes no longer than their copies), and calls with pageable buffers, which the host
+// copies itself: 1M shadow rays on 200,000 triangles 1.79 ms in one chunk, 1.50 in three,
+// pageable 5.1 and 3.2; 4M on 1M triangles 8.8 and 6.8 in four; pageable closest hits on 200,000
+// triangles 9.1 and 6.6.  Closest hits of pinned buffers are not: every chunk's traversal ends in
+// a tail of its longest rays, which the next chunk's only partly hides (1M rays on 1M triangles
+// 11.0 ms in one chunk, 11.9 in three; on 200,000 triangles 3.97 and 3.86).
+int64_t chunk_rays(int64_t n, bool cut) {
+    const int64_t parts = cut ? std::clamp<int64_t>(n >> 18, 1, 4) : 1;
+    return std::min(kChunkRays, (n + parts - 1) / parts);
+}
+
 // per-ray staging bytes: ray 32 + limit 4 + excl 8 in; prim 4 + t 4 + uv 8 (or occ 1) out
 constexpr size_t kInBytes = 32 + 4 + 8;
 constexpr size_t kOutBytes = 16;
@@ -448,8 +459,8 @@ Slot slot_of(cav_ctx* ctx, int k) {
 // on two streams.  Inputs already in pinned memory are copied directly; pageable
 // inputs and outputs go through the context's pinned slots.
 template <typename Launch, typename Finish>
-cav_status host_pipeline(cav_ctx* ctx, int64_t n, Launch launch, Finish finish) {
-    const int64_t chunks = (n + kChunkRays - 1) / kChunkRays;
+cav_status host_pipeline(cav_ctx* ctx, int64_t n, int64_t chunk, Launch launch, Finish finish) {
+    const int64_t chunks = (n + chunk - 1) / chunk;
     int64_t pending[2] = {-1, -1};
     for (int64_t c = 0; c < chunks; ++c) {
         const int k = (int)(c & 1);
@@ -489,8 +500,9 @@ cav_status cav_trace_closest_host(cav_ctx* ctx, const cav_bvh* bvh, const cav_ra
     if (st != CAV_OK) return st;
     st = order_after_build(ctx, bvh);
     if (st != CAV_OK) return st;
+    const int64_t chunk = chunk_rays(n, !(in_pinned && out_pinned));
     auto launch = [&](Slot s, int64_t c, cudaStream_t str, unsigned long long* counter) -> cav_status {
-        int64_t b = c * kChunkRays, m = std::min(kChunkRays, n - b);
+        const int64_t b = c * chunk, m = std::min(chunk, n - b);
         if (in_pinned) {
             CAV_CUDA(ctx, cudaMemcpyAsync(s.d_rays, rays + b, 32 * m, cudaMemcpyHostToDevice, str));
         } else {
@@ -516,13 +528,13 @@ cav_status cav_trace_closest_host(cav_ctx* ctx, const cav_bvh* bvh, const cav_ra
     };
     auto finish = [&](Slot s, int64_t c) -> cav_status {
         if (out_pinned) return CAV_OK;
-        int64_t b = c * kChunkRays, m = std::min(kChunkRays, n - b);
+        const int64_t b = c * chunk, m = std::min(chunk, n - b);
         memcpy(prim_id + b, s.h_out, 4 * m);
         if (t) memcpy(t + b, s.h_out + 4 * kChunkRays, 4 * m);
         if (uv) memcpy(uv + 2 * b, s.h_out + 8 * kChunkRays, 8 * m);
         return CAV_OK;
     };
-    return host_pipeline(ctx, n, launch, finish);
+    return host_pipeline(ctx, n, chunk, launch, finish);
 }
 
 cav_status cav_trace_any_host(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays, const float* limit,
@@ -538,8 +550,9 @@ cav_status cav_trace_any_host(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* r
     if (st != CAV_OK) return st;
     st = order_after_build(ctx, bvh);
     if (st != CAV_OK) return st;
+    const int64_t chunk = chunk_rays(n, true);
     auto launch = [&](Slot s, int64_t c, cudaStream_t str, unsigned long long* counter) -> cav_status {
-        int64_t b = c * kChunkRays, m = std::min(kChunkRays, n - b);
+        const int64_t b = c * chunk, m = std::min(chunk, n - b);
         const void* src_r = rays + b;
         const void* src_l = limit ? (const void*)(limit + b) : nullptr;
         const void* src_e = excl_mesh ? (const void*)(excl_mesh + 2 * b) : nullptr;
@@ -568,11 +581,11 @@ cav_status cav_trace_any_host(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* r
     };
     auto finish = [&](Slot s, int64_t c) -> cav_status {
         if (out_pinned) return CAV_OK;
-        int64_t b = c * kChunkRays, m = std::min(kChunkRays, n - b);
+        const int64_t b = c * chunk, m = std::min(chunk, n - b);
         memcpy(occluded + b, s.h_out, m);
         return CAV_OK;
     };
-    return host_pipeline(ctx, n, launch, finish);
+    return host_pipeline(ctx, n, chunk, launch, finish);
 }
 
 }  // extern "C"

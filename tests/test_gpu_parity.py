@@ -319,6 +319,29 @@ def test_host_buffer_path_over_several_chunks(cuda_ctx):
     bvh.free()
 
 
+@pytest.mark.parametrize("n", [(1 << 19) - 1, 1 << 19, 3 * (1 << 18) + 1, (1 << 20) + 3])
+def test_host_buffer_path_in_parts(cuda_ctx, n):
+    """Any-hit calls and calls with pageable buffers are cut into up to four chunks of 2^18
+    rays or more (the last one ragged): one, two, three and four of them."""
+    import torch
+
+    from cavalry_b200 import scenes
+
+    pos, idx = scenes.soup(3000, seed=64)
+    bvh = cuda_ctx.build(torch.from_numpy(pos).cuda(), torch.from_numpy(idx).cuda())
+    rays = scenes.closest_rays(n, seed=65)
+    srays, lim = scenes.shadow_rays(n, seed=66)
+    want = [a.cpu().numpy() for a in bvh.trace_closest(torch.from_numpy(rays).cuda())]
+    occ = bvh.trace_any(torch.from_numpy(srays).cuda(), torch.from_numpy(lim).cuda()).cpu().numpy()
+    for a, b in zip(bvh.trace_closest_host(rays), want):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    assert np.array_equal(bvh.trace_any_host(srays, lim), occ)
+    out = torch.full((n,), 9, dtype=torch.uint8).pin_memory()
+    bvh.trace_any_host(torch.from_numpy(srays).pin_memory(), torch.from_numpy(lim).pin_memory(), out=out)
+    assert np.array_equal(out.numpy(), occ)
+    bvh.free()
+
+
 @pytest.mark.parametrize("n", [7, 8, 50, 1000, 5000])
 @pytest.mark.parametrize("rounds", [1, 3])
 def test_treelets_on_ties_match_oracle(cuda_ctx, n, rounds):
