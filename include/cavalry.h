@@ -101,6 +101,7 @@ cav_status cav_ctx_inject(cav_ctx* ctx, int what, int count);
 cav_status cav_bvh_build(cav_ctx* ctx, const float* positions, int64_t num_vertices, const int32_t* indices,
                          const int32_t* mesh_ids, int64_t num_triangles, const float* scene_bounds, int rounds,
                          void* stream, cav_bvh** out);
+/* Frees a tree; waits for the device where that gives memory back (queries may be running). */
 cav_status cav_bvh_free(cav_bvh* bvh);
 int64_t cav_bvh_num_triangles(const cav_bvh* bvh);
 /* Tree depth (edges from the root to the deepest leaf); synchronises `stream`. */
