@@ -906,7 +906,7 @@ cav_status alloc_bvh(cav_ctx* ctx, int64_t n, cudaStream_t s, cav_bvh** out) {
 // device's work so far is waited for, since the tree may be in use on any stream.
 void bvh_release(cav_bvh* bvh, cudaStream_t s, bool async) {
     if (!bvh) return;
-    if (bvh->timed)
+    if (bvh->timed && !bvh->shared)
         for (int k = 0; k < 7; ++k) cudaEventDestroy(bvh->ev[k]);
     if (bvh->shared) {
         std::lock_guard<std::mutex> lk(bvh->shared->mu);
@@ -919,6 +919,8 @@ void bvh_release(cav_bvh* bvh, cudaStream_t s, bool async) {
         mem = nullptr;
         if (bvh->shared->refs.fetch_sub(1) == 1) {
             mem = bvh->shared->p;
+            if (bvh->timed)
+                for (int k = 0; k < 7; ++k) cudaEventDestroy(bvh->ev[k]);
             delete bvh->shared;
         }
     }
@@ -1238,6 +1240,16 @@ __device__ inline int find_tree(const int64_t* leaf_offs, int K, int64_t g) {
     return lo;
 }
 
+// All nodes of all trees, a thread each.
+__global__ void __launch_bounds__(kThreads) k_zero_nodes_batch(const BuildSeg* segs, const int64_t* leaf_offs, int K,
+                                                               int64_t total_nodes) {
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= total_nodes) return;
+    const int k = find_tree(leaf_offs, K, g);
+    float4* p = reinterpret_cast<float4*>(segs[k].nodes + (g - node_off(leaf_offs, k)));
+    p[0] = p[1] = p[2] = p[3] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
 // compact null: the internal nodes of each block's tile; else their numbers within their trees
 __global__ void __launch_bounds__(kScanThreads) k_number_batch(const BuildSeg* segs, const int64_t* leaf_offs, int K,
                                                                int64_t total, uint32_t* block_counts,
@@ -1366,14 +1378,14 @@ cav_status build_bvh_batch(cav_ctx* ctx, int K, const float* const* positions, c
     size_t scratch = 0;
     auto acc = [&](size_t b) { scratch += b + 256; };
     acc(sizeof(BuildSeg) * K);
-    acc(sizeof(int64_t) * (K + 1) * 2);
+    acc(sizeof(int64_t) * (K + 1) * 2 + 256);       // (an alignment for each of the two)
     acc(sizeof(float) * 6 * total);                 // leaf boxes
-    acc(sizeof(uint64_t) * total * 3);              // codes, codes copy, ping-pong
-    acc(sizeof(uint32_t) * total * 2);              // values ping-pong
+    acc(sizeof(uint64_t) * total * 3 + 512);        // codes, codes copy, ping-pong
+    acc(sizeof(uint32_t) * total * 2 + 256);        // values ping-pong
     acc(sizeof(uint32_t) * 2 * 8 * 256);            // histograms (codes, scene keys)
     acc(sizeof(uint32_t) * (8 + passes2) * (size_t)tiles * 256);  // look-back status
     acc(sizeof(uint32_t) * 32);                     // tile counters
-    acc(sizeof(int32_t) * 6 * K * 2);               // bounds (ordered ints, floats)
+    acc(sizeof(int32_t) * 6 * K * 2 + 256);         // bounds (ordered ints, floats)
     acc(sizeof(int32_t) * 8);                       // error flag
     acc(sizeof(uint32_t) * total_nodes);            // visited (refit, then treelets), then the nodes' numbers
     acc(sizeof(int32_t) * total);                   // treelet seeds, then each triangle's slot
@@ -1421,18 +1433,24 @@ cav_status build_bvh_batch(cav_ctx* ctx, int K, const float* const* positions, c
     CAV_CUDA(ctx, cudaMemsetAsync(counters, 0, sizeof(uint32_t) * 32, s));
     CAV_CUDA(ctx, cudaMemsetAsync(err, 0, sizeof(int32_t) * 8, s));
     CAV_CUDA(ctx, cudaMemsetAsync(visited, 0, sizeof(uint32_t) * total_int, s));
+    // The trees pass every stage together, so they share one set of events, and one launch zeroes
+    // the nodes of all of them: a memset, seven events and seven records for each tree took 48
+    // trees of 1,000 to 30,000 triangles 3.43 ms a build with 3 rounds, so it takes 2.35 (the
+    // host 0.66 and 0.22 ms).
+    cudaEvent_t ev[7];
+    for (int e = 0; e < 7; ++e) cudaEventCreate(&ev[e]);
     for (int k = 0; k < K; ++k) {
-        CAV_CUDA(ctx, cudaMemsetAsync(bv[k]->nodes, 0, sizeof(BNode) * (2 * num_triangles[k] - 1), s));
-        for (int e = 0; e < 7; ++e) cudaEventCreate(&bv[k]->ev[e]);
+        std::copy(ev, ev + 7, bv[k]->ev);
         bv[k]->timed = true;
-        cudaEventRecord(bv[k]->ev[0], s);
     }
+    k_zero_nodes_batch<<<div_up(total_nodes, kThreads), kThreads, 0, s>>>(dsegs, d_leaf, K, total_nodes);
+    cudaEventRecord(ev[0], s);
     const int gb = div_up(total, kThreads);
     if (!bounds) k_bounds_batch<<<div_up(6 * K, 256), 256, 0, s>>>(bounds_ord, K, 1, dbounds);
     k_leaf_boxes_batch<<<gb, kThreads, 0, s>>>(dsegs, d_leaf, K, total, leafbox, bounds_ord, err);
     if (!bounds) k_bounds_batch<<<div_up(6 * K, 256), 256, 0, s>>>(bounds_ord, K, 0, dbounds);
     k_morton_batch<<<gb, kThreads, 0, s>>>(leafbox, dsegs, d_leaf, K, total, dbounds, codes, codes_copy, vals_a);
-    for (int k = 0; k < K; ++k) cudaEventRecord(bv[k]->ev[1], s);
+    cudaEventRecord(ev[1], s);
     // sort by code (8 passes, stable), then by scene (1-2 passes, stable)
     CAV_CUDA(ctx, cudaFuncSetAttribute(k_onesweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem)));
     k_sort_hist<<<std::min(gb, ctx->num_sms * 8), kSortThreads, 0, s>>>(codes, total, 8, hist);
@@ -1462,11 +1480,11 @@ cav_status build_bvh_batch(cav_ctx* ctx, int K, const float* const* positions, c
     }
     CAV_CUDA(ctx, cudaGetLastError());
     k_scatter_batch<<<gb, kThreads, 0, s>>>(codes_copy, vin, dsegs, d_leaf, K, total);
-    for (int k = 0; k < K; ++k) cudaEventRecord(bv[k]->ev[2], s);
+    cudaEventRecord(ev[2], s);
     k_radix_batch<<<div_up(total_int, kThreads), kThreads, 0, s>>>(dsegs, d_int, K, total_int, err);
-    for (int k = 0; k < K; ++k) cudaEventRecord(bv[k]->ev[3], s);
+    cudaEventRecord(ev[3], s);
     k_refit_batch<<<gb, kThreads, 0, s>>>(leafbox, vin, dsegs, d_leaf, d_int, K, total, visited, err);
-    for (int k = 0; k < K; ++k) cudaEventRecord(bv[k]->ev[4], s);
+    cudaEventRecord(ev[4], s);
     CAV_CUDA(ctx, cudaGetLastError());
     // treelet rounds of all scenes (two launches per round and group of scenes), then the
     // traversal layout per scene
@@ -1478,7 +1496,7 @@ cav_status build_bvh_batch(cav_ctx* ctx, int K, const float* const* positions, c
             return fail(st);
         }
     }
-    for (int k = 0; k < K; ++k) cudaEventRecord(bv[k]->ev[5], s);
+    cudaEventRecord(ev[5], s);
     const int nblk = div_up(total_nodes, kScanTile);
     k_number_batch<<<nblk, kScanThreads, 0, s>>>(dsegs, d_leaf, K, total_nodes, blk, nullptr);
     k_scan_blocks<<<1, kScanThreads, 0, s>>>(blk, nblk);
@@ -1486,7 +1504,7 @@ cav_status build_bvh_batch(cav_ctx* ctx, int K, const float* const* positions, c
     k_tri_layout_batch<<<gb, kThreads, 0, s>>>(dsegs, d_leaf, K, total, slot_of);
     k_tnode_layout_batch<<<div_up(total_nodes, kThreads), kThreads, 0, s>>>(dsegs, d_leaf, K, total_nodes, compact, slot_of);
     k_poison_batch<<<div_up(K, 256), 256, 0, s>>>(err, dsegs, K);
-    for (int k = 0; k < K; ++k) cudaEventRecord(bv[k]->ev[6], s);
+    cudaEventRecord(ev[6], s);
     CAV_CUDA(ctx, cudaGetLastError());
     k_merge_error<<<1, 32, 0, s>>>(err, ctx->d_error);
     CAV_CUDA(ctx, cudaFreeAsync(sbase, s));
