@@ -18,6 +18,7 @@
 // mode: the quantised boxes contain the exact ones with a margin, so the closest-hit
 // distance is the same and only the choice between triangles at an equal distance may
 // differ; the any-hit answer is the same.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -321,10 +322,12 @@ __global__ void __launch_bounds__(kBuildThreads)
                 (blockIdx.x * blockDim.x + threadIdx.x) >> 3, (gridDim.x * blockDim.x) >> 3, gridDim.x);
 }
 
-// The views of many small trees (a batched build's), a block each: a tree's levels are a chain of
-// fetches, so one tree keeps the chip idle, and a launch, a copy back and a wait for each cost
-// more than its view.  48 trees of 1,000 to 30,000 triangles, built, viewed and asked 2,048
-// closest hits each: 8.6 ms with a view at a time (31 of them, 65 us each), 6.9 ms so.
+// The views of many small trees (a batched build's), a cluster of four blocks each (co-resident, as
+// the levels' barriers need): a tree's levels are a chain of fetches, so one tree keeps the chip
+// idle, and a launch, a copy back and a wait for each cost more than its view.  48 trees of 1,000 to
+// 30,000 triangles, asked 2,048 closest hits each after their build: 5.1 ms with a view at a time
+// (31 of them, 65 us each), 3.25 with a block for each tree, 2.87, 2.67 and 2.62 with two, four
+// and eight blocks.
 struct WideTree {
     const TNode* tn;
     const TriRec* tris_in;
@@ -336,17 +339,22 @@ struct WideTree {
     uint32_t tris;
 };
 constexpr int kGroupThreads = 512;
+constexpr int kGroupBlocks = 4;
 constexpr int64_t kGroupTris = 1 << 16;             // larger trees take the grid
 constexpr size_t kGroupBytes = (size_t)256 << 20;  // of the views together, at most
 
-__global__ void __launch_bounds__(kGroupThreads) k_wide_build_group(const WideTree* __restrict__ trees, WideCtr* ctrs) {
-    const WideTree t = trees[blockIdx.x];
-    WideCtr* ctr = ctrs + blockIdx.x;
-    if (threadIdx.x == 0) wide_init(t.root_box, t.task, ctr);
-    __threadfence();
-    __syncthreads();
-    wide_levels(t.tn, t.tris_in, t.task, t.out, t.tris_out, t.lbox, ctr, t.tris - 1, t.tris, 0, threadIdx.x >> 3,
-                blockDim.x >> 3, 1);
+__global__ void __cluster_dims__(kGroupBlocks) __launch_bounds__(kGroupThreads)
+    k_wide_build_group(const WideTree* __restrict__ trees, WideCtr* ctrs, uint64_t wait_ns) {
+    const uint32_t rank = blockIdx.x % kGroupBlocks;
+    const WideTree t = trees[blockIdx.x / kGroupBlocks];
+    WideCtr* ctr = ctrs + blockIdx.x / kGroupBlocks;
+    if (rank == 0 && threadIdx.x == 0) {
+        wide_init(t.root_box, t.task, ctr);
+        __threadfence();
+    }
+    cooperative_groups::this_cluster().sync();
+    wide_levels(t.tn, t.tris_in, t.task, t.out, t.tris_out, t.lbox, ctr, t.tris - 1, t.tris, wait_ns,
+                (rank * kGroupThreads + threadIdx.x) >> 3, kGroupBlocks * kGroupThreads >> 3, kGroupBlocks);
 }
 
 // ----------------------------------------------------------------------- traversal
@@ -1171,7 +1179,7 @@ cav_status ensure_wide_group(cav_ctx* ctx, const cav_bvh* bvh, cudaStream_t s) {
     WideCtr* dc = (WideCtr*)carve(sizeof(WideCtr) * K);
     cudaError_t e = cudaMemcpyAsync(dt, t.data(), sizeof(WideTree) * K, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
-        k_wide_build_group<<<K, kGroupThreads, 0, s>>>(dt, dc);
+        k_wide_build_group<<<K * kGroupBlocks, kGroupThreads, 0, s>>>(dt, dc, ctx->sort_wait_ns);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(c.data(), dc, sizeof(WideCtr) * K, cudaMemcpyDeviceToHost, s);
