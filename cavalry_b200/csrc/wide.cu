@@ -325,9 +325,9 @@ __global__ void __launch_bounds__(kBuildThreads)
 // The views of many small trees (a batched build's), a cluster of four blocks each (co-resident, as
 // the levels' barriers need): a tree's levels are a chain of fetches, so one tree keeps the chip
 // idle, and a launch, a copy back and a wait for each cost more than its view.  48 trees of 1,000 to
-// 30,000 triangles, asked 2,048 closest hits each after their build: 5.1 ms with a view at a time
-// (31 of them, 65 us each), 3.25 with a block for each tree, 2.87, 2.67 and 2.62 with two, four
-// and eight blocks.
+// 30,000 triangles: 31 views at 65 us each, one by one; the queries of 2,048 closest hits each, the
+// views among them, 3.25 ms with a block for each tree, 2.87, 2.67 and 2.62 with two, four and
+// eight blocks.
 struct WideTree {
     const TNode* tn;
     const TriRec* tris_in;
