@@ -116,3 +116,64 @@ def test_small_views_and_batches(size, n):
         bvh.free()
     finally:
         ctx.close()
+
+
+def plane_rays(name, n, rng):
+    """Rays whose lines lie in triangles' planes, where the triangle test's determinant and distance
+    are rounding noise: lines of sight between points of one tilted wall, and rays laid in the
+    planes of a soup's or of spheres' triangles, from anywhere in them."""
+    from cavalry_b200 import scenes
+
+    if name.startswith("wall"):
+        g, off = int(name[4:]), 5.0 if n & 1 else 0.0
+        i = np.arange(g + 1) / g
+        x, y = (a.ravel()[:, None] for a in np.meshgrid(i, i))
+        up = np.array([0.3, 0.5, 0.8]) / np.linalg.norm([0.3, 0.5, 0.8])
+        ux = np.cross(up, [0.0, 0.0, 1.0])
+        ux /= np.linalg.norm(ux)
+        uy = np.cross(up, ux)
+        pos = (x * ux + y * uy + off).astype(np.float32)
+        q = (np.arange(g)[:, None] * (g + 1) + np.arange(g)).ravel()
+        idx = np.concatenate([np.stack([q, q + 1, q + g + 1], 1), np.stack([q + 1, q + g + 2, q + g + 1], 1)])
+        a, b = rng.random((2, n, 2))
+        o = (a[:, :1] * ux + a[:, 1:] * uy + off).astype(np.float32)
+        p = (b[:, :1] * ux + b[:, 1:] * uy + off).astype(np.float32)
+    else:
+        pos, idx = geometry(name, 5000 if name == "soup" else 3, rng)
+        t = idx[rng.integers(0, len(idx), n)]
+        v0, v1, v2 = (pos[t[:, k]].astype(np.float64) for k in range(3))
+        a, b = rng.uniform(-6, 7, (n, 2)), rng.uniform(-1, 2, (n, 2))
+        o = (v0 + a[:, :1] * (v1 - v0) + a[:, 1:] * (v2 - v0)).astype(np.float32)
+        p = v0 + b[:, :1] * (v1 - v0) + b[:, 1:] * (v2 - v0)
+    d = p - o
+    length = np.maximum(np.linalg.norm(d, axis=1), 1e-20)
+    rays = scenes.make_rays(o, (d / length[:, None]).astype(np.float32))
+    return pos, np.ascontiguousarray(idx, np.int32), rays, (length * 0.999).astype(np.float32)
+
+
+@pytest.mark.parametrize("name,n", [("wall9", 100_000), ("wall32", 100_001), ("wall128", 200_001), ("soup", 1_000_000),
+                                    ("spheres", 1_000_000)])
+def test_any_hits_of_rays_in_triangle_planes(name, n):
+    """Bit for bit the binary traversal's, with a limit and without."""
+    import torch
+
+    import cavalry_b200 as cav
+
+    pos, idx, rays, limit = plane_rays(name, n, np.random.default_rng(n))
+    gpu = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    ctx = cav.Context(0)
+    try:
+        bvh = ctx.build(gpu(pos), gpu(idx), rounds=2)
+        r, lim = gpu(rays), gpu(limit)
+        limits = [lim, 0.3 * lim, None]
+        got = [bvh.trace_any(r, x) for x in limits]
+        assert bvh.has_fast_layout()
+        ctx.set_limits(max_trace_steps=BINARY)
+        want = [bvh.trace_any(r, x) for x in limits]
+        assert 0.02 * n < int(want[0].sum()) < 0.999 * n
+        for g, w in zip(got, want):
+            assert int((g != w).sum()) == 0
+        ctx.sync_check()
+        bvh.free()
+    finally:
+        ctx.close()
