@@ -182,6 +182,7 @@ struct cav_bvh {
     mutable cav::CNode* cnodes = nullptr;
     mutable cav::TriRec* ctris = nullptr;  // triangles in wide-leaf order
     mutable float4* lbox = nullptr;  // two per triangle of ctris: its box in the binary tree
+    mutable float boxes_per_line = 0.f;  // triangles' own boxes that a random line through the scene box meets
     mutable void* wide_arena = nullptr;
     mutable cav::SharedArena* wide_shared = nullptr;  // the view's arena when it was built with others
     // 0: no view; 1: a view the exact mode does not use; 2: one it does; -1: none could be made for it
@@ -281,7 +282,7 @@ cav_status trace_wide_any(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays,
 void free_wide(cav_bvh* bvh, cudaStream_t s, bool async);
 // The exact mode through the view: whether it can be used, and one launch of it (q: the rays,
 // the outputs and the binary tree).
-bool screen_ready(cav_ctx* ctx, const cav_bvh* bvh, int64_t n, cudaStream_t s);
+bool screen_ready(cav_ctx* ctx, const cav_bvh* bvh, bool any_hit, int64_t n, cudaStream_t s);
 cav_status trace_screened(cav_ctx* ctx, const cav_bvh* bvh, const TraceSeg& q, bool any_hit, int64_t n, cudaStream_t s,
                           unsigned long long* counter);
 cav_status trace_wide_segments(cav_ctx* ctx, bool any_hit, const TraceSeg* segs, int nseg, int64_t n, cudaStream_t s,

@@ -604,7 +604,7 @@ cav_status trace_closest(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays, 
     one.prim = prim;
     one.t = t;
     one.uv = uv;
-    if (!(flags & CAV_TRACE_CULL_ON_POP) && screen_ready(ctx, bvh, n, s))
+    if (!(flags & CAV_TRACE_CULL_ON_POP) && screen_ready(ctx, bvh, false, n, s))
         return trace_screened(ctx, bvh, one, false, n, s, counter);
     return launch_closest<false, false>(ctx, one, nullptr, 0, n, flags, s, counter, nullptr, use_short_stack(ctx, bvh),
                                         is_tiny(bvh));
@@ -634,7 +634,7 @@ cav_status trace_any(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays, cons
     one.limit = limit;
     one.excl = excl;
     one.occ = occ;
-    if (!(flags & CAV_TRACE_CULL_ON_POP) && screen_ready(ctx, bvh, n, s))
+    if (!(flags & CAV_TRACE_CULL_ON_POP) && screen_ready(ctx, bvh, true, n, s))
         return trace_screened(ctx, bvh, one, true, n, s, counter);
     return launch_any<false, false>(ctx, one, nullptr, 0, n, flags, s, counter, nullptr, use_short_stack(ctx, bvh),
                                         is_tiny(bvh));
@@ -711,7 +711,7 @@ cav_status trace_closest_dev(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* ra
     one.t = t;
     one.uv = uv;
     one.n_dev = n_dev;
-    if (screen_ready(ctx, bvh, 0, s)) return trace_screened(ctx, bvh, one, false, INT64_MAX, s, counter);
+    if (screen_ready(ctx, bvh, false, -1, s)) return trace_screened(ctx, bvh, one, false, INT64_MAX, s, counter);
     return launch_closest<false, false>(ctx, one, nullptr, 0, INT64_MAX, CAV_TRACE_EXACT, s, counter, nullptr,
                                         use_short_stack(ctx, bvh), is_tiny(bvh));
 }
@@ -725,7 +725,7 @@ cav_status trace_any_dev(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays, 
     one.excl = excl;
     one.occ = occ;
     one.n_dev = n_dev;
-    if (screen_ready(ctx, bvh, 0, s)) return trace_screened(ctx, bvh, one, true, INT64_MAX, s, counter);
+    if (screen_ready(ctx, bvh, true, -1, s)) return trace_screened(ctx, bvh, one, true, INT64_MAX, s, counter);
     return launch_any<false, false>(ctx, one, nullptr, 0, INT64_MAX, CAV_TRACE_EXACT, s, counter, nullptr,
                                     use_short_stack(ctx, bvh), is_tiny(bvh));
 }

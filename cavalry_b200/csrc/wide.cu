@@ -50,22 +50,31 @@ struct WideCtr {
     uint32_t failed;    // a barrier wait ran out, or the level bound was reached
     uint32_t unscreened;  // a triangle or the scene box outside the screening pass's range
     float margin;       // of the quantised boxes
+    float area;         // the triangles' own boxes, half areas summed (in no fixed order)
+    float root_area;    // and the scene box's
 };
 
 // Coordinates up to this are screened (see the screening note below); larger or non-finite
 // geometry always takes the binary traversal in the exact mode.
 constexpr float kScreenCoord = 1e9f;
 
+__device__ __forceinline__ float half_area(const float (&b)[6]) {
+    const float ex = b[3] - b[0], ey = b[4] - b[1], ez = b[5] - b[2];
+    return ex * ey + ey * ez + ez * ex;
+}
+
 __device__ void wide_init(const float* root_box, int32_t* task, WideCtr* ctr) {
-    float mag = 0.f;
+    float mag = 0.f, b[6];
     bool ok = true;
     for (int k = 0; k < 6; ++k) {
+        b[k] = root_box[k];
         mag = fmaxf(mag, fabsf(root_box[k]));
         ok = ok && fabsf(root_box[k]) <= kScreenCoord;
     }
     WideCtr c{};
     c.margin = mag * 4.76837158e-7f + 1e-30f;  // 2^-21: 4 ulps of the largest coordinate
     c.unscreened = ok ? 0u : 1u;
+    c.root_area = half_area(b);
     *ctr = c;
     task[0] = 0;  // the binary root becomes wide node 0
 }
@@ -108,11 +117,6 @@ __device__ bool wide_barrier(WideCtr* ctr, uint32_t blocks, uint32_t target, uin
     return ok != 0;
 }
 
-__device__ __forceinline__ float half_area(const float (&b)[6]) {
-    const float ex = b[3] - b[0], ey = b[4] - b[1], ez = b[5] - b[2];
-    return ex * ey + ey * ez + ez * ex;
-}
-
 // One launch builds the whole view: eight lanes per wide node (lane k holds child k while the
 // node is opened, then the child in slot k), the levels separated by a grid barrier (a block
 // barrier for trees small enough for one block).  Latency bounds it: a level is a chain of six
@@ -126,6 +130,7 @@ __device__ __forceinline__ void wide_levels(const TNode* __restrict__ tn, const 
     const int lane = threadIdx.x & 31, k8 = lane & 7, lead = lane & 24;
     const float margin = *(volatile float*)&ctr->margin;
     uint32_t begin = 0, end = 1;
+    float area = 0.f;  // of the own boxes that this lane places
     for (int level = 0; begin < end; ++level) {
         if (level >= kMaxWideLevels) {
             if (threadIdx.x == 0) atomicExch(&ctr->failed, 1u);
@@ -302,6 +307,7 @@ __device__ __forceinline__ void wide_levels(const TNode* __restrict__ tn, const 
                 tris_out[at] = r;
                 lbox[2 * (size_t)at] = make_float4(b[0], b[1], b[2], b[3]);
                 lbox[2 * (size_t)at + 1] = make_float4(b[4], b[5], __int_as_float(par), __int_as_float(ref));
+                area += half_area(b);
                 const float m = fmaxf(fmaxf(fmaxf(fabsf(r.e1.x), fabsf(r.e1.y)), fabsf(r.e1.z)),
                                       fmaxf(fmaxf(fabsf(r.e2.x), fabsf(r.e2.y)), fabsf(r.e2.z)));
                 const float sum = r.v0.x + r.v0.y + r.v0.z + r.e1.x + r.e1.y + r.e1.z + r.e2.x + r.e2.y + r.e2.z;
@@ -312,6 +318,9 @@ __device__ __forceinline__ void wide_levels(const TNode* __restrict__ tn, const 
         begin = end;
         end = begin + __ldcg(alloc);
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) area += __shfl_xor_sync(kFull, area, o);
+    if (lane == 0 && area > 0.f) atomicAdd(&ctr->area, area);
 }
 
 __global__ void __launch_bounds__(kBuildThreads)
@@ -480,27 +489,25 @@ __device__ __forceinline__ uint2 wstack_get(const uint2* sst, const uint2* lst, 
 //     can be far below its box's entry (of 1M shadow rays laid in such planes 200 to 800 differed when
 //     boxes beyond the limit were left out).  The rays that find no hit pay for it: 4M shadow rays
 //     over the 1M-triangle soup 8.9 ms (5.9 with the pruning), 26.3 in the binary tree.
-//   * Closest hit: the wide traversal tests every triangle whose box it enters below
-//     (1 + 2^-10) times the closest distance, leaves out those whose own box fails, and keeps
-//     the two smallest distances.  If only one triangle has the smallest and its `ml` is below
-//     the second (and within 2^-11 of the smallest), the binary traversal cannot have pruned the
-//     winner at any of its ancestors, and no triangle replaces it: that triangle is the answer.
+//   * Closest hit: the wide traversal tests every triangle whose box it enters up to the ray's
+//     tmax, whatever it has hit so far, and keeps the two smallest distances.  If only one triangle
+//     has the smallest, its own box passes and its `ml` is below the second, the binary traversal
+//     cannot have pruned the winner at any of its ancestors (a hit that prunes one has a distance of
+//     `ml` or less), and no triangle replaces it: that triangle is the answer.
 //   * Of two triangles with the smallest distance (a ray through a shared edge) the same holds
 //     for the one that the binary traversal tests first, the one on the side that it enters
-//     first at their lowest common ancestor.  (With `ml` at most the distance, instead of below
-//     the next one, 1 ray in 10,000 of a path tracer's bounces took up to 941 binary steps at the
-//     end of its launch: 4.06M rays over 1.3M triangles 1.84 ms against 1.32 now.)
+//     first at their lowest common ancestor.  (Handed to the binary steps instead, such ties, 1 ray
+//     in 10,000 of a path tracer's bounces, took up to 941 of them at the end of a launch.)
 // The winner's own box is tested once per ray, when the ray ends; if it fails, the wide search
 // runs again and leaves such triangles out as it goes (kModeCareful).  Every other ray (more
 // ties, a second hit as close as the box entry, a ray or scene out of range) takes the binary
-// steps themselves, in the same kernel: first with the search bounded just above the screened
-// distance (kModeBounded), and from the start if that finds nothing (kModeBinary).  A triangle test that
-// rounds a distance to more than 2^-10 before its own box's entry could still differ (a ray in
-// the triangle's plane to the last bits): of 1.16 G random closest-hit rays and as many any-hit
-// rays over soups, sphere scenes and the room none did, of rays laid in triangles' planes about
-// one in 2,000.
-constexpr float kSlack = 1.0009765625f;       // 1 + 2^-10: distances up to this past the closest are all seen
-constexpr float kNear = 1.00048828125f;       // 1 + 2^-11
+// steps themselves, in the same kernel (kModeBinary).
+// Leaving out boxes that a ray enters beyond its closest hit (with some slack) would be much
+// less work where boxes overlap densely, but no proof: a triangle that holds the ray's line in its
+// plane can have any tested distance, and the binary traversal may come to it before the hit (15
+// to 60 of 1M closest-hit rays laid in triangles' planes differed).  So the closest hits of many
+// rays on such trees are the binary traversal's own (kSparse below).
+constexpr float kSlack = 1.0009765625f;  // 1 + 2^-10, far above the rounding of an entry distance
 constexpr float kScreenDir = 1e6f, kScreenDirMin = 1e-6f;
 
 __device__ inline bool screenable(const f3& o, const f3& d) {
@@ -522,7 +529,7 @@ __device__ inline bool screenable(const f3& o, const f3& d) {
 // against 1.6 ms).  1M-triangle soup, fast mode, with and without sharing: 16,384 shadow rays
 // 0.12 against 1.4 ms, 65,536 closest-hit rays 1.5 against 6.1, 4M 35.7 against 43.8.
 struct ShareRec {
-    int32_t bound[32];  // closest: the smallest distance any lane of the ray has seen (float bits)
+    int32_t bound[32];  // closest, fast mode: the smallest distance any lane of the ray has seen (float bits)
     float best[32], second[32];  // the two smallest distances of the merged lanes (second negative: a lane failed)
     float u[32], v[32];
     int32_t slot[32];     // closest: the triangle at `best`; any: bits 1 hit, 4 failed
@@ -585,7 +592,7 @@ __device__ __forceinline__ int tested_first(const TNode* __restrict__ nodes, con
     return ca == first ? 1 : (cb == first ? 0 : -1);
 }
 
-enum { kModeWide = 0, kModeCareful = 1, kModeBounded = 2, kModeBinary = 3 };
+enum { kModeWide = 0, kModeCareful = 1, kModeBinary = 2 };
 
 // Idle lane iterations, per unit of the context's queue chunk (default 4), that pay for settling
 // a warp's ended rays and claiming new ones.
@@ -596,8 +603,9 @@ constexpr int kSettleCost = 8;
 // A warp holds at most `cap` rays of its own at a time: 32, less when there are fewer rays
 // than lanes (they are spread over the warps, and the other lanes help).
 // Registers: 72 for the exact closest hit (the two smallest distances and the search mode ride
-// along), 64 for the others; 4M soup rays took 38.1 ms at 72, 39.2 at 64, 40.6 at 80 and 53.1 at
-// 56 in the former, 33.7, 35.4 and 38.2 ms at 64, 72 and 80 in the fast mode's closest hit.
+// along), 64 for the others; in the former 180,000 rays of the 1M soup took 11.4 ms at 72, 11.8 at
+// 64 and 11.9 at 80 (2M camera rays over spheres 1.68, 1.64 and 1.62), 4M soup rays of the fast
+// mode's closest hit 33.7, 35.4 and 38.2 ms at 64, 72 and 80.
 template <bool kAny, bool kStats, bool kSeg, bool kExact, int kSmemN = 0>
 __global__ void __maxnreg__(kExact && !kAny ? 72 : 64)
     k_trace_wide(TraceSeg one, const TraceSeg* __restrict__ segs, int nseg, int64_t n, unsigned long long* counter,
@@ -714,15 +722,15 @@ __global__ void __maxnreg__(kExact && !kAny ? 72 : 64)
                         const float ml = own_box(one, slot, R, d);
                         if (!(ml >= 0.f)) {
                             next = kModeCareful;
-                        } else if (ml > tmax || !(ml <= best * kNear)) {
-                            next = kModeBounded;
+                        } else if (ml > tmax) {
+                            next = kModeBinary;
                         } else if (slot2 == -1) {
-                            if (!(ml < second)) next = kModeBounded;
+                            if (!(ml < second)) next = kModeBinary;
                         } else {  // a tie: of two, the first one tested keeps it
                             const float m2 = slot2 >= 0 ? own_box(one, slot2, R, d) : -1.f;
                             int first = slot2 >= 0 ? 1 : -1;
                             if (m2 >= 0.f) first = tested_first(one.nodes, one.lbox, slot, slot2, R.o, own_inv(R, d));
-                            if (first == 0 && m2 < second && m2 <= best * kNear && !(m2 > tmax)) {
+                            if (first == 0 && m2 < second && !(m2 > tmax)) {
                                 tgrp = make_uint2((uint32_t)slot2, 0x101u);  // test it once more, alone
                                 grp = make_uint2(0u, 0u);
                                 best = second = FLT_MAX;
@@ -731,16 +739,13 @@ __global__ void __maxnreg__(kExact && !kAny ? 72 : 64)
                                 bot = 0;
                                 finished = false;
                             } else if (first != 1 || !(ml < second)) {
-                                next = kModeBounded;
+                                next = kModeBinary;
                             }
                         }
                     }
-                } else if (!kAny && mode == kModeBounded && slot == -1) {
-                    next = kModeBinary;
                 }
                 if (next >= 0) {
-                    best = next == kModeBounded ? best * kNear : FLT_MAX;
-                    second = FLT_MAX;
+                    best = second = FLT_MAX;
                     bu = bv = 0.f;
                     slot = kAny ? 0 : -1;
                     slot2 = -1;
@@ -945,12 +950,14 @@ __global__ void __maxnreg__(kExact && !kAny ? 72 : 64)
                     }
                     uint32_t cbase, tbase, masks;
                     float bound;
-                    if (kAny) {
-                        bound = kExact ? __int_as_float(0x7f800000) : tmax;
+                    if (kExact) {
+                        bound = kAny ? __int_as_float(0x7f800000) : tmax * kSlack;
+                    } else if (kAny) {
+                        bound = tmax;
                     } else {
                         bound = best;
                         if (owner >= 0) bound = fminf(bound, __int_as_float(*(volatile int32_t*)&sh.bound[owner]));
-                        bound = fminf(kExact ? bound * kSlack : bound, tmax);
+                        bound = fminf(bound, tmax);
                     }
                     if (kStats) ++st.nodes;
                     const uint32_t h = node_hits(cn, idx, R, bound, cbase, tbase, masks);
@@ -991,7 +998,7 @@ __global__ void __maxnreg__(kExact && !kAny ? 72 : 64)
                         slot = (int32_t)at;
                         bu = u;
                         bv = v;
-                        if (owner >= 0) atomicMin(&sh.bound[owner], __float_as_int(t));
+                        if (!kExact && owner >= 0) atomicMin(&sh.bound[owner], __float_as_int(t));
                     } else if (!better && !(t > tmax)) {
                         if (kExact && mine && t == best) slot2 = slot2 == -1 ? (int32_t)at : -2;
                         else if (kExact) second = fminf(second, t);
@@ -1016,7 +1023,7 @@ __global__ void __maxnreg__(kExact && !kAny ? 72 : 64)
             const f3 inv = mk(1.f / d.x, 1.f / d.y, 1.f / d.z);
             const int32_t ref = (int32_t)grp.x;
             bool pop = false, failed = false;
-            if (!kAny && steps == 0 && mode == kModeBinary) {  // a missed root box ends the ray
+            if (!kAny && steps == 0) {  // a missed root box ends the ray
                 const float* rb = S.root_box;
                 if (!(slab(rb[0], rb[1], rb[2], rb[3], rb[4], rb[5], R.o, inv) >= 0.f)) finished = true;
             }
@@ -1055,8 +1062,7 @@ __global__ void __maxnreg__(kExact && !kAny ? 72 : 64)
                         finished = true;
                     }
                 } else if (tri_test(R.o, d, v0, e1, e2, t, u, v)) {
-                    // bounded: only below the bound; otherwise the first hit counts whatever its distance
-                    if (((mode == kModeBinary && slot < 0) || t < best) && !(t > tmax)) {
+                    if ((slot < 0 || t < best) && !(t > tmax)) {
                         best = t;
                         slot = id;
                         bu = u;
@@ -1203,6 +1209,7 @@ cav_status ensure_wide_group(cav_ctx* ctx, const cav_bvh* bvh, cudaStream_t s) {
         g[k]->cnodes = t[k].out;
         g[k]->ctris = t[k].tris_out;
         g[k]->lbox = t[k].lbox;
+        g[k]->boxes_per_line = c[k].area / c[k].root_area;
         g[k]->wide_state.store(c[k].unscreened ? 1 : 2, std::memory_order_release);
     }
     if (live == 0) {
@@ -1281,6 +1288,7 @@ cav_status ensure_wide(cav_ctx* ctx, const cav_bvh* bvh, cudaStream_t s) {
     bvh->cnodes = cn;
     bvh->ctris = ct;
     bvh->lbox = lbox;
+    bvh->boxes_per_line = h->area / h->root_area;
     bvh->wide_state.store(h->unscreened ? 1 : 2, std::memory_order_release);
     return CAV_OK;
 }
@@ -1309,16 +1317,28 @@ void free_wide(cav_bvh* bvh, cudaStream_t s, bool async) {
 // A batched build's trees get their views together.
 static int64_t screen_min_rays(const cav_bvh* bvh) { return bvh->n >= 4096 || bvh->shared ? 512 : 16384; }
 
-// Whether the exact mode's screening pass can run for n more rays on this tree, building the
-// view on the stream when the tree has been asked about enough of them (that first call waits
-// for the build).  False leaves the binary traversal: a lowered step limit, a stream in
-// capture without a view, no memory for one, or geometry out of the screening range.
-bool screen_ready(cav_ctx* ctx, const cav_bvh* bvh, int64_t n, cudaStream_t s) {
+// Closest hits go through the view where a line through the scene meets few triangles' boxes, or
+// the rays are few.  The search of the view follows the whole line, the binary traversal stops at
+// the hit but walks more nodes, and its launch waits for its longest ray: lines that meet 4 boxes
+// (1.3M triangles of spheres, 4M rays) 0.99 ms against 3.4 in the binary tree, 14 boxes (20,000 of a
+// soup, 1M rays) 1.29 against 1.40, 40 boxes (60,000) 262,144 rays 1.19 against 1.41 and 1M rays 3.1
+// against 2.6, 131 boxes (200,000) 65,536 rays 1.4 against 2.5 and 1M rays 9.0 against 6.0, 655 boxes
+// (1M) 65,536 rays 6.1 against 8.9, 262,144 rays 14.8 against 11.9 and 4M rays 158 against 66.
+constexpr float kSparse = 12.f;
+constexpr int64_t kFewRays = 3 << 16;
+
+// Whether the exact mode's screening pass serves n rays (negative: a number that only the device
+// knows) on this tree, building the view on the stream when the tree has been asked about enough of
+// them (that first call waits for the build).  False leaves the binary traversal: a lowered step
+// limit, a stream in capture without a view, no memory for one, geometry out of the screening
+// range, or many closest hits where boxes overlap densely.
+bool screen_ready(cav_ctx* ctx, const cav_bvh* bvh, bool any_hit, int64_t n, cudaStream_t s) {
     if (bvh->n <= kTinyTris) return false;
     if (ctx->max_trace_steps < kMaxSteps) return false;  // a lowered limit counts binary visits
     int state = bvh->wide_state.load(std::memory_order_acquire);
     if (state == 0) {
-        const int64_t seen = bvh->rays_seen.fetch_add(n) + n;
+        const int64_t more = std::max<int64_t>(n, 0);
+        const int64_t seen = bvh->rays_seen.fetch_add(more) + more;
         if (seen < screen_min_rays(bvh)) return false;
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
@@ -1333,7 +1353,7 @@ bool screen_ready(cav_ctx* ctx, const cav_bvh* bvh, int64_t n, cudaStream_t s) {
         }
         state = bvh->wide_state.load(std::memory_order_acquire);
     }
-    return state == 2;
+    return state == 2 && (any_hit || bvh->boxes_per_line <= kSparse || (n >= 0 && n <= kFewRays));
 }
 
 cav_status trace_screened(cav_ctx* ctx, const cav_bvh* bvh, const TraceSeg& q, bool any_hit, int64_t n, cudaStream_t s,

@@ -139,10 +139,9 @@ typedef struct cav_ray {
 
 /* trace flags */
 #define CAV_TRACE_EXACT 0u        /* the hits of the reference's order and pruning (BVH/BVH.h); default.  Found through
-                                     the compressed 8-wide view where that proves them, else (and until the tree has
-                                     been asked about enough rays to build the view, a call that then waits for the
-                                     build) by that traversal itself.  A ray that lies in a triangle's plane to the
-                                     last bits, where the triangle test's distance is rounding noise, may differ. */
+                                     the compressed 8-wide view where that proves them and pays, else (and until the
+                                     tree has been asked about enough rays to build the view, a call that then waits
+                                     for the build) by that traversal itself. */
 #define CAV_TRACE_FAST 2u         /* compressed 8-wide traversal of the same tree: identical hit distances,
                                      equal-distance ties may resolve to a different triangle than the reference order */
 #define CAV_TRACE_CULL_ON_POP 1u  /* also re-test a popped node against the current hit

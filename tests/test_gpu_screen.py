@@ -177,3 +177,33 @@ def test_any_hits_of_rays_in_triangle_planes(name, n):
         bvh.free()
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("name,n", [("wall32", 100_001), ("wall128", 150_000), ("soup", 100_000), ("soup", 1_000_000),
+                                    ("spheres", 1_000_000)])
+def test_closest_hits_of_rays_in_triangle_planes(name, n):
+    """Bit for bit the binary traversal's, through the view (few rays, or boxes that overlap little)
+    and past it, with a distance bound on part of the rays."""
+    import torch
+
+    import cavalry_b200 as cav
+
+    pos, idx, rays, limit = plane_rays(name, n, np.random.default_rng(n + 1))
+    rays[::3, 7] = 0.8 * limit[::3]
+    gpu = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    ctx = cav.Context(0)
+    try:
+        bvh = ctx.build(gpu(pos), gpu(idx), rounds=2)
+        r = gpu(rays)
+        bvh.trace_closest(r)
+        got = bvh.trace_closest(r)
+        assert bvh.has_fast_layout()
+        ctx.set_limits(max_trace_steps=BINARY)
+        want = bvh.trace_closest(r)
+        assert int((want[0] >= 0).sum()) > 0.02 * n
+        for g, w in zip(got, want):
+            assert torch.equal(g.view(torch.uint8), w.view(torch.uint8))
+        ctx.sync_check()
+        bvh.free()
+    finally:
+        ctx.close()
