@@ -913,18 +913,17 @@ void bvh_release(cav_bvh* bvh, cudaStream_t s, bool async) {
         auto& t = bvh->shared->trees;
         if ((size_t)bvh->shared_at < t.size()) t[bvh->shared_at] = nullptr;
     }
-    free_wide(bvh, s, async);
-    void* mem = bvh->arena;
+    void* mem[2] = {detach_wide(bvh), bvh->arena};
     if (bvh->shared) {
-        mem = nullptr;
+        mem[1] = nullptr;
         if (bvh->shared->refs.fetch_sub(1) == 1) {
-            mem = bvh->shared->p;
+            mem[1] = bvh->shared->p;
             if (bvh->timed)
                 for (int k = 0; k < 7; ++k) cudaEventDestroy(bvh->ev[k]);
             delete bvh->shared;
         }
     }
-    if (mem) release_memory(mem, s, async);
+    release_memory(mem, 2, s, async);
     delete bvh;
 }
 

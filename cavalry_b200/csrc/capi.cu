@@ -28,14 +28,19 @@ cudaError_t dev_alloc(cav_ctx* ctx, void** p, size_t bytes, cudaStream_t s, bool
 }
 
 // cudaFree waits for nothing when the memory came from a pool: the driver takes it as no longer
-// in use and may unmap or reuse it under a kernel that still reads it.
-void release_memory(void* p, cudaStream_t s, bool async) {
-    if (async) {
-        cudaFreeAsync(p, s);
-        return;
+// in use and may unmap or reuse it under a kernel that still reads it.  One wait serves all of it.
+void release_memory(void* const* p, int count, cudaStream_t s, bool async) {
+    bool waited = false;
+    for (int k = 0; k < count; ++k) {
+        if (!p[k]) continue;
+        if (async) {
+            cudaFreeAsync(p[k], s);
+            continue;
+        }
+        if (!waited) cudaDeviceSynchronize();
+        waited = true;
+        cudaFree(p[k]);
     }
-    cudaDeviceSynchronize();
-    cudaFree(p);
 }
 
 cav_status cuda_error(cav_ctx* ctx, cudaError_t e, const char* what) {

@@ -208,8 +208,9 @@ cav_status cuda_error(cav_ctx* ctx, cudaError_t e, const char* what);
 // Fails with cudaErrorMemoryAllocation while the context's injected allocation failures last
 // (cav_ctx_inject), so the error paths of every caller can be tested without exhausting HBM.
 cudaError_t dev_alloc(cav_ctx* ctx, void** p, size_t bytes, cudaStream_t s, bool async);
-// Frees memory of the device's pool: on the stream, or once all of the device's work is done.
-void release_memory(void* p, cudaStream_t s, bool async);
+// Frees memory of the device's pool (nulls are skipped): on the stream, or once all of the
+// device's work is done.
+void release_memory(void* const* p, int count, cudaStream_t s, bool async);
 
 // build.cu
 // Releases a tree (cav_bvh_free); async: stream-ordered frees on `s`, for callers (the
@@ -279,7 +280,8 @@ cav_status trace_wide_closest(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* r
 cav_status trace_wide_any(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays, const float* limit,
                           const int32_t* excl, int64_t n, const uint32_t* n_dev, uint8_t* occ, cudaStream_t s,
                           unsigned long long* counter, unsigned long long* stats = nullptr);
-void free_wide(cav_bvh* bvh, cudaStream_t s, bool async);
+// Takes a tree's view off it; the memory to free, or null while other trees' views are in it.
+void* detach_wide(cav_bvh* bvh);
 // The exact mode through the view: whether it can be used, and one launch of it (q: the rays,
 // the outputs and the binary tree).
 bool screen_ready(cav_ctx* ctx, const cav_bvh* bvh, bool any_hit, int64_t n, cudaStream_t s);

@@ -1293,19 +1293,19 @@ cav_status ensure_wide(cav_ctx* ctx, const cav_bvh* bvh, cudaStream_t s) {
     return CAV_OK;
 }
 
-void free_wide(cav_bvh* bvh, cudaStream_t s, bool async) {
+void* detach_wide(cav_bvh* bvh) {
     void* mem = bvh->wide_arena;
     if (bvh->wide_shared && bvh->wide_shared->refs.fetch_sub(1) == 1) {
         mem = bvh->wide_shared->p;
         delete bvh->wide_shared;
     }
-    if (mem) release_memory(mem, s, async);
     bvh->wide_shared = nullptr;
     bvh->wide_arena = nullptr;
     bvh->cnodes = nullptr;
     bvh->ctris = nullptr;
     bvh->lbox = nullptr;
     bvh->wide_state.store(0);
+    return mem;
 }
 
 // Rays that a tree must have been asked about before the exact mode builds its view.  The view
