@@ -913,17 +913,18 @@ void bvh_release(cav_bvh* bvh, cudaStream_t s, bool async) {
         auto& t = bvh->shared->trees;
         if ((size_t)bvh->shared_at < t.size()) t[bvh->shared_at] = nullptr;
     }
-    void* mem[2] = {detach_wide(bvh), bvh->arena};
+    std::vector<void*> mem;
+    detach_wide(bvh, s, async, mem);
+    if (!bvh->shared) mem.push_back(bvh->arena);
     if (bvh->shared) {
-        mem[1] = nullptr;
         if (bvh->shared->refs.fetch_sub(1) == 1) {
-            mem[1] = bvh->shared->p;
+            mem.push_back(bvh->shared->p);
             if (bvh->timed)
                 for (int k = 0; k < 7; ++k) cudaEventDestroy(bvh->ev[k]);
             delete bvh->shared;
         }
     }
-    release_memory(mem, 2, s, async);
+    release_memory(mem.data(), (int)mem.size(), s, async);
     delete bvh;
 }
 

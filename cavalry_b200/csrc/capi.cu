@@ -121,7 +121,8 @@ cav_status cav_ctx_create(int device, cav_ctx** out) {
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
     }
     cudaGetLastError();
-    if (cudaMalloc(&ctx->d_counters, sizeof(unsigned long long) * kCounterWords) != cudaSuccess ||
+    ctx->verdicts = cav::make_verdict_slots();
+    if (!ctx->verdicts || cudaMalloc(&ctx->d_counters, sizeof(unsigned long long) * kCounterWords) != cudaSuccess ||
         cudaMalloc(&ctx->d_error, sizeof(int) * kErrorWords) != cudaSuccess) {
         cudaGetLastError();
         cudaFree(ctx->d_counters);
@@ -146,7 +147,6 @@ cav_status cav_ctx_destroy(cav_ctx* ctx) {
         if (ctx->hevent[k]) cudaEventDestroy(ctx->hevent[k]);
     }
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
-    if (ctx->wide_host) cudaFreeHost(ctx->wide_host);
     if (ctx->dev_stage) cudaFree(ctx->dev_stage);
     cudaFree(ctx->d_counters);
     cudaFree(ctx->d_error);
@@ -216,7 +216,7 @@ cav_status cav_bvh_free(cav_bvh* bvh) {
 
 int64_t cav_bvh_num_triangles(const cav_bvh* bvh) { return bvh ? bvh->n : 0; }
 
-int cav_bvh_has_fast_layout(const cav_bvh* bvh) { return bvh && bvh->cnodes ? 1 : 0; }
+int cav_bvh_has_fast_layout(const cav_bvh* bvh) { return bvh && bvh->wide_state.load() > 0 ? 1 : 0; }
 
 cav_status cav_bvh_stage_times(cav_ctx* ctx, const cav_bvh* bvh, float* ms6) {
     if (!ctx || !bvh || !ms6) return CAV_ERR_INVALID_ARGUMENT;
@@ -506,6 +506,10 @@ cav_status cav_trace_closest_host(cav_ctx* ctx, const cav_bvh* bvh, const cav_ra
     st = order_after_build(ctx, bvh);
     if (st != CAV_OK) return st;
     const int64_t chunk = chunk_rays(n, !(in_pinned && out_pinned));
+    if (n > chunk && !(flags & (CAV_TRACE_FAST | CAV_TRACE_CULL_ON_POP))) {
+        st = share_view(ctx, bvh, false, n, ctx->hstream[0], ctx->hstream[1]);
+        if (st != CAV_OK) return st;
+    }
     auto launch = [&](Slot s, int64_t c, cudaStream_t str, unsigned long long* counter) -> cav_status {
         const int64_t b = c * chunk, m = std::min(chunk, n - b);
         if (in_pinned) {
@@ -556,6 +560,10 @@ cav_status cav_trace_any_host(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* r
     st = order_after_build(ctx, bvh);
     if (st != CAV_OK) return st;
     const int64_t chunk = chunk_rays(n, true);
+    if (n > chunk && !(flags & (CAV_TRACE_FAST | CAV_TRACE_CULL_ON_POP))) {
+        st = share_view(ctx, bvh, true, n, ctx->hstream[0], ctx->hstream[1]);
+        if (st != CAV_OK) return st;
+    }
     auto launch = [&](Slot s, int64_t c, cudaStream_t str, unsigned long long* counter) -> cav_status {
         const int64_t b = c * chunk, m = std::min(chunk, n - b);
         const void* src_r = rays + b;

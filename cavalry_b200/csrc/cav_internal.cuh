@@ -10,6 +10,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -115,6 +116,12 @@ static_assert(sizeof(TriRec) == 48, "TriRec must be 48 bytes");
 
 // ------------------------------------------------------------ host objects
 struct cav_bvh;
+namespace cav {
+struct VerdictSlots;
+struct ViewJob;
+struct WideCtr;
+std::shared_ptr<VerdictSlots> make_verdict_slots();  // null: no pinned memory
+}  // namespace cav
 struct cav_ctx {
     int device = 0;
     int num_sms = 148;
@@ -146,7 +153,7 @@ struct cav_ctx {
     size_t pinned_bytes = 0;
     void* dev_stage = nullptr;
     size_t dev_stage_bytes = 0;
-    void* wide_host = nullptr;  // pinned: a view build's counters
+    std::shared_ptr<cav::VerdictSlots> verdicts;  // where view builds report to the host
     cudaStream_t hstream[2] = {nullptr, nullptr};
     cudaEvent_t hevent[2] = {nullptr, nullptr};
     // Halton tables on the device, uploaded by the first scene and shared by all
@@ -182,12 +189,14 @@ struct cav_bvh {
     mutable cav::CNode* cnodes = nullptr;
     mutable cav::TriRec* ctris = nullptr;  // triangles in wide-leaf order
     mutable float4* lbox = nullptr;  // two per triangle of ctris: its box in the binary tree
-    mutable float boxes_per_line = 0.f;  // triangles' own boxes that a random line through the scene box meets
-    mutable void* wide_arena = nullptr;
-    mutable cav::SharedArena* wide_shared = nullptr;  // the view's arena when it was built with others
-    // 0: no view; 1: a view the exact mode does not use; 2: one it does; -1: none could be made for it
-    mutable std::atomic<int> wide_state{0};
-    mutable std::atomic<int64_t> rays_seen{0};  // exact-mode rays before there was a view
+    mutable const cav::WideCtr* wctr = nullptr;  // the view's counters (device)
+    mutable cav::ViewJob* view_job = nullptr;    // the build that made it, and its memory
+    mutable std::mutex view_mu;                  // one build of the view at a time (a batch's trees: shared->mu)
+    mutable std::atomic<int> wide_state{0};      // ViewState; the pointers above are set before it leaves kViewNone
+    // triangles' own boxes that a random line through the scene box meets, known from kViewReady on
+    mutable std::atomic<float> boxes_per_line{0.f};
+    mutable std::atomic<int64_t> rays_seen{0};  // exact-mode rays since the tree or the last view that got no memory
+    mutable std::atomic<int> view_misses{0};    // how often a view got no memory
     cav::TriRec* tris = nullptr;   // N
     float root_box[6];             // copied to the host at build time? no: device copy
     float* d_root_box = nullptr;   // 6 floats on device
@@ -257,6 +266,7 @@ struct TraceSeg {
     const CNode* cnodes;    // the tree's compressed 8-wide view (fast-mode launches; ensure_wide)
     const TriRec* ctris;
     const float4* lbox;
+    const WideCtr* gate;    // set: the launch serves the rays only if the view is (or, binary, is not) to serve them
 };
 cav_status trace_closest_segments(cav_ctx* ctx, const TraceSeg* segs, int nseg, int64_t n, uint32_t flags,
                                   cudaStream_t s, unsigned long long* counter);
@@ -280,11 +290,16 @@ cav_status trace_wide_closest(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* r
 cav_status trace_wide_any(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays, const float* limit,
                           const int32_t* excl, int64_t n, const uint32_t* n_dev, uint8_t* occ, cudaStream_t s,
                           unsigned long long* counter, unsigned long long* stats = nullptr);
-// Takes a tree's view off it; the memory to free, or null while other trees' views are in it.
-void* detach_wide(cav_bvh* bvh);
-// The exact mode through the view: whether it can be used, and one launch of it (q: the rays,
-// the outputs and the binary tree).
-bool screen_ready(cav_ctx* ctx, const cav_bvh* bvh, bool any_hit, int64_t n, cudaStream_t s);
+// Takes a tree's view off it and adds the memory to free, if no other trees' views are in it, to
+// `mem`.  async: frees on `s` will be ordered behind the view's build.
+void detach_wide(cav_bvh* bvh, cudaStream_t s, bool async, std::vector<void*>& mem);
+// The exact mode through the view: whether it is used, and one launch of it (q: the rays, the
+// outputs and the binary tree).  kUseBoth: what the device knows of the view decides, so the view's
+// launch and the binary traversal's both go out with q.gate set, and one of them does nothing.
+enum ViewUse { kUseBinary, kUseView, kUseBoth };
+ViewUse view_use(cav_ctx* ctx, const cav_bvh* bvh, bool any_hit, int64_t n, cudaStream_t s);
+// A call that spreads n rays over two streams of the context: a view that it begins on `a` serves `b`.
+cav_status share_view(cav_ctx* ctx, const cav_bvh* bvh, bool any_hit, int64_t n, cudaStream_t a, cudaStream_t b);
 cav_status trace_screened(cav_ctx* ctx, const cav_bvh* bvh, const TraceSeg& q, bool any_hit, int64_t n, cudaStream_t s,
                           unsigned long long* counter);
 cav_status trace_wide_segments(cav_ctx* ctx, bool any_hit, const TraceSeg* segs, int nseg, int64_t n, cudaStream_t s,

@@ -89,6 +89,7 @@ __global__ void __maxnreg__(kSeg || kStats ? 56 : kTraceRegs) k_closest(TraceSeg
         __syncthreads();
     }
     if (!kSeg && one.n_dev) n = *one.n_dev;
+    if (!kSeg && one.gate && view_serves(one.gate, false, n)) n = 0;
     const TNode* __restrict__ nodes = one.nodes;
     const TriRec* __restrict__ tris = one.tris;
     float rb0 = 0.f, rb1 = 0.f, rb2 = 0.f, rb3 = 0.f, rb4 = 0.f, rb5 = 0.f;
@@ -242,6 +243,7 @@ __global__ void __maxnreg__(kSeg || kStats ? 56 : kTraceRegs) k_any(TraceSeg one
         __syncthreads();
     }
     if (!kSeg && one.n_dev) n = *one.n_dev;
+    if (!kSeg && one.gate && view_serves(one.gate, true, n)) n = 0;
     const TNode* __restrict__ nodes = one.nodes;
     const TriRec* __restrict__ tris = one.tris;
     extern __shared__ int32_t sstack[];
@@ -604,8 +606,14 @@ cav_status trace_closest(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays, 
     one.prim = prim;
     one.t = t;
     one.uv = uv;
-    if (!(flags & CAV_TRACE_CULL_ON_POP) && screen_ready(ctx, bvh, false, n, s))
-        return trace_screened(ctx, bvh, one, false, n, s, counter);
+    if (!(flags & CAV_TRACE_CULL_ON_POP)) {
+        const ViewUse use = view_use(ctx, bvh, false, n, s);
+        if (use == kUseBoth) one.gate = bvh->wctr;
+        if (use != kUseBinary) {
+            const cav_status st = trace_screened(ctx, bvh, one, false, n, s, counter);
+            if (st != CAV_OK || use == kUseView) return st;
+        }
+    }
     return launch_closest<false, false>(ctx, one, nullptr, 0, n, flags, s, counter, nullptr, use_short_stack(ctx, bvh),
                                         is_tiny(bvh));
 }
@@ -634,8 +642,14 @@ cav_status trace_any(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays, cons
     one.limit = limit;
     one.excl = excl;
     one.occ = occ;
-    if (!(flags & CAV_TRACE_CULL_ON_POP) && screen_ready(ctx, bvh, true, n, s))
-        return trace_screened(ctx, bvh, one, true, n, s, counter);
+    if (!(flags & CAV_TRACE_CULL_ON_POP)) {
+        const ViewUse use = view_use(ctx, bvh, true, n, s);
+        if (use == kUseBoth) one.gate = bvh->wctr;
+        if (use != kUseBinary) {
+            const cav_status st = trace_screened(ctx, bvh, one, true, n, s, counter);
+            if (st != CAV_OK || use == kUseView) return st;
+        }
+    }
     return launch_any<false, false>(ctx, one, nullptr, 0, n, flags, s, counter, nullptr, use_short_stack(ctx, bvh),
                                         is_tiny(bvh));
 }
@@ -711,7 +725,12 @@ cav_status trace_closest_dev(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* ra
     one.t = t;
     one.uv = uv;
     one.n_dev = n_dev;
-    if (screen_ready(ctx, bvh, false, -1, s)) return trace_screened(ctx, bvh, one, false, INT64_MAX, s, counter);
+    const ViewUse use = view_use(ctx, bvh, false, -1, s);
+    if (use == kUseBoth) one.gate = bvh->wctr;
+    if (use != kUseBinary) {
+        const cav_status st = trace_screened(ctx, bvh, one, false, INT64_MAX, s, counter);
+        if (st != CAV_OK || use == kUseView) return st;
+    }
     return launch_closest<false, false>(ctx, one, nullptr, 0, INT64_MAX, CAV_TRACE_EXACT, s, counter, nullptr,
                                         use_short_stack(ctx, bvh), is_tiny(bvh));
 }
@@ -725,7 +744,12 @@ cav_status trace_any_dev(cav_ctx* ctx, const cav_bvh* bvh, const cav_ray* rays, 
     one.excl = excl;
     one.occ = occ;
     one.n_dev = n_dev;
-    if (screen_ready(ctx, bvh, true, -1, s)) return trace_screened(ctx, bvh, one, true, INT64_MAX, s, counter);
+    const ViewUse use = view_use(ctx, bvh, true, -1, s);
+    if (use == kUseBoth) one.gate = bvh->wctr;
+    if (use != kUseBinary) {
+        const cav_status st = trace_screened(ctx, bvh, one, true, INT64_MAX, s, counter);
+        if (st != CAV_OK || use == kUseView) return st;
+    }
     return launch_any<false, false>(ctx, one, nullptr, 0, INT64_MAX, CAV_TRACE_EXACT, s, counter, nullptr,
                                     use_short_stack(ctx, bvh), is_tiny(bvh));
 }

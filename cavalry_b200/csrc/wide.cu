@@ -23,8 +23,9 @@
 
 #include <algorithm>
 #include <cfloat>
+#include <cstring>
+#include <memory>
 #include <mutex>
-#include <string>
 
 #include "trace_common.cuh"
 
@@ -40,20 +41,6 @@ constexpr int kMaxWideLevels = 4096;  // a wide level consumes at least one bina
 constexpr float kGrow = 1.00000095f;  // 1 + 2^-20
 
 // ------------------------------------------------------------------- building the view
-// Device counters of one build.  nodes[l % 3]: wide nodes allocated for level l; level l
-// allocates from nodes[(l + 1) % 3] and nodes[l % 3] is cleared again one level later, so one
-// grid barrier per level is enough.
-struct WideCtr {
-    uint32_t nodes[3];
-    uint32_t tris;      // triangles placed
-    uint32_t bar;       // arrivals at the grid barrier, all levels
-    uint32_t failed;    // a barrier wait ran out, or the level bound was reached
-    uint32_t unscreened;  // a triangle or the scene box outside the screening pass's range
-    float margin;       // of the quantised boxes
-    float area;         // the triangles' own boxes, half areas summed (in no fixed order)
-    float root_area;    // and the scene box's
-};
-
 // Coordinates up to this are screened (see the screening note below); larger or non-finite
 // geometry always takes the binary traversal in the exact mode.
 constexpr float kScreenCoord = 1e9f;
@@ -63,7 +50,7 @@ __device__ __forceinline__ float half_area(const float (&b)[6]) {
     return ex * ey + ey * ez + ez * ex;
 }
 
-__device__ void wide_init(const float* root_box, int32_t* task, WideCtr* ctr) {
+__device__ void wide_init(const float* root_box, uint32_t tris, int32_t* task, WideCtr* ctr) {
     float mag = 0.f, b[6];
     bool ok = true;
     for (int k = 0; k < 6; ++k) {
@@ -72,6 +59,7 @@ __device__ void wide_init(const float* root_box, int32_t* task, WideCtr* ctr) {
         ok = ok && fabsf(root_box[k]) <= kScreenCoord;
     }
     WideCtr c{};
+    c.want = tris;
     c.margin = mag * 4.76837158e-7f + 1e-30f;  // 2^-21: 4 ulps of the largest coordinate
     c.unscreened = ok ? 0u : 1u;
     c.root_area = half_area(b);
@@ -79,8 +67,30 @@ __device__ void wide_init(const float* root_box, int32_t* task, WideCtr* ctr) {
     task[0] = 0;  // the binary root becomes wide node 0
 }
 
-__global__ void k_wide_init(const float* root_box, int32_t* task, WideCtr* ctr) {
-    if (threadIdx.x == 0) wide_init(root_box, task, ctr);
+__global__ void k_wide_init(const float* root_box, uint32_t tris, int32_t* task, WideCtr* ctr) {
+    if (threadIdx.x == 0) wide_init(root_box, tris, task, ctr);
+}
+
+// What came of a build of K views, in one word of pinned memory that the host looks at: kArrived,
+// whether some view failed or cannot be screened, and in the upper half the most boxes per line.
+// Also the sign that the views are complete.
+constexpr unsigned long long kArrived = 1, kSomeFailed = 2, kSomeUnscreened = 4;
+
+__global__ void k_wide_verdict(const WideCtr* __restrict__ ctr, int K, unsigned long long* host) {
+    unsigned bits = (unsigned)kArrived, most = 0;
+    for (int k = threadIdx.x; k < K; k += 32) {
+        const WideCtr c = ctr[k];
+        if (c.failed || c.tris != c.want) bits |= (unsigned)kSomeFailed;
+        if (c.unscreened) bits |= (unsigned)kSomeUnscreened;
+        const float lines = c.area / c.root_area;  // a NaN counts as infinitely many
+        most = max(most, __float_as_uint(lines >= 0.f ? lines : INFINITY));
+    }
+    bits = __reduce_or_sync(kFull, bits);
+    most = __reduce_max_sync(kFull, most);
+    if (threadIdx.x == 0) {
+        *(volatile unsigned long long*)host = ((unsigned long long)most << 32) | bits;
+        __threadfence_system();
+    }
 }
 
 // All blocks of the (co-resident, cooperatively launched) grid arrive; false once the build
@@ -358,7 +368,7 @@ __global__ void __cluster_dims__(kGroupBlocks) __launch_bounds__(kGroupThreads)
     const WideTree t = trees[blockIdx.x / kGroupBlocks];
     WideCtr* ctr = ctrs + blockIdx.x / kGroupBlocks;
     if (rank == 0 && threadIdx.x == 0) {
-        wide_init(t.root_box, t.task, ctr);
+        wide_init(t.root_box, t.tris, t.task, ctr);
         __threadfence();
     }
     cooperative_groups::this_cluster().sync();
@@ -617,6 +627,7 @@ __global__ void __maxnreg__(kExact && !kAny ? 72 : 64)
         __syncthreads();
     }
     if (!kSeg && one.n_dev) n = *one.n_dev;
+    if (kExact && one.gate && !view_serves(one.gate, kAny, n)) n = 0;
     bool once;
     const int cap = warp_share(n, min_cap, once);
     ShareRec& sh = shares[threadIdx.x >> 5];
@@ -1141,45 +1152,158 @@ cav_status trace_wide_segments(cav_ctx* ctx, bool any_hit, const TraceSeg* segs,
                    : launch_wide<false, true>(ctx, none, segs, nseg, n, s, counter, nullptr);
 }
 
+// ------------------------------------------------------------------ the view on the host
+// Pinned words for the verdicts of view builds, handed out one to a build.
+struct VerdictSlots {
+    static constexpr int kCount = 1024;
+    std::mutex mu;
+    unsigned long long* words = nullptr;
+    std::vector<int> free;
+    std::vector<int> late;  // given back before the verdict was written
+
+    bool arrived(int k) const { return (__atomic_load_n(words + k, __ATOMIC_ACQUIRE) & kArrived) != 0; }
+    int take() {
+        std::lock_guard<std::mutex> lk(mu);
+        for (size_t i = 0; i < late.size();)
+            if (arrived(late[i])) {
+                free.push_back(late[i]);
+                late[i] = late.back();
+                late.pop_back();
+            } else {
+                ++i;
+            }
+        if (free.empty()) return -1;
+        const int k = free.back();
+        free.pop_back();
+        words[k] = 0;
+        return k;
+    }
+    void give(int k, bool written) {
+        std::lock_guard<std::mutex> lk(mu);
+        (written || arrived(k) ? free : late).push_back(k);
+    }
+    ~VerdictSlots() {
+        if (!late.empty()) cudaDeviceSynchronize();
+        cudaFreeHost(words);
+    }
+};
+
+std::shared_ptr<VerdictSlots> make_verdict_slots() {
+    auto v = std::make_shared<VerdictSlots>();
+    if (cudaMallocHost((void**)&v->words, sizeof(*v->words) * VerdictSlots::kCount) != cudaSuccess) {
+        cudaGetLastError();
+        v->words = nullptr;
+        return nullptr;
+    }
+    for (int k = 0; k < VerdictSlots::kCount; ++k) v->free.push_back(k);
+    return v;
+}
+
+// One build of one or several trees' views: enqueued on a stream, complete once its verdict has
+// arrived (or `done`, for those who wait).
+struct ViewJob {
+    void* arena = nullptr;
+    std::atomic<int> refs{0};  // trees with a view in it
+    int trees = 0;
+    cudaEvent_t done = nullptr;
+    unsigned long long stream = 0;             // the streams on which work enqueued since comes after it
+    std::atomic<unsigned long long> also{0};
+    std::shared_ptr<VerdictSlots> slots;
+    int slot = -1;
+    ViewJob* before = nullptr;  // a build of the tree alone that had failed
+};
+
+// kViewBegun: enqueued, no verdict yet.  kViewMixed: complete, the tree's own verdict is on the device.
+// kViewUnscreened: a view that the exact mode does not use; kViewReady: one that it does.
+enum ViewState { kViewFailed = -1, kViewNone = 0, kViewUnscreened = 1, kViewReady = 2, kViewBegun = 3, kViewMixed = 4 };
+
 namespace {
-// The views of the batch that `bvh` was built in, those that are missing and small, in one launch.
-// Every tree of the batch is complete where `bvh` is: the same launches built them all.
-cav_status ensure_wide_group(cav_ctx* ctx, const cav_bvh* bvh, cudaStream_t s) {
-    std::lock_guard<std::mutex> lk(bvh->shared->mu);  // none of them is released meanwhile
-    std::vector<const cav_bvh*> g;
-    size_t need = 0;
+
+std::mutex& view_mutex(const cav_bvh* bvh) { return bvh->shared ? bvh->shared->mu : bvh->view_mu; }
+
+unsigned long long stream_id(cudaStream_t s) {
+    unsigned long long id = 0;
+    if (cudaStreamGetId(s, &id) != cudaSuccess) {
+        cudaGetLastError();
+        return ~0ull;  // no stream's
+    }
+    return id;
+}
+
+bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) return false;
+    cudaGetLastError();
+    return true;
+}
+
+// The state of a tree's view, with a verdict that has arrived taken over.
+int view_state(const cav_bvh* bvh) {
+    int st = bvh->wide_state.load(std::memory_order_acquire);
+    if (st != kViewBegun) return st;
+    const ViewJob* job = bvh->view_job;
+    const unsigned long long w = __atomic_load_n(job->slots->words + job->slot, __ATOMIC_ACQUIRE);
+    if (!(w & kArrived)) return st;
+    int next = kViewMixed;
+    if (!(w & (kSomeFailed | kSomeUnscreened))) next = kViewReady;
+    else if (job->trees == 1) next = (w & kSomeFailed) ? kViewFailed : kViewUnscreened;
+    float lines;
+    const uint32_t bits = (uint32_t)(w >> 32);
+    memcpy(&lines, &bits, 4);
+    bvh->boxes_per_line.store(lines);
+    bvh->wide_state.compare_exchange_strong(st, next);
+    return bvh->wide_state.load(std::memory_order_acquire);
+}
+
+// Enqueues the build of the view of `bvh` on the stream, together with the missing views of the
+// small trees of its batch; view_mutex(bvh) is held.  Every tree of a batch is complete where `bvh`
+// is: the same launches built them all.  Sets no error: the exact mode does without.
+cudaError_t begin_view(cav_ctx* ctx, const cav_bvh* bvh, cudaStream_t s) {
     auto round = [](size_t b) { return (b + 255) & ~(size_t)255; };
     auto bytes = [&](const cav_bvh* b) {
         return round(sizeof(CNode) * (size_t)(b->n - 1)) + round(sizeof(TriRec) * (size_t)b->n) +
                round(2 * sizeof(float4) * (size_t)b->n) + round(sizeof(int32_t) * (size_t)(b->n - 1));
     };
-    for (const cav_bvh* b : bvh->shared->trees)
-        if (b && b->wide_state.load(std::memory_order_acquire) <= 0 && b->n <= kGroupTris) {
-            g.push_back(b);
-            need += bytes(b);
+    std::vector<const cav_bvh*> g{bvh};
+    size_t need = bytes(bvh);
+    if (bvh->shared && bvh->n <= kGroupTris && bvh->wide_state.load() == kViewNone) {
+        for (const cav_bvh* b : bvh->shared->trees)
+            if (b && b != bvh && b->wide_state.load() == kViewNone && b->n <= kGroupTris && b->n > kTinyTris) {
+                g.push_back(b);
+                need += bytes(b);
+            }
+        if (need > kGroupBytes) {
+            g.resize(1);
+            need = bytes(bvh);
         }
-    const int K = (int)g.size();
-    if (K < 2 || need > kGroupBytes) return CAV_ERR_NOT_READY;
-    need += round(sizeof(WideTree) * K) + round(sizeof(WideCtr) * K);
-    void* arena = nullptr;
-    if (dev_alloc(ctx, &arena, need, s, true) != cudaSuccess) {
-        cudaGetLastError();
-        return CAV_ERR_NOT_READY;
     }
-    unsigned char* p = (unsigned char*)arena;
+    const int K = (int)g.size();
+    need += round(sizeof(WideTree) * K) + round(sizeof(WideCtr) * K);
+    auto job = std::make_unique<ViewJob>();
+    job->slots = ctx->verdicts;
+    job->slot = job->slots->take();
+    if (job->slot < 0) return cudaErrorMemoryAllocation;  // as many builds under way as there are words
+    cudaError_t e = dev_alloc(ctx, &job->arena, need, s, true);
+    if (e == cudaSuccess && (e = cudaEventCreateWithFlags(&job->done, cudaEventDisableTiming)) != cudaSuccess)
+        cudaFreeAsync(job->arena, s);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        job->slots->give(job->slot, true);
+        return e;
+    }
+    unsigned char* p = (unsigned char*)job->arena;
     auto carve = [&](size_t b) {
         unsigned char* r = p;
         p += round(b);
         return (void*)r;
     };
     std::vector<WideTree> t(K);
-    std::vector<WideCtr> c(K);
     for (int k = 0; k < K; ++k) {
         const cav_bvh* b = g[k];
         t[k].tn = b->tnodes;
         t[k].tris_in = b->tris;
         t[k].root_box = b->d_root_box;
-        t[k].out = (CNode*)carve(sizeof(CNode) * (size_t)(b->n - 1));
+        t[k].out = (CNode*)carve(sizeof(CNode) * (size_t)(b->n - 1));  // a wide node for each internal node at most
         t[k].tris_out = (TriRec*)carve(sizeof(TriRec) * (size_t)b->n);
         t[k].lbox = (float4*)carve(2 * sizeof(float4) * (size_t)b->n);
         t[k].task = (int32_t*)carve(sizeof(int32_t) * (size_t)(b->n - 1));
@@ -1187,125 +1311,98 @@ cav_status ensure_wide_group(cav_ctx* ctx, const cav_bvh* bvh, cudaStream_t s) {
     }
     WideTree* dt = (WideTree*)carve(sizeof(WideTree) * K);
     WideCtr* dc = (WideCtr*)carve(sizeof(WideCtr) * K);
-    cudaError_t e = cudaMemcpyAsync(dt, t.data(), sizeof(WideTree) * K, cudaMemcpyHostToDevice, s);
+    if (K > 1) {
+        // pageable memory: staged before the call returns
+        e = cudaMemcpyAsync(dt, t.data(), sizeof(WideTree) * K, cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) {
+            k_wide_build_group<<<K * kGroupBlocks, kGroupThreads, 0, s>>>(dt, dc, ctx->sort_wait_ns);
+            e = cudaGetLastError();
+        }
+    } else {
+        const WideTree& w = t[0];
+        k_wide_init<<<1, 32, 0, s>>>(w.root_box, w.tris, w.task, dc);
+        // about one wide node per four triangles, eight lanes each; every block co-resident
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wide_build, kBuildThreads, 0);
+        const int64_t room = (int64_t)ctx->num_sms * std::min(std::max(per_sm, 1), 8);
+        const int grid = (int)std::min<int64_t>(room, std::max<int64_t>(1, bvh->n * 2 / kBuildThreads));
+        uint32_t max_nodes = w.tris - 1, max_tris = w.tris;
+        uint64_t wait_ns = ctx->sort_wait_ns;
+        void* args[] = {(void*)&w.tn, (void*)&w.tris_in, (void*)&w.task, (void*)&w.out, (void*)&w.tris_out, (void*)&w.lbox,
+                        &dc,          &max_nodes,        &max_tris,      &wait_ns};
+        e = cudaLaunchCooperativeKernel((const void*)k_wide_build, dim3(grid), dim3(kBuildThreads), args, 0, s);
+    }
+    bool reports = false;
     if (e == cudaSuccess) {
-        k_wide_build_group<<<K * kGroupBlocks, kGroupThreads, 0, s>>>(dt, dc, ctx->sort_wait_ns);
+        k_wide_verdict<<<1, 32, 0, s>>>(dc, K, job->slots->words + job->slot);
         e = cudaGetLastError();
+        reports = e == cudaSuccess;
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(c.data(), dc, sizeof(WideCtr) * K, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = cudaEventRecord(job->done, s);
     if (e != cudaSuccess) {
-        cudaFreeAsync(arena, s);
-        return cuda_error(ctx, e, "fast traversal layout");
+        cudaGetLastError();
+        cudaFreeAsync(job->arena, s);
+        cudaEventDestroy(job->done);
+        job->slots->give(job->slot, !reports);
+        return e;
     }
-    auto* held = new SharedArena();
-    held->p = arena;
-    int live = 0;
-    for (int k = 0; k < K; ++k) live += !c[k].failed && c[k].tris == t[k].tris;
-    held->refs = live;
+    job->stream = stream_id(s);
+    job->trees = K;
+    job->refs = K;
+    if (K == 1) job->before = bvh->view_job;
+    ViewJob* held = job.release();
     for (int k = 0; k < K; ++k) {
-        if (c[k].failed || c[k].tris != t[k].tris) continue;
-        g[k]->wide_shared = held;
+        g[k]->view_job = held;
         g[k]->cnodes = t[k].out;
         g[k]->ctris = t[k].tris_out;
         g[k]->lbox = t[k].lbox;
-        g[k]->boxes_per_line = c[k].area / c[k].root_area;
-        g[k]->wide_state.store(c[k].unscreened ? 1 : 2, std::memory_order_release);
+        g[k]->wctr = dc + k;
+        g[k]->wide_state.store(kViewBegun, std::memory_order_release);
     }
-    if (live == 0) {
-        cudaFreeAsync(arena, s);
-        delete held;
-    }
-    return bvh->wide_state.load() > 0
-               ? CAV_OK
-               : set_error(ctx, CAV_ERR_CUDA, "fast traversal layout: not every triangle placed");
+    return cudaSuccess;
 }
+
 }  // namespace
 
+// The view of a tree, complete: built and waited for where it is missing.
 cav_status ensure_wide(cav_ctx* ctx, const cav_bvh* bvh, cudaStream_t s) {
-    if (bvh->wide_state.load(std::memory_order_acquire) > 0) return CAV_OK;
-    // serialised: several host threads (the server's lanes) may reach one tree at once; the
-    // view is published only once its build has completed on the device
-    static std::mutex build_mu;
-    std::lock_guard<std::mutex> lk(build_mu);
-    if (bvh->wide_state.load(std::memory_order_acquire) > 0) return CAV_OK;
-    if (bvh->shared && bvh->n <= kGroupTris) {
-        const cav_status st = ensure_wide_group(ctx, bvh, s);
-        if (st != CAV_ERR_NOT_READY) return st;  // else alone: the only one, too much together, or no memory
+    for (bool again = false;;) {
+        int st = view_state(bvh);
+        if (st == kViewReady || st == kViewUnscreened) return CAV_OK;
+        if (st == kViewBegun || st == kViewMixed) {
+            WideCtr c;
+            cudaError_t e = cudaEventSynchronize(bvh->view_job->done);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(&c, bvh->wctr, sizeof(c), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+            if (e != cudaSuccess) return cuda_error(ctx, e, "fast traversal layout");
+            const bool good = !c.failed && c.tris == c.want;
+            bvh->boxes_per_line.store(c.area / c.root_area);
+            bvh->wide_state.compare_exchange_strong(st, !good ? kViewFailed : (c.unscreened ? kViewUnscreened : kViewReady));
+            continue;
+        }
+        if (st == kViewFailed && again) return set_error(ctx, CAV_ERR_CUDA, "fast traversal layout: not every triangle placed");
+        again = true;
+        std::lock_guard<std::mutex> lk(view_mutex(bvh));  // several host threads may reach one tree at once
+        if (bvh->wide_state.load() > 0) continue;
+        const cudaError_t e = begin_view(ctx, bvh, s);
+        if (e != cudaSuccess) return cuda_error(ctx, e, "fast traversal layout");
     }
-    const int64_t n = bvh->n;
-    const int64_t nw = n - 1;  // each wide node but the root stands for a distinct binary internal node
-    size_t need = sizeof(CNode) * (size_t)nw + 256;
-    need += sizeof(TriRec) * (size_t)n + 256;
-    need += 2 * sizeof(float4) * (size_t)n + 256;
-    need += sizeof(int32_t) * (size_t)nw + 256;
-    need += sizeof(WideCtr) + 256;
-    if (!ctx->wide_host && cudaMallocHost(&ctx->wide_host, sizeof(WideCtr)) != cudaSuccess) {
-        cudaGetLastError();
-        ctx->wide_host = nullptr;
-        return set_error(ctx, CAV_ERR_OUT_OF_MEMORY, "fast traversal layout: pinned allocation failed");
-    }
-    void* arena = nullptr;  // stream-ordered: complete before the view is published below
-    if (dev_alloc(ctx, &arena, need, s, true) != cudaSuccess) {
-        cudaGetLastError();
-        return set_error(ctx, CAV_ERR_OUT_OF_MEMORY, "fast traversal layout: device allocation failed");
-    }
-    unsigned char* p = (unsigned char*)arena;
-    auto carve = [&](size_t bytes) {
-        unsigned char* r = (unsigned char*)(((uintptr_t)p + 255) & ~(uintptr_t)255);
-        p = r + bytes;
-        return (void*)r;
-    };
-    CNode* cn = (CNode*)carve(sizeof(CNode) * (size_t)nw);
-    TriRec* ct = (TriRec*)carve(sizeof(TriRec) * (size_t)n);
-    float4* lbox = (float4*)carve(2 * sizeof(float4) * (size_t)n);
-    int32_t* task = (int32_t*)carve(sizeof(int32_t) * (size_t)nw);
-    WideCtr* ctr = (WideCtr*)carve(sizeof(WideCtr));
-    k_wide_init<<<1, 32, 0, s>>>(bvh->d_root_box, task, ctr);
-    // about one wide node per four triangles, eight lanes each; every block co-resident
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wide_build, kBuildThreads, 0);
-    const int64_t room = (int64_t)ctx->num_sms * std::min(std::max(per_sm, 1), 8);
-    const int grid = (int)std::min<int64_t>(room, std::max<int64_t>(1, n * 2 / kBuildThreads));
-    uint32_t max_nodes = (uint32_t)nw, max_tris = (uint32_t)n;
-    uint64_t wait_ns = ctx->sort_wait_ns;
-    const TNode* tn = bvh->tnodes;
-    const TriRec* tin = bvh->tris;
-    void* args[] = {&tn, &tin, &task, &cn, &ct, &lbox, &ctr, &max_nodes, &max_tris, &wait_ns};
-    cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_wide_build, dim3(grid), dim3(kBuildThreads), args, 0, s);
-    WideCtr* h = (WideCtr*)ctx->wide_host;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h, ctr, sizeof(WideCtr), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cav_status st = CAV_OK;
-    if (e != cudaSuccess) st = cuda_error(ctx, e, "fast traversal layout");
-    else if (h->failed || h->tris != (uint32_t)n)
-        st = set_error(ctx, CAV_ERR_CUDA, "fast traversal layout: not every triangle placed");
-    if (st != CAV_OK) {
-        cudaFreeAsync(arena, s);
-        return st;
-    }
-    bvh->wide_arena = arena;
-    bvh->cnodes = cn;
-    bvh->ctris = ct;
-    bvh->lbox = lbox;
-    bvh->boxes_per_line = h->area / h->root_area;
-    bvh->wide_state.store(h->unscreened ? 1 : 2, std::memory_order_release);
-    return CAV_OK;
 }
 
-void* detach_wide(cav_bvh* bvh) {
-    void* mem = bvh->wide_arena;
-    if (bvh->wide_shared && bvh->wide_shared->refs.fetch_sub(1) == 1) {
-        mem = bvh->wide_shared->p;
-        delete bvh->wide_shared;
+void detach_wide(cav_bvh* bvh, cudaStream_t s, bool async, std::vector<void*>& mem) {
+    for (ViewJob* job = bvh->view_job; job;) {
+        ViewJob* const before = job->before;
+        if (job->refs.fetch_sub(1) == 1) {
+            if (async) cudaStreamWaitEvent(s, job->done, 0);
+            mem.push_back(job->arena);
+            cudaEventDestroy(job->done);
+            job->slots->give(job->slot, false);
+            delete job;
+        }
+        job = before;
     }
-    bvh->wide_shared = nullptr;
-    bvh->wide_arena = nullptr;
-    bvh->cnodes = nullptr;
-    bvh->ctris = nullptr;
-    bvh->lbox = nullptr;
-    bvh->wide_state.store(0);
-    return mem;
+    bvh->view_job = nullptr;
+    bvh->wide_state.store(kViewNone);
 }
 
 // Rays that a tree must have been asked about before the exact mode builds its view.  The view
@@ -1317,43 +1414,48 @@ void* detach_wide(cav_bvh* bvh) {
 // A batched build's trees get their views together.
 static int64_t screen_min_rays(const cav_bvh* bvh) { return bvh->n >= 4096 || bvh->shared ? 512 : 16384; }
 
-// Closest hits go through the view where a line through the scene meets few triangles' boxes, or
-// the rays are few.  The search of the view follows the whole line, the binary traversal stops at
-// the hit but walks more nodes, and its launch waits for its longest ray: lines that meet 4 boxes
-// (1.3M triangles of spheres, 4M rays) 0.99 ms against 3.4 in the binary tree, 14 boxes (20,000 of a
-// soup, 1M rays) 1.29 against 1.40, 40 boxes (60,000) 262,144 rays 1.19 against 1.41 and 1M rays 3.1
-// against 2.6, 131 boxes (200,000) 65,536 rays 1.4 against 2.5 and 1M rays 9.0 against 6.0, 655 boxes
-// (1M) 65,536 rays 6.1 against 8.9, 262,144 rays 14.8 against 11.9 and 4M rays 158 against 66.
-constexpr float kSparse = 12.f;
-constexpr int64_t kFewRays = 3 << 16;
-
-// Whether the exact mode's screening pass serves n rays (negative: a number that only the device
-// knows) on this tree, building the view on the stream when the tree has been asked about enough of
-// them (that first call waits for the build).  False leaves the binary traversal: a lowered step
-// limit, a stream in capture without a view, no memory for one, geometry out of the screening
-// range, or many closest hits where boxes overlap densely.
-bool screen_ready(cav_ctx* ctx, const cav_bvh* bvh, bool any_hit, int64_t n, cudaStream_t s) {
-    if (bvh->n <= kTinyTris) return false;
-    if (ctx->max_trace_steps < kMaxSteps) return false;  // a lowered limit counts binary visits
-    int state = bvh->wide_state.load(std::memory_order_acquire);
-    if (state == 0) {
+// How n rays (negative: a number that only the device knows) of the exact mode go.  Once the tree
+// has been asked about enough of them its view's build is enqueued on the stream; nothing waits for
+// it.  Until its verdict has arrived, calls on that stream come after it and let the device
+// decide, and those on other streams take the binary traversal.  So do a lowered step limit, a
+// stream in capture without a complete view, no memory for one (asked for again after twice
+// as many rays as the last time), geometry out of the screening range, and many closest hits where
+// boxes overlap densely.
+ViewUse view_use(cav_ctx* ctx, const cav_bvh* bvh, bool any_hit, int64_t n, cudaStream_t s) {
+    if (bvh->n <= kTinyTris) return kUseBinary;
+    if (ctx->max_trace_steps < kMaxSteps) return kUseBinary;  // a lowered limit counts binary visits
+    int st = view_state(bvh);
+    if (st == kViewNone) {
         const int64_t more = std::max<int64_t>(n, 0);
         const int64_t seen = bvh->rays_seen.fetch_add(more) + more;
-        if (seen < screen_min_rays(bvh)) return false;
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-            cudaGetLastError();
-            return false;
+        if (seen < screen_min_rays(bvh) << std::min(bvh->view_misses.load(), 24)) return kUseBinary;
+        if (capturing(s)) return kUseBinary;
+        std::lock_guard<std::mutex> lk(view_mutex(bvh));
+        if (bvh->wide_state.load() == kViewNone && begin_view(ctx, bvh, s) != cudaSuccess) {
+            bvh->view_misses.fetch_add(1);
+            bvh->rays_seen.store(0);
+            return kUseBinary;
         }
-        const std::string said = ctx->last_error;
-        if (ensure_wide(ctx, bvh, s) != CAV_OK) {  // the binary traversal needs no view
-            ctx->last_error = said;
-            bvh->wide_state.store(-1);
-            return false;
-        }
-        state = bvh->wide_state.load(std::memory_order_acquire);
+        st = view_state(bvh);
     }
-    return state == 2 && (any_hit || bvh->boxes_per_line <= kSparse || (n >= 0 && n <= kFewRays));
+    if (st == kViewBegun) {
+        const unsigned long long id = stream_id(s);
+        const bool after = id == bvh->view_job->stream || id == bvh->view_job->also.load();
+        return after && !capturing(s) ? kUseBoth : kUseBinary;
+    }
+    if (st == kViewMixed) return kUseBoth;
+    if (st != kViewReady) return kUseBinary;
+    if (any_hit || bvh->boxes_per_line.load() <= kSparse) return kUseView;
+    return n < 0 ? kUseBoth : (n <= kFewRays ? kUseView : kUseBinary);
+}
+
+cav_status share_view(cav_ctx* ctx, const cav_bvh* bvh, bool any_hit, int64_t n, cudaStream_t a, cudaStream_t b) {
+    if (view_use(ctx, bvh, any_hit, n, a) != kUseBoth || view_state(bvh) != kViewBegun) return CAV_OK;
+    ViewJob* job = bvh->view_job;
+    if (job->stream != stream_id(a)) return CAV_OK;
+    CAV_CUDA(ctx, cudaStreamWaitEvent(b, job->done, 0));
+    job->also.store(stream_id(b));
+    return CAV_OK;
 }
 
 cav_status trace_screened(cav_ctx* ctx, const cav_bvh* bvh, const TraceSeg& q, bool any_hit, int64_t n, cudaStream_t s,

@@ -68,7 +68,8 @@ cav_status cav_ctx_set_limits(cav_ctx* ctx, double sort_wait_s, int64_t max_trac
  *     meaningful;
  *   CAV_INJECT_ALLOC_FAIL: the count-th next device allocation made for this context (build
  *     arenas and scratch, scene uploads, render path state, server job buffers) fails once,
- *     and the call that made it returns CAV_ERR_OUT_OF_MEMORY (the others succeed);
+ *     and the call that made it returns CAV_ERR_OUT_OF_MEMORY (the others succeed; an exact-mode
+ *     query whose 8-wide view it is succeeds without it);
  *   CAV_INJECT_MLP_STALL (count > 0 on, 0 off): in the tcgen05 MLP forward, each warpgroup
  *     issues no MMA and no commit for its first tile, so its bounded completion wait runs
  *     out; the call ends with CAV_ERR_TIMEOUT from cav_sync_check and outputs that are not
@@ -139,9 +140,10 @@ typedef struct cav_ray {
 
 /* trace flags */
 #define CAV_TRACE_EXACT 0u        /* the hits of the reference's order and pruning (BVH/BVH.h); default.  Found through
-                                     the compressed 8-wide view where that proves them and pays, else (and until the
-                                     tree has been asked about enough rays to build the view, a call that then waits
-                                     for the build) by that traversal itself. */
+                                     the compressed 8-wide view where that proves them and pays, else by that
+                                     traversal itself.  The view is enqueued by the call that has asked the tree about
+                                     enough rays, and serves other streams once it is complete; a call waits for
+                                     nothing, and does without the view where there is no memory for it. */
 #define CAV_TRACE_FAST 2u         /* compressed 8-wide traversal of the same tree: identical hit distances,
                                      equal-distance ties may resolve to a different triangle than the reference order */
 #define CAV_TRACE_CULL_ON_POP 1u  /* also re-test a popped node against the current hit

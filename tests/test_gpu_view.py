@@ -1,0 +1,194 @@
+"""GPU tests of how a tree's 8-wide view comes about in the exact mode: enqueued by the query that
+has asked about enough rays, waited for by nobody, done without where there is no memory for it
+or the stream is being captured.  Answers are the binary traversal's throughout."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+BINARY = (1 << 22) - 1  # one below the default limit: the same answers from the binary traversal
+
+
+def _tree(ctx, n, seed=3, rays=20_000):
+    import torch
+
+    from cavalry_b200 import scenes
+
+    pos, idx = scenes.soup(n, seed=seed)
+    bvh = ctx.build(torch.from_numpy(pos).cuda(), torch.from_numpy(idx).cuda(), rounds=1)
+    shadow, limit = scenes.shadow_rays(rays, seed=seed + 1)
+    return (bvh, torch.from_numpy(scenes.closest_rays(rays, seed=seed)).cuda(), torch.from_numpy(shadow).cuda(),
+            torch.from_numpy(limit).cuda())
+
+
+def _same(got, want):
+    import torch
+
+    return all(torch.equal(g.view(torch.uint8), w.view(torch.uint8)) for g, w in zip(got, want))
+
+
+def _binary(ctx, bvh, rays, shadow, limit):
+    import torch
+
+    ctx.set_limits(max_trace_steps=BINARY)
+    want = [*bvh.trace_closest(rays), bvh.trace_any(shadow, limit)]
+    ctx.set_limits()
+    torch.cuda.synchronize()
+    return want
+
+
+def test_a_query_that_begins_the_view_waits_for_nothing():
+    """Behind half a second of other work on its stream the first queries return at once, and one
+    on another stream is answered meanwhile, before the view that it cannot use yet."""
+    import torch
+
+    import cavalry_b200 as cav
+
+    ctx = cav.Context(0)
+    try:
+        warm, rays, shadow, limit = _tree(ctx, 30_000, seed=9)  # modules loaded, memory pool grown
+        for _ in range(2):
+            warm.trace_closest(rays), warm.trace_any(shadow, limit)
+        warm.trace_closest(rays, flags=cav.TRACE_FAST)
+        torch.cuda.synchronize()
+        bvh, rays, shadow, limit = _tree(ctx, 30_000)
+        want = _binary(ctx, bvh, rays, shadow, limit)
+        assert not bvh.has_fast_layout()
+        a, b = torch.cuda.Stream(), torch.cuda.Stream()
+        # outputs exist beforehand: the caching allocator is not what is tested
+        outs = [(torch.empty(len(rays), dtype=torch.int32, device="cuda"), torch.empty(len(rays), device="cuda"),
+                 torch.empty((len(rays), 2), device="cuda"), torch.empty(len(rays), dtype=torch.uint8, device="cuda"))
+                for _ in range(2)]
+        torch.cuda.synchronize()
+        with torch.cuda.stream(a):
+            torch.cuda._sleep(1_000_000_000)
+        for s, o in ((a, outs[0]), (b, outs[1])):
+            bvh.trace_closest(rays, stream=s, out=o[:3])
+            bvh.trace_any(shadow, limit, stream=s, out=o[3])
+            if s is a:
+                assert bvh.has_fast_layout()  # begun
+        b.synchronize()
+        assert not a.query()
+        assert _same(outs[1], want)
+        a.synchronize()
+        assert _same(outs[0], want)
+        assert _same([*bvh.trace_closest(rays), bvh.trace_any(shadow, limit)], want)
+        ctx.sync_check()
+        bvh.free(), warm.free()
+    finally:
+        ctx.close()
+
+
+def test_no_memory_for_the_view():
+    """The query succeeds without it, and a later one has it."""
+    import cavalry_b200 as cav
+
+    ctx = cav.Context(0)
+    try:
+        bvh, rays, shadow, limit = _tree(ctx, 30_000)
+        want = _binary(ctx, bvh, rays, shadow, limit)
+        ctx.inject(cav.INJECT_ALLOC_FAIL, 1)
+        assert _same(bvh.trace_closest(rays), want)
+        assert not bvh.has_fast_layout()
+        assert _same([bvh.trace_any(shadow, limit)], want[3:])  # asked about more than twice 512 rays
+        assert bvh.has_fast_layout()
+        assert _same([*bvh.trace_closest(rays), bvh.trace_any(shadow, limit)], want)
+        ctx.sync_check()
+        bvh.free()
+    finally:
+        ctx.inject(cav.INJECT_NONE)
+        ctx.close()
+
+
+@pytest.mark.parametrize("view", [False, True])
+def test_a_stream_in_capture(view):
+    """A captured query takes the view that is complete, or the binary traversal."""
+    import torch
+
+    import cavalry_b200 as cav
+
+    ctx = cav.Context(0)
+    try:
+        bvh, rays, shadow, limit = _tree(ctx, 30_000)
+        want = _binary(ctx, bvh, rays, shadow, limit)
+        if view:
+            bvh.trace_any(shadow, limit)
+            torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            got = [*bvh.trace_closest(rays), bvh.trace_any(shadow, limit)]
+        assert bool(bvh.has_fast_layout()) == view
+        for o in got:
+            o.fill_(1)
+        g.replay()
+        torch.cuda.synchronize()
+        assert _same(got, want)
+        ctx.sync_check()
+        del g
+        bvh.free()
+    finally:
+        ctx.close()
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_threads_that_reach_first_views_together(batch):
+    """Four threads, each with a context and a stream of its own, query the same trees, the fast
+    mode (which waits for the view) among them; trees are freed while others are still queried."""
+    import torch
+
+    import cavalry_b200 as cav
+    from cavalry_b200 import scenes
+
+    main = cav.Context(0)
+    ctxs = [cav.Context(0) for _ in range(4)]
+    try:
+        geo = [scenes.soup(n, seed=n) for n in (5000, 9001, 200, 30_000)]
+        geo = [(torch.from_numpy(p).cuda(), torch.from_numpy(i).cuda()) for p, i in geo]
+        trees = main.build_batch(geo, rounds=1) if batch else [main.build(p, i, rounds=1) for p, i in geo]
+        rays = torch.from_numpy(scenes.closest_rays(20_000, seed=5)).cuda()
+        main.set_limits(max_trace_steps=BINARY)
+        want = [t.trace_closest(rays) for t in trees]
+        main.set_limits()
+        torch.cuda.synchronize()
+        bad, gate = [], threading.Barrier(4)
+
+        def work(k):
+            try:
+                s = torch.cuda.Stream()
+                gate.wait()
+                with torch.cuda.stream(s):
+                    for r in range(6):
+                        for j, t in enumerate(trees):
+                            b = cav.Bvh(ctxs[k], t.handle, t.n, owned=False)  # through this thread's context
+                            if k == 3 and r == 2:
+                                dist = b.trace_closest(rays, flags=cav.TRACE_FAST)[1]
+                                s.synchronize()
+                                if not torch.equal(dist, want[j][1]):
+                                    bad.append((k, j, "fast"))
+                            got = b.trace_closest(rays)
+                            s.synchronize()
+                            if not _same(got, want[j]):
+                                bad.append((k, r, j))
+                ctxs[k].sync_check()
+            except Exception as e:  # noqa: BLE001
+                bad.append((k, repr(e)))
+
+        ts = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+        for t in ts:
+            t.start()
+        for t in ts:
+            t.join()
+        assert bad == []
+        for t in trees[:2]:
+            t.free()
+        got = [t.trace_closest(rays) for t in trees[2:]]
+        assert all(_same(g, w) for g, w in zip(got, want[2:]))
+        for t in trees[2:]:
+            t.free()
+        main.sync_check()
+    finally:
+        for c in ctxs:
+            c.close()
+        main.close()
