@@ -355,7 +355,7 @@ struct WideTree {
     CNode* out;
     TriRec* tris_out;
     float4* lbox;
-    uint32_t tris;
+    uint32_t tris, nodes;
 };
 constexpr int kGroupThreads = 512;
 constexpr int kGroupBlocks = 4;
@@ -372,7 +372,7 @@ __global__ void __cluster_dims__(kGroupBlocks) __launch_bounds__(kGroupThreads)
         __threadfence();
     }
     cooperative_groups::this_cluster().sync();
-    wide_levels(t.tn, t.tris_in, t.task, t.out, t.tris_out, t.lbox, ctr, t.tris - 1, t.tris, wait_ns,
+    wide_levels(t.tn, t.tris_in, t.task, t.out, t.tris_out, t.lbox, ctr, t.nodes, t.tris, wait_ns,
                 (rank * kGroupThreads + threadIdx.x) >> 3, kGroupBlocks * kGroupThreads >> 3, kGroupBlocks);
 }
 
@@ -1219,6 +1219,13 @@ enum ViewState { kViewFailed = -1, kViewNone = 0, kViewUnscreened = 1, kViewRead
 
 namespace {
 
+// Wide nodes that a view of n triangles has at most.  A node has eight children, or triangles only
+// (two or more): with F of the former and L of the latter, F + L - 1 of the children are nodes, so
+// n >= L + 7 F + 1 and L <= 7 F + 1, and F + L is at most 4 (n - 2) / 7 + 1.  A child whose box area is
+// no number is never opened, so infinite geometry can need a node for each internal node of the
+// tree: its build fails within the bound and is done again without it (full).
+uint32_t most_nodes(int64_t n, bool full) { return (uint32_t)(full ? n - 1 : std::min(n - 1, 4 * (n - 2) / 7 + 1)); }
+
 std::mutex& view_mutex(const cav_bvh* bvh) { return bvh->shared ? bvh->shared->mu : bvh->view_mu; }
 
 unsigned long long stream_id(cudaStream_t s) {
@@ -1260,9 +1267,10 @@ int view_state(const cav_bvh* bvh) {
 // is: the same launches built them all.  Sets no error: the exact mode does without.
 cudaError_t begin_view(cav_ctx* ctx, const cav_bvh* bvh, cudaStream_t s) {
     auto round = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const bool full = bvh->wide_state.load() == kViewFailed;
     auto bytes = [&](const cav_bvh* b) {
-        return round(sizeof(CNode) * (size_t)(b->n - 1)) + round(sizeof(TriRec) * (size_t)b->n) +
-               round(2 * sizeof(float4) * (size_t)b->n) + round(sizeof(int32_t) * (size_t)(b->n - 1));
+        return round(sizeof(CNode) * (size_t)most_nodes(b->n, full)) + round(sizeof(TriRec) * (size_t)b->n) +
+               round(2 * sizeof(float4) * (size_t)b->n) + round(sizeof(int32_t) * (size_t)most_nodes(b->n, full));
     };
     std::vector<const cav_bvh*> g{bvh};
     size_t need = bytes(bvh);
@@ -1303,10 +1311,11 @@ cudaError_t begin_view(cav_ctx* ctx, const cav_bvh* bvh, cudaStream_t s) {
         t[k].tn = b->tnodes;
         t[k].tris_in = b->tris;
         t[k].root_box = b->d_root_box;
-        t[k].out = (CNode*)carve(sizeof(CNode) * (size_t)(b->n - 1));  // a wide node for each internal node at most
+        t[k].nodes = most_nodes(b->n, full);
+        t[k].out = (CNode*)carve(sizeof(CNode) * (size_t)t[k].nodes);
         t[k].tris_out = (TriRec*)carve(sizeof(TriRec) * (size_t)b->n);
         t[k].lbox = (float4*)carve(2 * sizeof(float4) * (size_t)b->n);
-        t[k].task = (int32_t*)carve(sizeof(int32_t) * (size_t)(b->n - 1));
+        t[k].task = (int32_t*)carve(sizeof(int32_t) * (size_t)t[k].nodes);
         t[k].tris = (uint32_t)b->n;
     }
     WideTree* dt = (WideTree*)carve(sizeof(WideTree) * K);
@@ -1326,7 +1335,7 @@ cudaError_t begin_view(cav_ctx* ctx, const cav_bvh* bvh, cudaStream_t s) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wide_build, kBuildThreads, 0);
         const int64_t room = (int64_t)ctx->num_sms * std::min(std::max(per_sm, 1), 8);
         const int grid = (int)std::min<int64_t>(room, std::max<int64_t>(1, bvh->n * 2 / kBuildThreads));
-        uint32_t max_nodes = w.tris - 1, max_tris = w.tris;
+        uint32_t max_nodes = w.nodes, max_tris = w.tris;
         uint64_t wait_ns = ctx->sort_wait_ns;
         void* args[] = {(void*)&w.tn, (void*)&w.tris_in, (void*)&w.task, (void*)&w.out, (void*)&w.tris_out, (void*)&w.lbox,
                         &dc,          &max_nodes,        &max_tris,      &wait_ns};

@@ -192,3 +192,40 @@ def test_threads_that_reach_first_views_together(batch):
         for c in ctxs:
             c.close()
         main.close()
+
+
+def test_a_view_with_a_node_for_each_binary_node():
+    """Flat boxes of infinite extent have no area to open by, so every wide node holds two children:
+    more nodes than finite geometry can have.  The fast mode still gets its view, alone and in a
+    batch, and the exact mode's answers stay the binary traversal's."""
+    import torch
+
+    import cavalry_b200 as cav
+    from cavalry_b200 import scenes
+
+    ctx = cav.Context(0)
+    try:
+        n = 600
+        pos = np.zeros((3 * n, 3), np.float32)
+        pos[0::3, 0], pos[1::3, 0] = -np.inf, np.inf
+        pos[2::3, 1] = np.linspace(0.0, 1.0, n)
+        pos[:, 1] = np.repeat(pos[2::3, 1], 3)  # each in a plane of its own, flat in y
+        idx = np.arange(3 * n, dtype=np.int32).reshape(n, 3)
+        geo = (torch.from_numpy(pos).cuda(), torch.from_numpy(idx).cuda())
+        other = tuple(torch.from_numpy(a).cuda() for a in scenes.soup(5000, seed=1))
+        rays = torch.from_numpy(scenes.closest_rays(20_000, seed=2)).cuda()
+        trees = [ctx.build(*geo, rounds=0), *ctx.build_batch([geo, other], rounds=0)]
+        for t in trees:
+            ctx.set_limits(max_trace_steps=BINARY)
+            want = t.trace_closest(rays)
+            ctx.set_limits()
+            for _ in range(2):
+                assert _same(t.trace_closest(rays), want)
+                assert torch.equal(t.trace_closest(rays, flags=cav.TRACE_FAST)[1], want[1])
+            assert t.has_fast_layout()
+            assert _same(t.trace_closest(rays), want)
+        ctx.sync_check()
+        for t in trees:
+            t.free()
+    finally:
+        ctx.close()
