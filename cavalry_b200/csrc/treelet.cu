@@ -720,12 +720,12 @@ __global__ void k_treelet_seeds_batch(const TreeletSeg* __restrict__ segs, const
 // The same persistent walkers over a group of trees: a seed names its tree.
 __global__ void __launch_bounds__(kWalkWarps * 32, kWalkBlocksPerSm)
     k_treelet_batch(const TreeletSeg* __restrict__ segs, const int64_t* __restrict__ leaf_off,
-                    const int2* __restrict__ list, uint32_t* visited, int* err, const uint32_t* __restrict__ seeds,
-                    uint32_t* claim) {
+                    const int2* __restrict__ list, uint32_t most, uint32_t* visited, int* err,
+                    const uint32_t* __restrict__ seeds, uint32_t* claim) {
     __shared__ WarpSmem smem[kWalkWarps];
     WarpSmem& S = smem[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
-    const uint32_t total = *seeds;
+    const uint32_t total = min(*seeds, most);  // what the list holds, also of a build that failed
     for (;;) {
         uint32_t i = 0;
         if (lane == 0) i = atomicAdd(claim, 1u);
@@ -793,8 +793,8 @@ cav_status treelet_rounds_batch(cav_ctx* ctx, const TreeletSeg* segs, const Tree
             int2* list = reinterpret_cast<int2*>(leaf_list);
             k_treelet_seeds_batch<<<div_up(nodes, 256), 256, 0, s>>>(segs, leaf_off, k0, k1, list, counters + K, visited,
                                                                      ctx->d_error + 1);
-            k_treelet_batch<<<(unsigned)grid, kWalkWarps * 32, 0, s>>>(segs, leaf_off, list, visited, ctx->d_error + 1,
-                                                                      counters + K, counters + K + 1);
+            k_treelet_batch<<<(unsigned)grid, kWalkWarps * 32, 0, s>>>(segs, leaf_off, list, (uint32_t)(leaves / 2), visited,
+                                                                      ctx->d_error + 1, counters + K, counters + K + 1);
         }
         k0 = k1;
     }

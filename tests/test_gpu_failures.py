@@ -232,3 +232,38 @@ def test_mlp_completion_wait_runs_out_and_reports():
         ref.free()
     finally:
         ctx.close()
+
+
+def test_sort_lookback_wait_runs_out_in_a_batched_build():
+    """The same stall in a batched build with treelet rounds: whatever the unsorted codes made of the
+    trees, the rounds stay within their lists, every tree traces safely with no hits, and the next
+    batch is that of a context that never failed."""
+    import cavalry_b200 as cav
+    from cavalry_b200 import scenes
+
+    ctx = cav.Context(0)
+    try:
+        geo = [tuple(_gpu(a) for a in _soup(n, seed=n)) for n in (12_000, 300, 25_000, 2, 7000)]
+        rays = _gpu(scenes.closest_rays(4096, seed=31))
+        ctx.set_limits(sort_wait_s=0.05)
+        ctx.inject(cav.INJECT_SORT_STALL, 1)
+        trees = ctx.build_batch(geo, rounds=3)
+        with pytest.raises(cav.CavError) as e:
+            ctx.sync_check()
+        assert e.value.status == CAV_ERR_TIMEOUT
+        for t in trees:
+            assert (t.trace_closest(rays)[0].cpu().numpy() == -1).all()
+        ctx.sync_check()
+        for t in trees:
+            t.free()
+        ctx.inject(cav.INJECT_NONE)
+        ctx.set_limits()
+        trees = ctx.build_batch(geo, rounds=3)
+        ctx.sync_check()
+        for t, g in zip(trees, geo):
+            alone = ctx.build(*g, rounds=3)
+            assert np.array_equal(t.export_nodes(), alone.export_nodes())
+            t.free(), alone.free()
+    finally:
+        ctx.inject(cav.INJECT_NONE)
+        ctx.close()
