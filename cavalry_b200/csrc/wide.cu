@@ -360,6 +360,11 @@ struct WideTree {
 constexpr int kGroupThreads = 512;
 constexpr int kGroupBlocks = 4;
 constexpr int64_t kGroupTris = 1 << 16;             // larger trees take the grid
+// And so does a tree of more than this many triangles for each of the group: few clusters leave most
+// of the chip idle (views and queries of 2,048 rays: two trees of 5,000 triangles 0.23 ms together and
+// 0.26 one by one, of 20,000 0.48 and 0.42, of 60,000 1.06 and 0.80; of 60,000 four 1.61 and 1.57,
+// eight 2.77 and 3.18, sixteen 5.1 and 6.4).
+constexpr int64_t kGroupShare = 1 << 13;
 constexpr size_t kGroupBytes = (size_t)256 << 20;  // of the views together, at most
 
 __global__ void __cluster_dims__(kGroupBlocks) __launch_bounds__(kGroupThreads)
@@ -1280,7 +1285,7 @@ cudaError_t begin_view(cav_ctx* ctx, const cav_bvh* bvh, cudaStream_t s) {
                 g.push_back(b);
                 need += bytes(b);
             }
-        if (need > kGroupBytes) {
+        if (need > kGroupBytes || bvh->n > kGroupShare * (int64_t)g.size()) {
             g.resize(1);
             need = bytes(bvh);
         }
@@ -1414,13 +1419,13 @@ void detach_wide(cav_bvh* bvh, cudaStream_t s, bool async, std::vector<void*>& m
     bvh->wide_state.store(kViewNone);
 }
 
-// Rays that a tree must have been asked about before the exact mode builds its view.  The view
-// of a tree of 10,000 triangles or more costs less than what its first batch saves, down to
-// 64 rays (soups, closest hit, a call with the view's build against the binary traversal:
-// 10,000 triangles and 512 rays 157 against 283 us, 100,000 and 512 rays 305 against 1,162 us,
-// 1M and 512 rays 1.6 against 8.2 ms); smaller trees save 10 to 30 us a call and the view
-// costs 70 us.
-// A batched build's trees get their views together.
+// Rays that a tree must have been asked about before the exact mode builds its view.  From 4,096
+// triangles on the view is worth it with the first 512 rays or soon after (closest hits, the call
+// with the view's build, the binary traversal, and the next call: soups of 4,200 triangles 124,
+// 135 and 56 us, of 10,000 147, 234 and 73 us, of 100,000 0.41, 1.12 and 0.25 ms, of 1M 2.6, 7.3 and
+// 1.8 ms; spheres, whose lines meet few boxes, of 20,498 136, 64 and 46 us, of 327,698 302, 279 and
+// 64 us).  Smaller trees gain less than they pay for many calls (1,000 triangles and 16,384 rays
+// 106, 66 and 60 us; 2,000 125, 94 and 71).  A batched build's trees get their views together.
 static int64_t screen_min_rays(const cav_bvh* bvh) { return bvh->n >= 4096 || bvh->shared ? 512 : 16384; }
 
 // How n rays (negative: a number that only the device knows) of the exact mode go.  Once the tree
