@@ -2,8 +2,9 @@
 // walking bottom-up from the leaves with an arrival counter per node, dynamic
 // programming over the 128 leaf subsets staged in shared memory.
 //
-// Output is bit-identical to the reference's optimizeBVH (BVH/Optimization.cu:467-525
-// with optimizeTreelet :49-462): same treelet formation (expand the largest-area
+// Output is that of the reference's optimizeBVH (BVH/Optimization.cu:467-525 with
+// optimizeTreelet :49-462) up to the rounding of surface areas (subset_area below): same
+// treelet formation (expand the largest-area
 // node, first lane on ties), same partition enumeration order per subset, the same
 // warp min-reduction tree for the 6- and 7-leaf subsets, and the same reuse of node
 // ids by lane during reconstruction.  It differs in mechanics only:
@@ -126,8 +127,11 @@ __device__ inline void reduce_partition(float& tc, int& p) {
     p = __shfl_sync(kFull, p, (int)win);
 }
 
-// The area of a union of treelet leaves, rounded as this pass always has (the other order of
-// the contraction than surface_area).
+// The area of a union of treelet leaves, rounded as this pass always has: the other order of the
+// contraction than surface_area (the build's, and the one that the reference's build kernels were
+// seen to have).  Partitions whose costs are a rounding apart can fall the other way for it: trees
+// of icospheres differ from the oracle's own rounding in a part of their nodes, and are the
+// oracle's node for node with this one.
 __device__ __forceinline__ float subset_area(f3 lo, f3 hi) {
     const f3 e = hi - lo;
     return 2.f * fmaf(e.x, e.z, fmaf(e.y, e.z, __fmul_rn(e.x, e.y)));

@@ -70,6 +70,17 @@ static float surface_area(const float* bmin, const float* bmax) {
     float s = fmaf(ex, ez, fmaf(ex, ey, ey * ez));
     return 2.0f * s;
 }
+/* The same sum contracted the other way, fma(ex, ez, fma(ey, ez, ex*ey)): what the treelet pass
+ * under test has.  The treelet rounds of this file use it while the switch below is on. */
+static int g_other_area;
+void orc_treelet_area(int other) { g_other_area = other; }
+static float treelet_area(const float* bmin, const float* bmax) {
+    if (!g_other_area) return surface_area(bmin, bmax);
+    float ex = bmax[0] - bmin[0];
+    float ey = bmax[1] - bmin[1];
+    float ez = bmax[2] - bmin[2];
+    return 2.0f * fmaf(ex, ez, fmaf(ey, ez, ex * ey));
+}
 /* SAH.h:10-12: area * 1.0 * n in double, returned as float. */
 static float leaf_cost(float area, int n) { return (float)((double)area * 1.0 * (double)n); }
 /* SAH.h:15-17: area * 1.2 + l + r in double (first add contracted), returned as float. */
@@ -398,7 +409,7 @@ static void treelet(ONode* nodes, int32_t root) {
             if (!any) { memcpy(bmin, L->bmin, 12); memcpy(bmax, L->bmax, 12); any = 1; }
             else box_union(bmin, bmax, L->bmin, L->bmax, bmin, bmax);
         }
-        area[s] = any ? surface_area(bmin, bmax) : 0.0f;
+        area[s] = any ? treelet_area(bmin, bmax) : 0.0f;
         opt_cost[s] = -1.0f;
         opt_part[s] = 0;
     }
@@ -537,7 +548,7 @@ static void treelet(ONode* nodes, int32_t root) {
             n->end = nend[l];
             memcpy(n->bmin, nbmin[l], 12);
             memcpy(n->bmax, nbmax[l], 12);
-            n->area = surface_area(n->bmin, n->bmax);
+            n->area = treelet_area(n->bmin, n->bmax);
         } else {
             /* the reference stores an uninitialised box/prim range here and then
              * overwrites box/area in the refresh loop; prim range stays unspecified */
@@ -553,7 +564,7 @@ static void treelet(ONode* nodes, int32_t root) {
             const ONode* a = &nodes[n->left];
             const ONode* b = &nodes[n->right];
             box_union(a->bmin, a->bmax, b->bmin, b->bmax, n->bmin, n->bmax);
-            n->area = surface_area(n->bmin, n->bmax);
+            n->area = treelet_area(n->bmin, n->bmax);
         }
         if (n->is_leaf) n->cost = leaf_cost(n->area, n->end - n->begin + 1);
         else n->cost = internal_cost3(n->area, nodes[n->left].cost, nodes[n->right].cost);

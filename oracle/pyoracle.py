@@ -40,6 +40,7 @@ def oracle_lib() -> ctypes.CDLL:
         L.orc_trace_closest.argtypes = [P, P, P, P, I64, P, P, P, P]
         L.orc_trace_any.argtypes = [P, P, P, P, P, P, P, I64, P]
         L.orc_treelet_rounds.argtypes = [P, I64, ctypes.c_int]
+        L.orc_treelet_area.argtypes = [ctypes.c_int]
         L.orc_morton.argtypes = [P, I64, P, P]
         L.orc_leaf_boxes.argtypes = [P, P, I64, P]
         L.orc_scene_bounds.argtypes = [P, I64, P]
@@ -48,8 +49,9 @@ def oracle_lib() -> ctypes.CDLL:
     return _orc
 
 
-def build(pos: np.ndarray, idx: np.ndarray, bounds=None, codes=None, rounds: int = 0) -> dict:
-    """Oracle LBVH build.  codes: optional unsorted Morton codes to use instead of computing them."""
+def build(pos: np.ndarray, idx: np.ndarray, bounds=None, codes=None, rounds: int = 0, other_area: bool = False) -> dict:
+    """Oracle LBVH build.  codes: optional unsorted Morton codes to use instead of computing them.
+    other_area: the treelet rounds round surface areas as the GPU's do (the other contraction)."""
     pos = np.ascontiguousarray(pos, np.float32)
     idx = np.ascontiguousarray(idx, np.int32)
     n = idx.shape[0]
@@ -63,8 +65,10 @@ def build(pos: np.ndarray, idx: np.ndarray, bounds=None, codes=None, rounds: int
     }
     b = None if bounds is None else np.ascontiguousarray(bounds, np.float32)
     c = None if codes is None else np.ascontiguousarray(codes, np.uint64)
+    oracle_lib().orc_treelet_area(int(other_area))
     st = oracle_lib().orc_build(_c(pos), _c(idx), n, _c(b), _c(c), int(rounds), _c(out["codes"]), _c(out["sorted"]),
                                 _c(out["perm"]), _c(out["merged"]), _c(out["final"]), _c(out["bounds"]))
+    oracle_lib().orc_treelet_area(0)
     if st != 0:
         raise ValueError(f"orc_build failed ({st})")
     return out

@@ -362,3 +362,29 @@ def test_treelets_on_ties_match_oracle(cuda_ctx, n, rounds):
     nodes_equal(bvh.export_nodes(), o["final"], f"lattice {n} rounds {rounds}")
     cuda_ctx.sync_check()
     bvh.free()
+
+
+@pytest.mark.parametrize("level,rounds", [(1, 1), (2, 3), (3, 3)])
+def test_treelets_on_icospheres_match_oracle(cuda_ctx, level, rounds):
+    """Icospheres' triangles come in near-equal pairs, whose partitions' costs are a rounding apart:
+    the trees are the oracle's bit for bit with the treelet pass's own contraction of surface
+    areas; with the build's contraction (the oracle's default) 0.4, 5.6 and 10 % of the nodes
+    differ in these scenes."""
+    import torch
+
+    from cavalry_b200 import scenes
+    from oracle import pyoracle as po
+
+    s = scenes.sphere_scene(8, level, seed=5)
+    pos, idx = s["positions"], s["indices"]
+    bvh = cuda_ctx.build(torch.from_numpy(pos).cuda(), torch.from_numpy(idx).cuda(), rounds=rounds)
+    mu, _, _ = bvh.export_stages()
+    got = bvh.export_nodes()
+    o = po.build(pos, idx, codes=mu, rounds=rounds, other_area=True)
+    nodes_equal(got, o["final"], f"icospheres level {level} rounds {rounds}")
+    o = po.build(pos, idx, codes=mu, rounds=rounds)["final"]
+    same = (got["left"] == o["left"]) & (got["right"] == o["right"]) & (got["bmin"] == o["bmin"]).all(1)
+    same &= (got["bmax"] == o["bmax"]).all(1)
+    print(f"level {level} rounds {rounds}: {1 - same.mean():.4f} of the nodes differ")
+    assert 0.85 < same.mean() < 1.0
+    bvh.free()
