@@ -384,16 +384,18 @@ namespace {
 // Rays per pipelined chunk: at most what the staging slots hold.
 constexpr int64_t kChunkRays = (int64_t)1 << 22;
 
-// Of a call that is cut for the sake of its copies, up to four chunks of 2^18 rays or more: the
-// first chunk's copy in and the last one's copy out overlap nothing.  Any-hit calls are (their
-// traversal takes no longer than their copies), and calls with pageable buffers, which the host
-// copies itself: 1M shadow rays on 200,000 triangles 1.79 ms in one chunk, 1.50 in three,
-// pageable 5.1 and 3.2; 4M on 1M triangles 8.8 and 6.8 in four; pageable closest hits on 200,000
-// triangles 9.1 and 6.6.  Closest hits of pinned buffers are not: every chunk's traversal ends in
-// a tail of its longest rays, which the next chunk's only partly hides (1M rays on 1M triangles
-// 11.0 ms in one chunk, 11.9 in three; on 200,000 triangles 3.97 and 3.86).
-int64_t chunk_rays(int64_t n, bool cut) {
-    const int64_t parts = cut ? std::clamp<int64_t>(n >> 18, 1, 4) : 1;
+// Of a call that is cut for the sake of its copies, up to four chunks of `least` rays or more: the
+// first chunk's copy in and the last one's copy out overlap nothing.  Any-hit calls are cut into
+// chunks of 2^18 (their traversal takes no longer than their copies), and so are closest hits with
+// pageable buffers, which the host copies itself, where the traversal has a short tail (the view, and
+// the fast mode): 1M shadow rays on 200,000 triangles 2.1 ms in one chunk and 2.0 to 2.3 in three,
+// pageable 4.6 and 3.4; 4M on 1M triangles 11.3 and 8.8 in four.  The binary traversal of closest hits ends in
+// a tail of its longest rays, which the next chunk's only partly hides: pageable 1M rays on 1M
+// triangles 26.3 ms in one chunk and 34.3 in three, on 200,000 11.5 and 11.4, but 4M rays there 36.2
+// and 29.8 in four, so their chunks are of 2^20.  Closest hits of pinned buffers are not cut (1M rays
+// on 1M triangles 21.6 and 32.4, on 200,000 6.8 and 9.0).
+int64_t chunk_rays(int64_t n, bool cut, int64_t least = (int64_t)1 << 18) {
+    const int64_t parts = cut ? std::clamp<int64_t>(n / least, 1, 4) : 1;
     return std::min(kChunkRays, (n + parts - 1) / parts);
 }
 
@@ -505,7 +507,8 @@ cav_status cav_trace_closest_host(cav_ctx* ctx, const cav_bvh* bvh, const cav_ra
     if (st != CAV_OK) return st;
     st = order_after_build(ctx, bvh);
     if (st != CAV_OK) return st;
-    const int64_t chunk = chunk_rays(n, !(in_pinned && out_pinned));
+    const bool tail = !(flags & CAV_TRACE_FAST) && !view_is_sparse(bvh);
+    const int64_t chunk = chunk_rays(n, !(in_pinned && out_pinned), (int64_t)1 << (tail ? 20 : 18));
     if (n > chunk && !(flags & (CAV_TRACE_FAST | CAV_TRACE_CULL_ON_POP))) {
         st = share_view(ctx, bvh, false, n, ctx->hstream[0], ctx->hstream[1]);
         if (st != CAV_OK) return st;

@@ -298,6 +298,7 @@ void detach_wide(cav_bvh* bvh, cudaStream_t s, bool async, std::vector<void*>& m
 // launch and the binary traversal's both go out with q.gate set, and one of them does nothing.
 enum ViewUse { kUseBinary, kUseView, kUseBoth };
 ViewUse view_use(cav_ctx* ctx, const cav_bvh* bvh, bool any_hit, int64_t n, cudaStream_t s);
+bool view_is_sparse(const cav_bvh* bvh);  // whether any number of closest hits is known to go through the view
 // A call that spreads n rays over two streams of the context: a view that it begins on `a` serves `b`.
 cav_status share_view(cav_ctx* ctx, const cav_bvh* bvh, bool any_hit, int64_t n, cudaStream_t a, cudaStream_t b);
 cav_status trace_screened(cav_ctx* ctx, const cav_bvh* bvh, const TraceSeg& q, bool any_hit, int64_t n, cudaStream_t s,

@@ -1,6 +1,6 @@
 // The compressed 8-wide view of the binary tree, and persistent-warp traversal over it: the
-// fast traversal mode (CAV_TRACE_FAST), and the screening pass that answers nearly every ray
-// of the exact mode.
+// fast traversal mode (CAV_TRACE_FAST), and the screening pass that answers the rays of the exact
+// mode that go this way (view_use).
 //
 // Layout (CNode, 96 bytes) after Ylitie, Karras and Laine, "Efficient Incoherent Ray
 // Traversal on GPUs Through Compressed Wide BVHs" (HPG 2017): up to eight children per
@@ -542,7 +542,9 @@ __device__ inline bool screenable(const f3& o, const f3& d) {
 // to give: taking the nearest group instead made 65,536 closest-hit rays 1.85 against 1.44 ms.
 // Waiting for a hit or a number of steps before sharing a ray measured slower too (2.7 and 2.2
 // against 1.6 ms).  1M-triangle soup, fast mode, with and without sharing: 16,384 shadow rays
-// 0.12 against 1.4 ms, 65,536 closest-hit rays 1.5 against 6.1, 4M 35.7 against 43.8.
+// 0.12 against 1.4 ms, 65,536 closest-hit rays 1.5 against 6.1, 4M 35.7 against 43.8.  (Closest-hit
+// times of the kernel's variants here and below are of searches that end at the hit found, as the
+// fast mode's do.)
 struct ShareRec {
     int32_t bound[32];  // closest, fast mode: the smallest distance any lane of the ray has seen (float bits)
     float best[32], second[32];  // the two smallest distances of the merged lanes (second negative: a lane failed)
@@ -1428,6 +1430,10 @@ void detach_wide(cav_bvh* bvh, cudaStream_t s, bool async, std::vector<void*>& m
 // 106, 66 and 60 us; 2,000 125, 94 and 71).  A batched build's trees get their views together.
 static int64_t screen_min_rays(const cav_bvh* bvh) { return bvh->n >= 4096 || bvh->shared ? 512 : 16384; }
 
+bool view_is_sparse(const cav_bvh* bvh) {
+    return view_state(bvh) == kViewReady && bvh->boxes_per_line.load() <= kSparse;
+}
+
 // How n rays (negative: a number that only the device knows) of the exact mode go.  Once the tree
 // has been asked about enough of them its view's build is enqueued on the stream; nothing waits for
 // it.  Until its verdict has arrived, calls on that stream come after it and let the device
@@ -1459,7 +1465,7 @@ ViewUse view_use(cav_ctx* ctx, const cav_bvh* bvh, bool any_hit, int64_t n, cuda
     }
     if (st == kViewMixed) return kUseBoth;
     if (st != kViewReady) return kUseBinary;
-    if (any_hit || bvh->boxes_per_line.load() <= kSparse) return kUseView;
+    if (any_hit || view_is_sparse(bvh)) return kUseView;
     return n < 0 ? kUseBoth : (n <= kFewRays ? kUseView : kUseBinary);
 }
 

@@ -229,3 +229,46 @@ def test_a_view_with_a_node_for_each_binary_node():
             t.free()
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("scene,n", [("soup", 2**21 - 1), ("soup", 2**21), ("soup", 2**21 + 3), ("spheres", 2**19 - 1),
+                                     ("spheres", 2**19 + 3)])
+def test_host_calls_at_their_first_view(scene, n):
+    """Closest hits from pageable buffers below, at and above the sizes where they are cut into two
+    chunks (2^20 rays each in the binary traversal, 2^18 through the view), on a tree whose first call
+    begins the view and on the same tree with the view: the device call's results."""
+    import torch
+
+    import cavalry_b200 as cav
+    from cavalry_b200 import scenes
+
+    ctx = cav.Context(0)
+    try:
+        if scene == "soup":
+            pos, idx = scenes.soup(40_000, seed=6)
+        else:
+            s = scenes.sphere_scene(8, 2, seed=6)
+            pos, idx = s["positions"], s["indices"]
+        geo = (torch.from_numpy(pos).cuda(), torch.from_numpy(idx).cuda())
+        rays = scenes.closest_rays(n, seed=7)
+        shadow, limit = scenes.shadow_rays(n, seed=8)
+        want = None
+        for first in (True, False):
+            bvh = ctx.build(*geo, rounds=2)
+            if want is None:
+                ctx.set_limits(max_trace_steps=BINARY)
+                want = [a.cpu().numpy() for a in bvh.trace_closest(torch.from_numpy(rays).cuda())]
+                occ = bvh.trace_any(torch.from_numpy(shadow).cuda(), torch.from_numpy(limit).cuda()).cpu().numpy()
+                ctx.set_limits()
+            if not first:
+                bvh.trace_any(torch.from_numpy(shadow).cuda())
+                torch.cuda.synchronize()
+                assert bvh.has_fast_layout()
+                bvh.trace_any(torch.from_numpy(shadow).cuda())
+            got = bvh.trace_closest_host(rays)
+            assert all(np.array_equal(g.view(np.uint8), w.view(np.uint8)) for g, w in zip(got, want))
+            assert np.array_equal(bvh.trace_any_host(shadow, limit), occ)
+            ctx.sync_check()
+            bvh.free()
+    finally:
+        ctx.close()
