@@ -45,7 +45,7 @@ HIT_BYTES = 16  # prim id 4 + t 4 + uv 8
 # 36 B (three float3 vertices) per triangle tested, counted by the instrumented kernel
 NODE_BYTES = 64
 TRI_BYTES = 36
-WIDE_NODE_BYTES = 96  # node of the compressed 8-wide view (the fast mode, and the exact mode through it)
+WIDE_NODE_BYTES = 96  # node of the compressed 8-wide view (the fast mode)
 
 
 def parse():
@@ -355,8 +355,8 @@ def run_ours(args):
     e2e_value = N_RAYS * world / (e2e_total / args.steps * 1e-3) / 1e6
 
     peak, peak_kind = measured_peaks()
-    # the exact mode runs on the compressed 8-wide view; nodes_per_ray is the binary traversal's count
-    bytes_per_ray = RAY_BYTES + HIT_BYTES + WIDE_NODE_BYTES * fnodes / N_RAYS + TRI_BYTES * ftris / N_RAYS
+    # so many closest hits on so dense a tree take the binary traversal (wide.cu, view_use)
+    bytes_per_ray = RAY_BYTES + HIT_BYTES + NODE_BYTES * nodes_per_ray + TRI_BYTES * tris_per_ray
     achieved = bytes_per_ray * N_RAYS / (ms_per_step * 1e-3) / 1e9
     prof = committed_profile()
     traffic = prof.get("dram_bytes_per_launch")
@@ -408,9 +408,10 @@ def run_ours(args):
             # The node-fetch stream is measured against the HBM copy peak (the algorithmic
             # bytes of the scope table), but with the rays in Morton order nearly all of it is
             # served by L2 and DRAM carries well under a percent of the peak: the kernel is
-            # bound by instruction issue (eight box tests per node), not by HBM.  The time is
-            # the whole step's (sort included).
-            "bound": "issue",
+            # bound by the L1 data pipe's wavefronts (one per lane per 32-byte node half,
+            # ncu), not by HBM, and that pipe's rate is the fraction to read.  The time is the
+            # whole step's (sort included).
+            "bound": "l1/l2",
             "achieved": round(achieved, 1),
             "peak": peak,
             "unit": "GB/s",
@@ -423,11 +424,9 @@ def run_ours(args):
             "lts_throughput_pct": prof.get("lts_throughput_pct"),
             "l2_hit_rate_pct": prof.get("l2_hit_rate_pct"),
             "algorithmic_bytes_per_ray": round(bytes_per_ray, 2),
-            "nodes_per_ray": round(fnodes / N_RAYS, 3),
-            "tris_per_ray": round(ftris / N_RAYS, 3),
-            "binary_nodes_per_ray": round(nodes_per_ray, 3),
-            "binary_tris_per_ray": round(tris_per_ray, 3),
-            "kernel": "k_trace_wide<closest, exact> (compressed 8-wide nodes, 96 B)",
+            "nodes_per_ray": round(nodes_per_ray, 3),
+            "tris_per_ray": round(tris_per_ray, 3),
+            "kernel": "k_closest (binary nodes, 64 B)",
         },
         "clocks": clk,
         "anyhit_mrays_s": round(N_RAYS / (statistics.mean(any_ms) * 1e-3) / 1e6, 2),

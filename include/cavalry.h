@@ -214,11 +214,14 @@ cav_status cav_set_trace_config(cav_ctx* ctx, int block_threads, int blocks_per_
  * Traversal-stack override of a mode's single-tree launches (the autotuner sets it):
  *   flags      : CAV_TRACE_EXACT or CAV_TRACE_FAST, the mode whose stack is set
  *   stack      : exact mode: 64 (used only where the tree's depth fits) or 128 entries per
- *                lane, 0 = 128; fast mode: 0
- *   smem_stack : entries per lane kept in shared memory (exact: 16 or 0, fast: 8 or 0); the
- *                rest of the stack is in local memory.  Shared entries cost one L1 wavefront
- *                per push or pop whatever the lanes' depths, and leave less L1 for node data.
- * Results do not depend on either choice.
+ *                lane, 0 = 128, of the binary traversal (the search of the 8-wide view always
+ *                has 128); fast mode: 0
+ *   smem_stack : entries per lane kept in shared memory (exact: 16 or 0, of which the search of
+ *                the view keeps 8 or 0; fast: 8 or 0); the rest of the stack is in local memory.
+ *                Shared entries cost one L1 wavefront per push or pop whatever the lanes'
+ *                depths, and leave less L1 for node data.
+ * Until the call is made, searches of the view (fast or exact) keep 8 for closest hits and none for
+ * any hits, and the binary traversal none.  Results do not depend on either choice.
  */
 cav_status cav_set_trace_stack(cav_ctx* ctx, uint32_t flags, int stack, int smem_stack);
 
@@ -455,7 +458,8 @@ cav_status cav_server_stats(cav_server* server, cav_server_stats_t* out);
  * a 64-entry traversal stack when the tree's depth allows it, else 128; the stack's first
  * 16 entries in shared memory or all of it in local memory) and installs the fastest in ctx
  * for later single-tree traversals (merged launches always use the full stack in local
- * memory).  ms is the best launch time of the chosen shape on the sample; smem_stack is the
+ * memory).  What is timed is what such a batch runs: the exact mode's search of the 8-wide view, where
+ * the batch goes that way, has no choice of stack size (cav_set_trace_stack).  ms is the best launch time of the chosen shape on the sample; smem_stack is the
  * number of stack entries per lane the chosen shape keeps in shared memory (exact mode 16 or
  * 0, fast mode 8 or 0). */
 typedef struct cav_trace_config_t {
@@ -538,8 +542,8 @@ cav_status cav_render_guided(cav_ctx* ctx, cav_scene* scene, const cav_render_op
 
 /* Builds the BVHs of num_scenes scenes with one launch per LBVH stage across all of them
  * (leaf boxes and per-scene bounds, Morton codes, one stable sort of every code plus one
- * stable pass on the scene index, the radix trees, the refits); treelet rounds and the
- * traversal layout then run per scene.  out[k] is identical to cav_bvh_build of scene k
+ * stable pass on the scene index, the radix trees, the refits); treelet rounds then run for
+ * groups of scenes and the traversal layout for all.  out[k] is identical to cav_bvh_build of scene k
  * alone.  positions[k], indices[k], mesh_ids[k] (mesh_ids may be NULL) are DEVICE arrays;
  * num_vertices, num_triangles: host arrays (vertex indices are checked against num_vertices
  * as in cav_bvh_build); scene_bounds: NULL (computed) or num_scenes x 6 host floats.  At
@@ -549,8 +553,11 @@ cav_status cav_bvh_build_batch(cav_ctx* ctx, int num_scenes, const float* const*
                                const int32_t* const* mesh_ids, const int64_t* num_triangles,
                                const float* scene_bounds, int rounds, void* stream, cav_bvh** out);
 
-/* Device-side event timing of the last build's stages (ms): leaf boxes + Morton,
- * sort, radix tree, refit, treelet rounds, layout.  Valid after the stream is synced. */
+/* Device-side event timing of the tree's build stages (ms): leaf boxes + Morton, sort, radix
+ * tree, refit, treelet rounds, layout.  Valid after the stream is synced.  For trees of up to 2,048
+ * triangles built alone the first number is that of the first four stages, which are one launch
+ * (the other three are 0); the trees of a batched build pass each stage together and all report
+ * the batch's times. */
 cav_status cav_bvh_stage_times(cav_ctx* ctx, const cav_bvh* bvh, float* ms6);
 
 #ifdef __cplusplus
