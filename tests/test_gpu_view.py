@@ -272,3 +272,49 @@ def test_host_calls_at_their_first_view(scene, n):
             bvh.free()
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("dense", [False, True])
+def test_graph_renders_with_and_without_a_view(dense, tmp_path):
+    """An exact graph render captures the view's launches where the view is complete, with the binary
+    ones beside them where only the device knows which serve the rays (densely overlapping boxes), and
+    the binary ones where there is no view: the stream-ordered render's film and ray counts."""
+    import torch
+
+    import cavalry_b200 as cav
+    from cavalry_b200 import scenes
+
+    ctx = cav.Context(0)
+    try:
+        s = scenes.soup_scene(40_000, seed=4) if dense else scenes.sphere_scene(8, 2, seed=5)
+        path = str(tmp_path / "scene.pbrt")
+        scenes.write_pbrt(path, s, width=96, height=64, spp=4, max_depth=5, ply=True)
+        sc = ctx.load_pbrt(path, bvh_rounds=2)
+        bvh = sc.bvh()
+        nodes = bvh.export_nodes()
+        e = (nodes["bmax"] - nodes["bmin"]).astype(np.float64)
+        area = e[:, 0] * e[:, 1] + e[:, 1] * e[:, 2] + e[:, 2] * e[:, 0]
+        lines = area[nodes["is_leaf"].astype(bool)].sum() / area[0]
+        assert lines > 13 if dense else lines < 11  # the rule's line is at 12
+        films, counts = [], []
+        rays = torch.from_numpy(scenes.closest_rays(20_000, seed=1)).cuda()
+        for view in (False, True):
+            if view:
+                bvh.trace_any(rays)
+                torch.cuda.synchronize()
+                assert bvh.has_fast_layout()
+            f, w, _ = sc.render(graph=True)
+            films.append((f, w))
+            counts.append((sc.stats().closest_rays, sc.stats().shadow_rays))
+            assert bool(bvh.has_fast_layout()) == view
+        f, w, _ = sc.render()
+        films.append((f, w))
+        counts.append((sc.stats().closest_rays, sc.stats().shadow_rays))
+        assert counts[0] == counts[1] == counts[2] and counts[0][0] > 20_000
+        for f, w in films[1:]:
+            assert np.array_equal(w, films[0][1])
+            assert np.allclose(f, films[0][0], rtol=2e-5, atol=1e-6)  # float film sums in another order
+        ctx.sync_check()
+        del sc, bvh
+    finally:
+        ctx.close()
